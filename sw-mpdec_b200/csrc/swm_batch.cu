@@ -279,7 +279,6 @@ static JacobiArgs batch_jac_desc(const swm_batch* b, const BProblem& q, int k, i
   jj.xa = q.xa[qs];
   jj.xb = q.xb[qs];
   jj.out = (k == 5) ? q.h : q.hbuf[m - 1][k & 1];
-  jj.recip = b->fast ? 1 : 0;
   return jj;
 }
 

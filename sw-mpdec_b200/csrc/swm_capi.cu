@@ -5,6 +5,7 @@
 // state lives on the device as three planes [ny][nx]; one step is the fixed
 // sequence of kernels below, captured once into a CUDA graph (dt is read from
 // device memory, so the graph is replayed unchanged every step).
+#include <algorithm>
 #include <array>
 #include <atomic>
 #include <cmath>
@@ -97,14 +98,14 @@ struct swm_solver {
   double* fv[4] = {};
   double* fxm[4] = {};
   double* fym[4] = {};
-  // Patankar system
-  double *cS = nullptr, *cW = nullptr, *cE = nullptr, *cN = nullptr, *cD = nullptr;
-  // stencil mPDeC5: the systems of substeps 3 and 4 when a correction iteration's
-  // three substeps are assembled in one launch ([q][S, W, E, N, D], q = m - 3)
-  double* cset[2][5] = {};
-  double *csr_mass = nullptr, *csr_diag = nullptr;
+  // Patankar systems: set 0, and in mPDeC5 sets 1 and 2 for the other substeps of a
+  // correction iteration (planes S, W, E, N, D, or CSR Mass and Diagonal); xa, xb: the
+  // iterates of each set's solve (sets 1, 2 only when the three are solved together)
+  double* cset[kMaxSys][5] = {};
+  double *csr_mass[kMaxSys] = {}, *csr_diag[kMaxSys] = {};
   int *rowstart = nullptr, *cols = nullptr;
-  double *xa = nullptr, *xb = nullptr, *rhs_compat = nullptr;
+  double *xa[kMaxSys] = {}, *xb[kMaxSys] = {}, *rhs_compat = nullptr;
+  bool grouped = false;  // a correction's three systems are solved by one launch
   // well-balanced reference
   double *fxwb = nullptr, *fywb = nullptr, *swb = nullptr;
   bool have_wb = false;
@@ -128,8 +129,8 @@ struct swm_solver {
   char* out_dev = nullptr;
   char* out_host = nullptr;  // pinned
   size_t out_cap = 0;
-  double* stage = nullptr;  // ghosted staging (3*(nx+6)*(ny+6))
-  double* stage2 = nullptr;
+  double* stage = nullptr;  // ghosted staging (3*(nx+6)*(ny+6)), shared with xa, xb
+  double* stage2 = nullptr;  // the same, shared with set 0
   // pinned host mirrors
   double* h_dt = nullptr;
   JacobiCtl* h_ctl = nullptr;
@@ -138,7 +139,7 @@ struct swm_solver {
   // graph
   cudaGraphExec_t graph = nullptr;
   bool graph_failed = false;
-  int jac_blocks = 0;
+  JacobiGrid jac_grid{};
   int n_solves = 0;
   // grid-barrier watchdog of the Jacobi launches (polls before giving up)
   long long spin_limit = kDefaultSpinLimit;
@@ -198,10 +199,23 @@ static bool fast_patankar(const swm_params& p) {
   return p.precision != SWM_PREC_FP64 && p.solver == SWM_SOLVER_STENCIL;
 }
 
+// Sweeps per Jacobi pass at most; 0 (and the CSR solver) leaves it to the kernel.
 static int jacobi_block_of(const swm_params& p) {
-  if (p.solver == SWM_SOLVER_CSR) return 1;
-  return p.jacobi_block > 0 ? p.jacobi_block : 4;
+  if (p.solver == SWM_SOLVER_CSR) return kMaxBlock;
+  return p.jacobi_block > 0 ? p.jacobi_block : kMaxBlock;
 }
+
+static int jacobi_form(const swm_params& p) {
+  if (p.solver == SWM_SOLVER_CSR) return kSysCsr;
+  return fast_patankar(p) ? kSysRecip : kSysDiv;
+}
+
+// The three substeps of an mPDeC5 correction depend only on the previous correction, so
+// their systems are solved by one launch: one set of passes, barriers and tails instead
+// of three.  That takes up to 17 more planes; beyond
+// kGroupCells one system alone keeps every SM busy for many passes' worth of rows, and
+// the memory is left to larger grids.
+constexpr size_t kGroupCells = size_t(1) << 23;
 
 static RhsArgs make_rhs_args(swm_solver* s, const double* h, const double* hu, const double* hv,
                              int slot) {
@@ -510,15 +524,28 @@ static int enqueue_patankar(swm_solver* s) {
     CK(launch_rhs(s, make_rhs_args(s, s->h, s->hu, s->hv, 0)));
     prof_mark(s, -1);
   }
-  int solve = 0;
+  int solve = 0, last_solve[5] = {-1, -1, -1, -1, -1};  // by substep: its latest solve
   // the three substeps of an mPDeC5 correction iteration depend only on the previous
-  // iteration, so (split and FMA forms, stencil layout) they are assembled in one
-  // launch into three systems, then solved one after another
-  const bool fused = !csr && ms == 4 && fast_patankar(s->p) && s->cset[1][4] != nullptr;
+  // iteration: the split and FMA forms assemble them in one launch (stencil layout), and
+  // they are solved together unless the grid is large (kGroupCells)
+  const bool fused = !csr && ms == 4 && fast_patankar(s->p);
   for (int k = 1; k <= kc; ++k) {
     const int mlo = (k == kc) ? ms : 2;
-    const bool fuse_k = fused && k < kc;
+    const bool last = (k == kc);
+    const bool fuse_k = fused && !last, group_k = s->grouped && ms == 4 && !last;
+    JacobiGroup ja{};
+    ja.nx = s->nx;
+    ja.ny = s->ny;
+    ja.maxiter = s->p.jacobi_maxiter;
+    ja.block = jacobi_block_of(s->p);
+    ja.form = jacobi_form(s->p);
+    fill_thresh(s, ja.thresh);
+    ja.rowstart = s->rowstart;
+    ja.cols = s->cols;
+    ja.ctl = s->ctl;
+    ja.spin_limit = s->spin_limit;
     for (int m = mlo; m <= ms; ++m) {
+      const int set = (fuse_k || group_k) ? m - 2 : 0;  // substep m's system
       AssembleArgs aa{};
       aa.nx = s->nx;
       aa.ny = s->ny;
@@ -539,24 +566,19 @@ static int enqueue_patankar(swm_solver* s) {
         aa.fym[r] = s->fym[slot];
         aa.hp[r] = (r == 0 || k == 1) ? s->h : s->hbuf[r][(k - 1) & 1];
       }
-      const bool last = (k == kc);
       aa.hu_out = last ? s->hu : s->hum[m - 1];
       aa.hv_out = last ? s->hv : s->hvm[m - 1];
-      aa.cS = s->cS;
-      aa.cW = s->cW;
-      aa.cE = s->cE;
-      aa.cN = s->cN;
-      aa.cD = s->cD;
-      aa.csr_mass = s->csr_mass;
-      aa.csr_diag = s->csr_diag;
+      aa.cS = s->cset[set][0];
+      aa.cW = s->cset[set][1];
+      aa.cE = s->cset[set][2];
+      aa.cN = s->cset[set][3];
+      aa.cD = s->cset[set][4];
+      aa.csr_mass = s->csr_mass[set];
+      aa.csr_diag = s->csr_diag[set];
       aa.rhs_out = compat ? s->rhs_compat : nullptr;
       aa.fast = fast_patankar(s->p) ? 1 : 0;
       aa.inv_dx = 1.0 / s->gr.dx;
       aa.inv_dy = 1.0 / s->gr.dy;
-      // substep m's system: the first set, or for a fused iteration the m-th
-      double* sys[5] = {s->cS, s->cW, s->cE, s->cN, s->cD};
-      if (fuse_k && m > 2)
-        for (int c = 0; c < 5; ++c) sys[c] = s->cset[m - 3][c];
       if (!fuse_k) {
         NvtxRange r("patankar assembly");
         prof_mark(s, 1);
@@ -573,47 +595,41 @@ static int enqueue_patankar(swm_solver* s) {
           for (int r = 0; r < 4; ++r) ma.theta[q][r] = kTheta5[mq - 1][r];
           ma.hu_out[q] = s->hum[mq - 1];
           ma.hv_out[q] = s->hvm[mq - 1];
-          double* const* set = q == 0 ? nullptr : s->cset[q - 1];
-          ma.cS[q] = q == 0 ? s->cS : set[0];
-          ma.cW[q] = q == 0 ? s->cW : set[1];
-          ma.cE[q] = q == 0 ? s->cE : set[2];
-          ma.cN[q] = q == 0 ? s->cN : set[3];
-          ma.cD[q] = q == 0 ? s->cD : set[4];
+          ma.cS[q] = s->cset[q][0];
+          ma.cW[q] = s->cset[q][1];
+          ma.cE[q] = s->cset[q][2];
+          ma.cN[q] = s->cset[q][3];
+          ma.cD[q] = s->cset[q][4];
         }
         prof_mark(s, 1);
         CK(launch_assemble_multi(ma, s->stream));
         prof_mark(s, -1);
       }
-      JacobiArgs ja{};
-      ja.nx = s->nx;
-      ja.ny = s->ny;
-      ja.solve_idx = solve < kMaxSolves ? solve : kMaxSolves - 1;
-      ja.maxiter = s->p.jacobi_maxiter;
-      fill_thresh(s, ja.thresh);
-      ja.b = compat ? s->rhs_compat : s->h;
-      ja.cS = sys[0];
-      ja.cW = sys[1];
-      ja.cE = sys[2];
-      ja.cN = sys[3];
-      ja.cD = sys[4];
-      ja.rowstart = s->rowstart;
-      ja.cols = s->cols;
-      ja.mass = s->csr_mass;
-      ja.diag = s->csr_diag;
-      ja.xa = s->xa;
-      ja.xb = s->xb;
-      ja.out = last ? s->h : s->hbuf[m - 1][k & 1];
-      ja.ctl = s->ctl;
-      ja.block = jacobi_block_of(s->p);
-      ja.recip = fast_patankar(s->p) ? 1 : 0;
-      ja.spin_limit = s->spin_limit;
-      {
+      const int xs = group_k ? set : 0;
+      JacobiSys& y = ja.sys[ja.nsys++];
+      y.b = compat ? s->rhs_compat : s->h;
+      y.cS = s->cset[set][0];
+      y.cW = s->cset[set][1];
+      y.cE = s->cset[set][2];
+      y.cN = s->cset[set][3];
+      y.cD = s->cset[set][4];
+      y.mass = s->csr_mass[set];
+      y.diag = s->csr_diag[set];
+      y.xa = s->xa[xs];
+      y.xb = s->xb[xs];
+      y.out = last ? s->h : s->hbuf[m - 1][k & 1];
+      y.solve_idx = solve;
+      y.hint_idx = last_solve[m];
+      last_solve[m] = solve;
+      static_assert(13 <= kMaxSolves, "every solve of a step has its slot");
+      solve++;
+      if (!group_k || m == ms) {
         NvtxRange r("jacobi");
         prof_mark(s, 2);
-        CK(launch_jacobi(ja, csr, s->jac_blocks, s->stream));
+        CK(launch_jacobi(ja, s->jac_grid, s->stream));
         prof_mark(s, -1);
+        ja.nsys = 0;
       }
-      solve++;
     }
     if (k < kc) {  // RHS at Ua(m) (timediscretization.f90:550-557)
       for (int m = 2; m <= ms; ++m) {
@@ -749,23 +765,33 @@ int swm_create(const swm_params* p, swm_handle* out) {
     AL(s->fxm[r], nfx);
     AL(s->fym[r], nfy);
   }
+  s->grouped = p->timescheme == 5 && N <= kGroupCells;
+  const int nsets = s->grouped || (p->timescheme == 5 && fast_patankar(*p)) ? kMaxSys : 1;
+  // The first set's system and the iterates double as the staging arrays of
+  // swm_set_state / swm_get_state (a solve never runs beside those), so each is at least
+  // one ghosted array long.
+  const size_t ghosted = 3 * (nx + 6) * (ny + 6);
+  const size_t nx_it = s->grouped ? kMaxSys : 1;
+  AL(s->stage, std::max(2 * nx_it * N, ghosted));
+  for (size_t q = 0; q < nx_it; ++q) {
+    s->xa[q] = s->stage + 2 * q * N;
+    s->xb[q] = s->xa[q] + N;
+  }
+  AL(s->stage2, std::max(5 * N, ghosted));
+  for (int q = 0; q < nsets; ++q) {
+    double* sys = s->stage2;
+    if (q > 0) AL(sys, 5 * N);
+    if (csr) {
+      s->csr_mass[q] = sys;
+      AL(s->csr_diag[q], N);
+    } else {
+      for (int c = 0; c < 5; ++c) s->cset[q][c] = sys + c * N;
+    }
+  }
   if (csr) {
-    AL(s->csr_mass, 5 * N);
-    AL(s->csr_diag, N);
     AL(s->rowstart, N + 1);
     AL(s->cols, 5 * N);
-  } else {
-    AL(s->cS, N);
-    AL(s->cW, N);
-    AL(s->cE, N);
-    AL(s->cN, N);
-    AL(s->cD, N);
-    if (p->timescheme == 5 && fast_patankar(*p))
-      for (int q = 0; q < 2; ++q)
-        for (int c = 0; c < 5; ++c) AL(s->cset[q][c], N);
   }
-  AL(s->xa, N);
-  AL(s->xb, N);
   if ((p->timescheme == 7 || p->timescheme == 6) && p->mpdec2_compat) AL(s->rhs_compat, N);
   if (p->timescheme <= 4)
     for (int k = 0; k < 7; ++k)
@@ -780,8 +806,6 @@ int swm_create(const swm_params* p, swm_handle* out) {
   s->bad = reinterpret_cast<int*>(s->lam + 2);
   AL(s->ctl, 1);
   AL(s->summary, 2 + 512);
-  AL(s->stage, 3 * (nx + 6) * (ny + 6));
-  AL(s->stage2, 3 * (nx + 6) * (ny + 6));
 #undef AL
   if (lib_malloc_host((void**)&s->h_dt, sizeof(double)) != cudaSuccess ||
       lib_malloc_host((void**)&s->h_ctl, sizeof(JacobiCtl)) != cudaSuccess ||
@@ -849,8 +873,10 @@ int swm_create(const swm_params* p, swm_handle* out) {
         cudaSuccess)
       return cleanup(fail(SWM_ERR_CUDA, "bathymetry table upload failed"));
   }
-  s->jac_blocks = jacobi_grid_blocks(csr, jacobi_block_of(s->p), s->device, fast_patankar(s->p));
-  if (s->jac_blocks < 1) return cleanup(fail(SWM_ERR_CUDA, "Jacobi kernel cannot be resident"));
+  s->jac_grid = {jacobi_grid_blocks(jacobi_form(s->p), true, s->device),
+                 jacobi_grid_blocks(jacobi_form(s->p), false, s->device)};
+  if (s->jac_grid.tile_blocks < 1 || s->jac_grid.strip_blocks < 1)
+    return cleanup(fail(SWM_ERR_CUDA, "Jacobi kernel cannot be resident"));
   // the RHS kernels' shared-memory attribute is set on first launch
   if (cudaDeviceSynchronize() != cudaSuccess)
     return cleanup(fail(SWM_ERR_CUDA, "initialisation failed"));
@@ -1473,8 +1499,8 @@ int swm_debug_jacobi(swm_handle s, const double* mass, const double* diag, const
   double* out = s->hbuf[1][1];
   CK(cudaMemcpy(b, rhs, N * sizeof(double), cudaMemcpyHostToDevice));
   if (csr) {
-    CK(cudaMemcpy(s->csr_mass, mass, 5 * N * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(s->csr_diag, diag, N * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(s->csr_mass[0], mass, 5 * N * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(s->csr_diag[0], diag, N * sizeof(double), cudaMemcpyHostToDevice));
   } else {
     // the fast solver's planes hold the row divided by its Diagonal and rhs/Diagonal
     // (the fast assembly writes the same: products with RN(1/D))
@@ -1488,37 +1514,40 @@ int swm_debug_jacobi(swm_handle s, const double* mass, const double* diag, const
       pl[3 * N + k] = fast ? mass[5 * k + 4] * r : mass[5 * k + 4];
       pl[4 * N + k] = fast ? rhs[k] * r : diag[k];
     }
-    CK(cudaMemcpy(s->cS, pl.data(), N * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(s->cW, pl.data() + N, N * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(s->cE, pl.data() + 2 * N, N * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(s->cN, pl.data() + 3 * N, N * sizeof(double), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(s->cD, pl.data() + 4 * N, N * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(s->cset[0][0], pl.data(), N * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(s->cset[0][1], pl.data() + N, N * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(s->cset[0][2], pl.data() + 2 * N, N * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(s->cset[0][3], pl.data() + 3 * N, N * sizeof(double), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(s->cset[0][4], pl.data() + 4 * N, N * sizeof(double), cudaMemcpyHostToDevice));
   }
   CK(cudaMemset(s->ctl, 0, sizeof(JacobiCtl)));
-  JacobiArgs ja{};
+  JacobiGroup ja{};
   ja.nx = s->nx;
   ja.ny = s->ny;
-  ja.solve_idx = 0;
+  ja.nsys = 1;
   ja.maxiter = s->p.jacobi_maxiter;
+  ja.block = jacobi_block_of(s->p);
+  ja.form = jacobi_form(s->p);
   fill_thresh(s, ja.thresh);
-  ja.b = b;
-  ja.cS = s->cS;
-  ja.cW = s->cW;
-  ja.cE = s->cE;
-  ja.cN = s->cN;
-  ja.cD = s->cD;
   ja.rowstart = s->rowstart;
   ja.cols = s->cols;
-  ja.mass = s->csr_mass;
-  ja.diag = s->csr_diag;
-  ja.xa = s->xa;
-  ja.xb = s->xb;
-  ja.out = out;
   ja.ctl = s->ctl;
-  ja.block = jacobi_block_of(s->p);
-  ja.recip = fast_patankar(s->p) ? 1 : 0;
   ja.spin_limit = s->spin_limit;
-  CK(launch_jacobi(ja, csr, s->jac_blocks, s->stream));
+  JacobiSys& y = ja.sys[0];
+  y.b = b;
+  y.cS = s->cset[0][0];
+  y.cW = s->cset[0][1];
+  y.cE = s->cset[0][2];
+  y.cN = s->cset[0][3];
+  y.cD = s->cset[0][4];
+  y.mass = s->csr_mass[0];
+  y.diag = s->csr_diag[0];
+  y.xa = s->xa[0];
+  y.xb = s->xb[0];
+  y.out = out;
+  y.solve_idx = 0;
+  y.hint_idx = -1;
+  CK(launch_jacobi(ja, s->jac_grid, s->stream));
   CK(cudaStreamSynchronize(s->stream));
   CK(cudaMemcpy(sol, out, N * sizeof(double), cudaMemcpyDeviceToHost));
   JacobiCtl c;

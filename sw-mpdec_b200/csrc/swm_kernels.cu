@@ -11,6 +11,7 @@
 #include "../../include/swm.h"
 #include "swm_kernels.cuh"
 #include "swm_solve.cuh"
+#include "swm_strip.cuh"
 
 namespace swm {
 
@@ -288,223 +289,519 @@ cudaError_t launch_combo(const ComboArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// One CSR pass (one sweep): sparse_matmul (jacobi_iteration.f90:25-43) + update.
-__device__ void csr_pass(const JacobiArgs& a, const double* xin, double* xout, bool first,
-                         Acc& acc, unsigned long long (*s_acc)[3]) {
-  const int n = a.nx * a.ny;
-  const int stride = gridDim.x * blockDim.x;
-  // rows per thread between flushes of the part sums (every thread of the block
-  // takes part in a flush, so the count is the block's, not the thread's)
-  const long long rows_per_flush = (long long)kAccFlushCells * stride;
-  for (long long base = blockIdx.x * blockDim.x; base < n; base += rows_per_flush) {
-    if (base != blockIdx.x * blockDim.x) acc_reduce<1>(acc, s_acc);
-    const int end = (int)((n - base > rows_per_flush) ? base + rows_per_flush : n);
-    for (int row = (int)base + threadIdx.x; row < end; row += stride) {
-      double prod = 0.;
-      for (int sp = a.rowstart[row]; sp <= a.rowstart[row + 1] - 1; ++sp)
-        if (SWM_IN_RANGE(sp - 1, 5LL * n, kChkCsr) && SWM_IN_RANGE(a.cols[sp - 1] - 1, n, kChkCsr))
-          prod = __dadd_rn(prod, __dmul_rn(a.mass[sp - 1], __ldcg(&xin[a.cols[sp - 1] - 1])));
-      const double xv = __ddiv_rn(__dsub_rn(a.b[row], prod), a.diag[row]);
-      xout[row] = xv;
-      acc_put<1>(acc, fabs(__dsub_rn(xv, __ldcg(&xin[row]))));
-      if (first) acc_put<0>(acc, fabs(0. - a.b[row]));
+// ---------------------------------------------------------------------------
+// Jacobi on the systems of one grid: one cooperative launch, passes of up to T sweeps
+// (strip_chunk) separated by a bounded grid barrier; every CTA takes the same decisions
+// from the same sums.
+//
+// Stop rule: mean|x^{k+1} - x^k| <= tol after every sweep (jacobi_iteration.f90:71-81)
+// on the exact sum of |dx| rounded to multiples of 2^-100.  A pass sums |dx| in FP64, in
+// any order: n terms, so within n 2^-53 < 2^-24 of the sum of the unrounded terms, and
+// those are within n 2^-101 of the rounded ones.  Outside kBand of the threshold the
+// order therefore cannot change the decision; a sum inside the band (about one solve in
+// 10^5, or tol = 0) hands the system to solve_exact, which goes on from the pass's input
+// one sweep at a time with exact integer sums.  The iterates and the stop index depend
+// on neither tiling, launch shape nor atomic order.
+// ---------------------------------------------------------------------------
+constexpr double kBand = 0x1p-20;
+
+// Grid barrier number `nth` (1, 2, ..) of a launch on its own arrival counter (zero when
+// the launch starts), by one thread: everything its block wrote before a block barrier is
+// visible to every block after it.  The count only grows, so an arrival is one atomic and
+// a wait one polled word.  False when the wait gave up (status -4).
+__device__ __forceinline__ bool arrive_and_wait(unsigned int* ctr, unsigned int nth,
+                                                long long spin_limit, int* status) {
+  const unsigned int target = nth * gridDim.x;
+  __threadfence();
+  unsigned int c;
+  asm volatile("atom.add.acq_rel.gpu.u32 %0, [%1], 1;" : "=r"(c) : "l"(ctr) : "memory");
+  bool ok = true;
+  if (c + 1 != target) {
+    long long spins = 0;
+    for (;;) {
+      asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(c) : "l"(ctr) : "memory");
+      if (c >= target) break;
+      if (++spins > spin_limit || spin_limit <= 0) {
+        ok = false;
+        atomicExch(status, -4);
+        break;
+      }
     }
   }
+  __threadfence();
+  return ok;
 }
 
-template <int TB, bool CSR, bool RECIP>
-__global__ void __launch_bounds__(JNT, 2) jacobi_kernel(const JacobiArgs a) {
-  extern __shared__ __align__(16) double jsm[];
-  __shared__ unsigned long long s_acc[kMaxBlock + 1][3];
-  __shared__ unsigned long long s_tot[kMaxBlock + 1][3];
+// State of one system between passes, held identically by every CTA.
+struct SysState {
+  const double* xin;
+  double* xout;
+  int k;            // sweeps done
+  int Tp;           // sweeps of the coming pass
+  int active;       // still iterating
+  int first;        // the coming pass is the first
+  int rollback;     // the coming pass redoes the last one with Tp sweeps
+  int zero;         // converged before the first sweep: the reference returns 0
+  int maxhit;
+  int exact;        // a sum fell inside the band: solve_exact goes on from xin
+  float r_prev;     // residual sum of the last sweep of the previous pass (planning)
+};
+
+// 1 stop, 0 go on, -1 inside the band (NaN and infinite sums go on, as in exact sums).
+__device__ __forceinline__ int stop_decision(double s, double thresh, double n) {
+  const double slack = n * 0x1p-100;
+  if (!(s <= thresh * (1.0 + kBand) + slack)) return 0;
+  return s <= thresh * (1.0 - kBand) - slack ? 1 : -1;
+}
+
+// Sweeps of a pass when `left` more are expected: as few passes as blk allows, evenly.
+__device__ __forceinline__ int even_pass(int left, int blk) {
+  const int np = (left + blk - 1) / blk;
+  return np > 0 ? (left + np - 1) / np : blk;
+}
+
+// sum: the pass's residual sums; hint: sweeps of the same substep's previous solve, or 0.
+__device__ __forceinline__ void sys_decide(const JacobiGroup& a, const JacobiSys& y, SysState& S,
+                                           const double* sum, int hint, int blk, double thresh) {
+  const double n = (double)a.nx * a.ny;
+  if (S.rollback) {  // the redone pass delivered the final iterate
+    S.active = 0;
+    S.xin = S.xout;
+    return;
+  }
+  if (a.form != kSysRecip && !(sum[1] < 0.5 * kBadSum)) {
+    S.exact = 1;  // an operand the fast divisions do not take
+    S.active = 0;
+    return;
+  }
+  if (S.first) {
+    const int d = stop_decision(sum[0], thresh, n);
+    if (d != 0) {
+      S.active = 0;
+      if (d > 0)
+        S.zero = 1;
+      else
+        S.exact = 1;
+      return;
+    }
+  }
+  int stop = 0;
+  for (int t = 1; t <= S.Tp && stop == 0; ++t) {
+    const int d = stop_decision(sum[t], thresh, n);
+    if (d < 0) {
+      S.exact = 1;
+      S.active = 0;
+      return;
+    }
+    if (d > 0) stop = t;
+  }
+  S.first = 0;
+  if (stop > 0) {
+    S.k += stop;
+    if (stop < S.Tp) {  // the stop falls inside the pass: redo it with `stop` sweeps
+      S.rollback = 1;
+      S.Tp = stop;
+    } else {
+      S.active = 0;
+      S.xin = S.xout;
+    }
+    return;
+  }
+  S.k += S.Tp;
+  if (S.k >= a.maxiter) {
+    S.active = 0;
+    S.maxhit = 1;
+    S.xin = S.xout;
+    return;
+  }
+  // Sweeps still needed: from the hint while it holds, else from the decay of the last
+  // two sweeps.  Only pass lengths depend on it.
+  const float rT = (float)sum[S.Tp];
+  const float rP = S.Tp >= 2 ? (float)sum[S.Tp - 1] : S.r_prev;
+  S.r_prev = rT;
+  int left = blk + 1;  // unknown: a full pass
+  if (hint > S.k) {
+    left = hint - S.k;
+  } else if (rP > 0.f && rT > 0.f && rT < rP && thresh > 0.) {
+    const float need = __log2f((float)thresh / rT) / __log2f(rT / rP);
+    if (need > 0.f && need < 1000.f) left = (int)ceilf(need);
+  }
+  if (left < 1) left = 1;
+  int Tp = left > blk ? blk : left;
+  if (hint > S.k) Tp = even_pass(left, blk);
+  if (a.maxiter - S.k < Tp) Tp = a.maxiter - S.k;
+  S.Tp = Tp;
+  // the next pass writes the other ping-pong buffer or, when it is expected to be the
+  // last, the destination (unless that is the rhs or the pass's input)
+  S.xin = S.xout;
+  S.xout = (S.xin == y.xa) ? y.xb : y.xa;
+  if (left <= Tp && y.out != y.b && y.out != S.xin) S.xout = y.out;
+}
+
+// Work split of a pass over `nact` systems: chunks per strip so that the slowest warp's
+// rows (its chunks, each with 2 Tp rows of overlap) are fewest, for one to four chunks a
+// warp.  Called by a whole warp.
+__device__ __forceinline__ int strip_chunks(int nact, int strips, int ny, int Tp, int warps) {
+  const unsigned r = 1 + (threadIdx.x & 3), per = (unsigned)nact * strips;
+  const unsigned most = (ny + 3) / 4;
+  unsigned ch = r * warps / per;
+  ch = ch < 1 ? 1 : (ch > most ? most : ch);
+  const unsigned cost = ((per * ch + warps - 1) / warps) * ((ny + ch - 1) / ch + 2 * Tp);
+  unsigned best = cost, pick = ch;
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    const unsigned c2 = __shfl_xor_sync(0xffffffffu, best, o);
+    const unsigned h2 = __shfl_xor_sync(0xffffffffu, pick, o);
+    if (c2 < best || (c2 == best && h2 < pick)) {
+      best = c2;
+      pick = h2;
+    }
+  }
+  return (int)pick;
+}
+
+// One row of a system, the CSR rows through the pattern.
+template <int FORM>
+__device__ double row_update(const JacobiGroup& a, const JacobiSys& y, const double* xin, int row) {
+  double p = 0.;
+  if constexpr (FORM == kSysCsr) {
+    const int n = a.nx * a.ny;
+    for (int sp = a.rowstart[row]; sp <= a.rowstart[row + 1] - 1; ++sp)
+      if (SWM_IN_RANGE(sp - 1, 5LL * n, kChkCsr) && SWM_IN_RANGE(a.cols[sp - 1] - 1, n, kChkCsr))
+        p = __dadd_rn(p, __dmul_rn(y.mass[sp - 1], __ldcg(&xin[a.cols[sp - 1] - 1])));
+    return __ddiv_rn(__dsub_rn(y.b[row], p), y.diag[row]);
+  }
+  const int i = row % a.nx, j = row / a.nx, base = row - i;
+  const int im = i == 0 ? a.nx - 1 : i - 1, ip = i == a.nx - 1 ? 0 : i + 1;
+  const int jm = j == 0 ? a.ny - 1 : j - 1, jp = j == a.ny - 1 ? 0 : j + 1;
+  p = __dmul_rn(y.cS[row], __ldcg(&xin[jm * a.nx + i]));
+  p = __dadd_rn(p, __dmul_rn(y.cW[row], __ldcg(&xin[base + im])));
+  p = __dadd_rn(p, __dmul_rn(y.cE[row], __ldcg(&xin[base + ip])));
+  p = __dadd_rn(p, __dmul_rn(y.cN[row], __ldcg(&xin[jp * a.nx + i])));
+  if (FORM == kSysRecip) return __dsub_rn(y.cD[row], p);
+  return __ddiv_rn(__dsub_rn(y.b[row], p), y.cD[row]);
+}
+
+// The rest of a solve one sweep at a time, residuals summed exactly in integer limbs.
+// Returns false when a barrier wait gave up.
+template <int FORM>
+__device__ __noinline__ bool solve_exact(const JacobiGroup& a, const JacobiSys& y, SysState& S,
+                                         int* pass, unsigned int* nbar) {
+  __shared__ unsigned long long s_acc[2][3];
+  __shared__ unsigned long long s_tot[2][3];
   __shared__ int s_ok;
-  JacobiCtl* ctl = a.ctl;
-  int p = *((volatile int*)&ctl->pass_next);
-  const double* xin = a.b;
-  double* xout = a.xa;
-  const double* result = nullptr;
-  bool first = true, zero_result = false, maxhit = false;
-  int k = 0, final_k = 0;
-  const int blk = CSR ? 1 : (a.block < 1 ? 1 : (a.block > TB ? TB : a.block));
-  int plan = blk;            // sweeps of the next pass (plan_sweeps)
-  bool expect_stop = false;  // the residual decay reaches the threshold within it
-  double r_prev = -1.0;
-  const double thresh_d = limbs_value(a.thresh[0], a.thresh[1], a.thresh[2]);
-  Acc acc;
-  acc_zero(acc);
+  unsigned int* bar = &a.ctl->bar[a.sys[0].solve_idx];
+  const int n = a.nx * a.ny, stride = gridDim.x * blockDim.x;
+  const double* xin = S.xin;
+  int k = S.k, stop = -1;
+  const bool first0 = S.first != 0;
+  bool first = first0;
   for (;;) {
-    int Tp = plan;
-    if (a.maxiter - k < Tp) Tp = a.maxiter - k;
-    if (Tp < 1) Tp = 1;
-    for (int q = threadIdx.x; q < (kMaxBlock + 1) * 3; q += blockDim.x) (&s_acc[0][0])[q] = 0ull;
+    double* xout = (xin == y.xa) ? y.xb : y.xa;
+    if (threadIdx.x < 6) (&s_acc[0][0])[threadIdx.x] = 0ull;
     __syncthreads();
-    if (CSR)
-      csr_pass(a, xin, xout, first, acc, s_acc);
-    else
-      stencil_tiles<TB, RECIP, false>(a, xin, xout, Tp, first, acc, jsm, blockIdx.x, s_acc);
-    acc_reduce<TB>(acc, s_acc);
+    Acc acc;
+    acc_zero(acc);
+    int since = 0;
+    for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
+      if (++since > kAccFlushCells) {  // block-uniform
+        acc_reduce<1>(acc, s_acc);
+        since = 1;
+      }
+      const int row = base + threadIdx.x;
+      if (row < n) {
+        const double v = row_update<FORM>(a, y, xin, row);
+        xout[row] = v;
+        acc_put<1>(acc, fabs(__dsub_rn(v, __ldcg(&xin[row]))));
+        if (first) acc_put<0>(acc, fabs(0. - y.b[row]));
+      }
+    }
+    acc_reduce<1>(acc, s_acc);
     __syncthreads();
-    const int slot = p % kResSlots;
-    if (threadIdx.x < (Tp + 1) * 3) {
-      int t = threadIdx.x / 3, l = threadIdx.x % 3;
-      unsigned long long v = s_acc[t][l];
-      if (v) atomicAdd(&ctl->acc[slot][t][l], v);
+    const int slot = *pass % kResSlots;
+    if (threadIdx.x < 6) {
+      const unsigned long long v = (&s_acc[0][0])[threadIdx.x];
+      if (v) atomicAdd(&(&a.ctl->acc[slot][0][0])[threadIdx.x], v);
     }
-    if (!grid_barrier(ctl, a.spin_limit, &s_ok)) return;
-    if (threadIdx.x < (Tp + 1) * 3) {
-      int t = threadIdx.x / 3, l = threadIdx.x % 3;
-      s_tot[t][l] = __ldcg(&ctl->acc[slot][t][l]);
-    }
-    if (blockIdx.x == 0) {  // recycle the slot of pass p-1 (read by everyone before barrier p)
-      const int z = (p + 2) % kResSlots;
-      for (int q = threadIdx.x; q < (kMaxBlock + 1) * 3; q += blockDim.x)
-        (&ctl->acc[z][0][0])[q] = 0ull;
+    __syncthreads();
+    if (threadIdx.x == 0) s_ok = arrive_and_wait(bar, ++*nbar, a.spin_limit, &a.ctl->status);
+    __syncthreads();
+    if (!s_ok) return false;
+    if (threadIdx.x < 6) (&s_tot[0][0])[threadIdx.x] = __ldcg(&(&a.ctl->acc[slot][0][0])[threadIdx.x]);
+    if (blockIdx.x == 0 && threadIdx.x < 6) {
+      (&a.ctl->acc[(*pass + 2) % kResSlots][0][0])[threadIdx.x] = 0ull;
       __threadfence();
     }
     __syncthreads();
-    p++;
-    int stop = -1;
+    if (threadIdx.x == 0) ++*pass;
     if (first && limbs_le(s_tot[0][0], s_tot[0][1], s_tot[0][2], a.thresh)) {
       stop = 0;
-    } else {
-      for (int t = 1; t <= Tp; ++t)
-        if (limbs_le(s_tot[t][0], s_tot[t][1], s_tot[t][2], a.thresh)) {
-          stop = t;
-          break;
-        }
+      break;
     }
     first = false;
-    if (stop == 0) {
-      zero_result = true;
-      final_k = 0;
+    ++k;
+    xin = xout;
+    if (limbs_le(s_tot[1][0], s_tot[1][1], s_tot[1][2], a.thresh)) {
+      stop = k;
       break;
     }
-    if (stop > 0) {
-      final_k = k + stop;
-      if (stop < Tp && !CSR) {  // the stop falls inside the pass: redo it with `stop` sweeps
-        for (int q = threadIdx.x; q < (kMaxBlock + 1) * 3; q += blockDim.x)
-          (&s_acc[0][0])[q] = 0ull;
-        __syncthreads();
-        stencil_tiles<TB, RECIP, false>(a, xin, xout, stop, false, acc, jsm, blockIdx.x, s_acc);
-        acc_reduce<TB>(acc, s_acc);
-        if (!grid_barrier(ctl, a.spin_limit, &s_ok)) return;
-        if (blockIdx.x == 0) {
-          const int z = (p + 2) % kResSlots;
-          for (int q = threadIdx.x; q < (kMaxBlock + 1) * 3; q += blockDim.x)
-            (&ctl->acc[z][0][0])[q] = 0ull;
+    if (k >= a.maxiter) break;
+    __syncthreads();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    S.k = stop == 0 ? 0 : k;
+    S.xin = xin;
+    S.zero = stop == 0;
+    S.maxhit = stop < 0;
+  }
+  __syncthreads();
+  return true;
+}
+
+// TILES: a block per tile (small grids), else a warp per chunk of a strip.
+template <int FORM, bool TILES>
+__global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
+                                  TILES ? 1 : (FORM == kSysRecip ? 3 : 2))
+    jacobi_kernel(const __grid_constant__ JacobiGroup a) {
+  using G = Strip<FORM>;
+  using TG = Tile<FORM>;
+  constexpr int T = kPassT, NW = TILES ? kTileWarps : kStripWarps;
+  extern __shared__ __align__(16) unsigned char jring[];
+  __shared__ SysState st[kMaxSys];
+  __shared__ double s_sum[NW][kMaxSys][T + 1], s_tot[kMaxSys][T + 1];
+  __shared__ int s_ok, s_xpass, s_nact, s_ch, s_act[kMaxSys], s_hint[kMaxSys];
+  __shared__ unsigned int s_nbar;
+  JacobiCtl* ctl = a.ctl;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int blk = a.block < 1 ? 1 : (a.block > T ? T : a.block);
+  const double thresh = limbs_value(a.thresh[0], a.thresh[1], a.thresh[2]);
+  const int strips = (a.nx + G::U - 1) / G::U, warps = gridDim.x * kStripWarps;
+  const int tiles = TILES ? strips * ((a.ny + TG::UY - 1) / TG::UY) : 0;
+  static_assert(G::U == TG::UX, "strips and tiles deliver the same columns");
+  double2* ring = reinterpret_cast<double2*>(jring + (TILES ? 0 : warp * G::warp_bytes));
+  // the systems still iterating and the pass's split, by warp 0
+  auto plan = [&]() {
+    int na = 0, most = 0;
+    for (int q = 0; q < a.nsys; ++q)
+      if (st[q].active) {
+        if (lane == 0) s_act[na] = q;
+        ++na;
+        most = max(most, st[q].Tp);
+      }
+    const int ch = !TILES && na ? strip_chunks(na, strips, a.ny, most, warps) : 1;
+    if (lane == 0) {
+      s_nact = na;
+      s_ch = ch;
+    }
+  };
+  int pass = 0;  // warp 0: position in the ring of sums
+  if (warp == 0) {
+    pass = *((volatile int*)&ctl->pass_next);
+    if (lane < a.nsys) {
+      const JacobiSys& y = a.sys[lane];
+      SysState& S = st[lane];
+      const int hint = y.hint_idx >= 0 ? __ldcg(&ctl->iters[y.hint_idx]) : 0;
+      s_hint[lane] = hint;
+      S.Tp = hint > 0 ? even_pass(hint, blk) : blk;
+      if (S.Tp > a.maxiter) S.Tp = a.maxiter;
+      S.xin = y.b;
+      S.xout = (hint > 0 && hint <= S.Tp && y.out != y.b) ? y.out : y.xa;
+      S.k = 0;
+      S.active = 1;
+      S.first = 1;
+      S.rollback = S.zero = S.maxhit = S.exact = 0;
+      S.r_prev = -1.f;
+    }
+    if (lane == 0) {
+      s_xpass = *((volatile int*)&ctl->exact_next);
+      s_nbar = 0;
+      s_ok = 1;
+    }
+    __syncwarp();
+    plan();
+  }
+  __syncthreads();
+  StripRow<FORM> cf[TILES ? TG::RW : 1];  // tiles: the rows held, of tile `held`
+  int held = -1;
+  bool held_bad = false;
+  while (s_nact > 0) {
+    for (int q = lane; q < kMaxSys * (T + 1); q += 32) (&s_sum[warp][0][0])[q] = 0.;
+    __syncwarp();
+    const int nact = s_nact;
+    auto flush = [&](int q, int Tp, double (&sum)[T + 1]) {
+#pragma unroll
+      for (int t = 0; t <= T; ++t) {
+        if (t > Tp) break;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum[t] += __shfl_down_sync(0xffffffffu, sum[t], o);
+        if (lane == 0) s_sum[warp][q][t] += sum[t];
+      }
+    };
+    auto aligned = [&](const JacobiSys& y, const SysState& S) {
+      unsigned long long al = (unsigned long long)S.xin | (unsigned long long)S.xout |
+                              (unsigned long long)y.b;
+      if constexpr (FORM == kSysCsr)
+        al |= (unsigned long long)y.mass | (unsigned long long)y.diag;
+      else
+        al |= (unsigned long long)y.cS | (unsigned long long)y.cW | (unsigned long long)y.cE |
+              (unsigned long long)y.cN | (unsigned long long)y.cD;
+      return (al & 15ull) == 0;
+    };
+    if constexpr (TILES) {
+      for (int it = blockIdx.x; it < nact * tiles; it += gridDim.x) {
+        const int q = s_act[it / tiles], tile = it % tiles;
+        const JacobiSys& y = a.sys[q];
+        const SysState& S = st[q];
+        const int Tp = S.Tp, strip = tile % strips, j0 = (tile / strips) * TG::UY;
+        const StripLane L = strip_lane<FORM>(a.nx, a.nx, strip, aligned(y, S));
+        if (held != q * tiles + tile) {  // a block with one tile keeps its rows of the system
+          held = q * tiles + tile;
+          held_bad = false;
+          tile_rows<FORM>(y, a.nx, a.ny, a.nx, wrap(j0 + warp * TG::RW - T, a.ny), L, cf, held_bad);
+        }
+        double sum[T + 1];
+        tile_pass<FORM>(S.xin, S.xout, a.nx, a.ny, a.nx, Tp, S.first != 0, j0, L, cf, held_bad,
+                        ring, sum);
+        flush(q, Tp, sum);
+        __syncthreads();  // the edge rows are read
+      }
+    } else {
+      const int ch = s_ch, R = (a.ny + ch - 1) / ch, items = nact * strips * ch;
+      // items in (system, chunk, strip) order over all CTAs first, so that few items
+      // spread over many SMs and neighbouring strips stream together
+      for (int it = warp * gridDim.x + blockIdx.x; it < items; it += warps) {
+        const int strip = it % strips, rest = it / strips;
+        const int q = s_act[rest / ch], j0 = (rest % ch) * R, rows = min(R, a.ny - j0);
+        if (rows <= 0) continue;
+        const JacobiSys& y = a.sys[q];
+        const SysState& S = st[q];
+        const int Tp = S.Tp;
+        double sum[T + 1];
+        strip_pass<FORM>(y, S.xin, S.xout, a.nx, a.ny, a.nx, a.nx, Tp, S.first != 0, strip, j0,
+                         rows, aligned(y, S), ring, sum);
+        flush(q, Tp, sum);
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      // the block's sums, the grid barrier, then every block's decisions from the totals
+      const int slot = pass % kResSlots;
+      static_assert(kMaxSys * (T + 1) <= 32, "a lane per sum");
+      const int q = lane / (T + 1), t = lane % (T + 1);
+      const bool mine = q < a.nsys && st[q < kMaxSys ? q : 0].active;
+      if (mine) {
+        double v = s_sum[0][q][t];
+        for (int w = 1; w < NW; ++w) v += s_sum[w][q][t];
+        if (v != 0.) atomicAdd(&ctl->sum[slot][q][t], v);
+      }
+      __syncwarp();
+      if (lane == 0)
+        s_ok = arrive_and_wait(&ctl->bar[a.sys[0].solve_idx], ++s_nbar, a.spin_limit, &ctl->status);
+      __syncwarp();
+      if (s_ok) {
+        if (mine) s_tot[q][t] = __ldcg(&ctl->sum[slot][q][t]);
+        if (blockIdx.x == 0) {  // recycle the slot of the pass before this one
+          for (int z = lane; z < kMaxSys * (kMaxBlock + 1); z += 32)
+            (&ctl->sum[(pass + 2) % kResSlots][0][0])[z] = 0.;
           __threadfence();
         }
-        p++;
+        __syncwarp();
+        if (lane < a.nsys && st[lane].active)
+          sys_decide(a, a.sys[lane], st[lane], s_tot[lane], s_hint[lane], blk, thresh);
+        __syncwarp();
+        plan();
+        ++pass;
       }
-      result = xout;
-      break;
     }
-    if (!CSR) {
-      const double rT = limbs_value(s_tot[Tp][0], s_tot[Tp][1], s_tot[Tp][2]);
-      const double rP =
-          Tp >= 2 ? limbs_value(s_tot[Tp - 1][0], s_tot[Tp - 1][1], s_tot[Tp - 1][2]) : r_prev;
-      r_prev = rT;
-      plan = plan_sweeps(rT, rP, thresh_d, blk);
-      expect_stop = rP > 0. && rT > 0. && rT < rP && thresh_d > 0. &&
-                    log(thresh_d / rT) / log(rT / rP) <= (double)blk;
-    }
-    k += Tp;
-    if (k >= a.maxiter) {
-      final_k = k;
-      maxhit = true;
-      result = xout;
-      break;
-    }
-    // the next pass writes the other ping-pong buffer, or, when it is expected to be
-    // the last, the destination itself (unless that is the rhs or holds xin), which
-    // saves copying the result there
-    xin = xout;
-    xout = (xin == a.xa) ? a.xb : a.xa;
-    if (expect_stop && a.out != a.b && a.out != xin) xout = a.out;
+    __syncthreads();
+    if (!s_ok) return;
   }
-  // deliver the final iterate (haVec of the reference) to its destination
+  for (int q = 0; q < a.nsys; ++q)
+    if (st[q].exact && !solve_exact<FORM>(a, a.sys[q], st[q], &s_xpass, &s_nbar)) return;
+  // deliver the final iterates (haVec of the reference) to their destinations
   const int n = a.nx * a.ny;
-  if (zero_result || result != a.out) {
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x)
-      a.out[q] = zero_result ? 0. : __ldcg(&result[q]);
+  for (int q = 0; q < a.nsys; ++q) {
+    const JacobiSys& y = a.sys[q];
+    if (!st[q].zero && st[q].xin == y.out) continue;
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
+      y.out[c] = st[q].zero ? 0. : __ldcg(&st[q].xin[c]);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    ctl->iters[a.solve_idx] = final_k;
-    if (maxhit && ctl->status == 0) ctl->status = 1;
-    *((volatile int*)&ctl->pass_next) = p;
+  if (blockIdx.x == 0 && threadIdx.x < a.nsys) {
+    const SysState& S = st[threadIdx.x];
+    ctl->iters[a.sys[threadIdx.x].solve_idx] = S.zero ? 0 : S.k;
+    if (S.maxhit) atomicCAS(&ctl->status, 0, 1);
+    if (threadIdx.x == 0) {
+      *((volatile int*)&ctl->pass_next) = pass;
+      *((volatile int*)&ctl->exact_next) = s_xpass;
+    }
   }
 }
 
-template <int TB, bool CSR, bool RECIP>
-static const void* jacobi_fn() {
-  return reinterpret_cast<const void*>(&jacobi_kernel<TB, CSR, RECIP>);
+struct JacobiLaunch {
+  const void* fn;
+  int threads, width, height;  // cells one block (tiles) or one chunk of a strip delivers
+  size_t smem;
+};
+
+template <int FORM>
+static JacobiLaunch jacobi_launch_of(bool tiles) {
+  if (tiles)
+    return {reinterpret_cast<const void*>(&jacobi_kernel<FORM, true>), kTileNT, Tile<FORM>::UX,
+            Tile<FORM>::UY, Tile<FORM>::bytes};
+  return {reinterpret_cast<const void*>(&jacobi_kernel<FORM, false>), kStripNT, Strip<FORM>::U, 8,
+          Strip<FORM>::bytes};
 }
 
-template <bool RECIP>
-static const void* pick_stencil(int block, size_t* smem) {
-  if (block <= 1) {
-    *smem = JTile<1>::bytes;
-    return jacobi_fn<1, false, RECIP>();
-  }
-  if (block <= 2) {
-    *smem = JTile<2>::bytes;
-    return jacobi_fn<2, false, RECIP>();
-  }
-  if (block <= 4) {
-    *smem = JTile<4>::bytes;
-    return jacobi_fn<4, false, RECIP>();
-  }
-  *smem = JTile<8>::bytes;
-  return jacobi_fn<8, false, RECIP>();
+static JacobiLaunch jacobi_pick(int form, bool tiles) {
+  if (form == kSysRecip) return jacobi_launch_of<kSysRecip>(tiles);
+  return form == kSysDiv ? jacobi_launch_of<kSysDiv>(tiles) : jacobi_launch_of<kSysCsr>(tiles);
 }
 
-static const void* pick_jacobi(bool csr, int block, bool recip, size_t* smem) {
-  if (csr) {
-    *smem = 0;
-    return jacobi_fn<1, true, false>();
-  }
-  return recip ? pick_stencil<true>(block, smem) : pick_stencil<false>(block, smem);
-}
-
-int jacobi_grid_blocks(bool csr, int block, int device, bool recip) {
-  size_t smem = 0;
-  const void* fn = pick_jacobi(csr, block, recip, &smem);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, JNT, smem) != cudaSuccess)
+int jacobi_grid_blocks(int form, bool tiles, int device) {
+  const JacobiLaunch l = jacobi_pick(form, tiles);
+  int per_sm = 0, sms = 0;
+  cudaFuncSetAttribute(l.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, l.fn, l.threads, l.smem) !=
+      cudaSuccess)
     return -1;
-  int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  if (per_sm < 1) return -1;
-  return per_sm * sms;
+  return per_sm < 1 ? -1 : per_sm * sms;
 }
 
-cudaError_t launch_jacobi(const JacobiArgs& a, bool csr, int grid_blocks, cudaStream_t s) {
-  size_t smem = 0;
-  const void* fn = pick_jacobi(csr, a.block, a.recip != 0, &smem);
-  int n = a.nx * a.ny;
-  int blocks = grid_blocks;
-  if (csr) {
-    int need = (n + JNT - 1) / JNT;
-    if (need < blocks) blocks = need;
-  } else {
-    int tiles = ((a.nx + JBX - 1) / JBX) * ((a.ny + JBY - 1) / JBY);
-    if (tiles < blocks) blocks = tiles;
+// Tiles while they make at most kTileWaves rounds over the resident blocks, strips beyond.
+// Measured per step (13 solves of 10 to 14 sweeps, B200), tiles against strips: split
+// 256^2 182 / 266 us, 512^2 (300 tiles of a launch's three systems over 148 blocks) 315 /
+// 346, 768^2 (630 tiles) 553 / 479, 2048^2 2675 / 1920; FP64 512^2 (390 tiles) 393 / 458,
+// 768^2 (840 tiles) 745 / 635.
+constexpr int kTileWaves = 3;
+
+cudaError_t launch_jacobi(const JacobiGroup& a, const JacobiGrid& g, cudaStream_t s) {
+  JacobiLaunch l = jacobi_pick(a.form, true);
+  const long long tiles = (long long)a.nsys * ((a.nx + l.width - 1) / l.width) *
+                          ((a.ny + l.height - 1) / l.height);
+  long long blocks = tiles, most = g.tile_blocks;
+  if (tiles > (long long)kTileWaves * g.tile_blocks) {
+    l = jacobi_pick(a.form, false);
+    // no more blocks than chunks of `height` rows give work to
+    const long long items = (long long)a.nsys * ((a.nx + l.width - 1) / l.width) *
+                            ((a.ny + l.height - 1) / l.height);
+    blocks = (items + kStripWarps - 1) / kStripWarps;
+    most = g.strip_blocks;
   }
-  if (blocks < 1) blocks = 1;
+  if (blocks > most) blocks = most;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(JNT);
-  cfg.dynamicSmemBytes = smem;
+  cfg.gridDim = dim3((unsigned)(blocks < 1 ? 1 : blocks));
+  cfg.blockDim = dim3(l.threads);
+  cfg.dynamicSmemBytes = l.smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  void* args[] = {const_cast<JacobiArgs*>(&a)};
-  return cudaLaunchKernelExC(&cfg, fn, args);
+  void* args[] = {const_cast<JacobiGroup*>(&a)};
+  return cudaLaunchKernelExC(&cfg, l.fn, args);
 }
 
 template <int TB, bool RECIP>

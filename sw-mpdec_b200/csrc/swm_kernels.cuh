@@ -19,13 +19,25 @@ constexpr int kMaxSolves = 16;  // solves recorded per step
 // A limit <= 0 makes every wait that is not already open give up at once.
 constexpr long long kDefaultSpinLimit = 1LL << 26;
 
+// Independent systems of one grid solved together by one launch: the three substeps of a
+// correction iteration.
+constexpr int kMaxSys = 3;
+
+// How a system is stored: planes holding the row divided by its Diagonal and b/Diagonal
+// (split and FMA forms), planes and Diagonal (FP64 form), or the reference's CSR values
+// Mass[5N] in slot order S, W, C, E, N (finitevolume.f90:234-261) and Diagonal.
+enum { kSysRecip = 0, kSysDiv = 1, kSysCsr = 2 };
+
 struct JacobiCtl {
-  unsigned long long acc[kResSlots][kMaxBlock + 1][3];  // [slot][0 = initial, 1..T sweeps][limb]
-  unsigned int bar_count;
-  unsigned int bar_gen;
+  // ring of passes: residual sums of every system, [0] initial, [1..] per sweep
+  double sum[kResSlots][kMaxSys][kMaxBlock + 1];
+  // ring of exact passes (one sweep each): limbs of the initial residual and the sweep's
+  unsigned long long acc[kResSlots][2][3];
+  unsigned int bar[kMaxSolves];  // barrier arrivals of the launch whose first solve it is
   int iters[kMaxSolves];  // iterations of each solve of the current step
   int status;             // 0 ok, 1 maxiter, -4 watchdog
-  int pass_next;          // pass counter carried across solves (slot ring position)
+  int pass_next;          // pass counter carried across solves (sum ring position)
+  int exact_next;         // the same of exact passes (acc ring position)
 };
 
 struct AssembleArgs {
@@ -94,18 +106,39 @@ struct JacobiArgs {
   const double* cE;
   const double* cN;
   const double* cD;
-  // CSR
-  const int* rowstart;    // 1-based (finitevolume.f90:230,267)
-  const int* cols;        // 1-based
-  const double* mass;
+  double* xa;             // ping-pong buffers
+  double* xb;
+  double* out;            // final iterate destination
+};
+
+// One system of a JacobiGroup.
+struct JacobiSys {
+  const double* b;        // rhs (= hp(1) = h^n)
+  const double* cS;       // stencil planes (see JacobiArgs)
+  const double* cW;
+  const double* cE;
+  const double* cN;
+  const double* cD;
+  const double* mass;     // CSR values, Mass[5N] and Diagonal
   const double* diag;
   double* xa;             // ping-pong buffers
   double* xb;
   double* out;            // final iterate destination
+  int solve_idx;          // slot in ctl->iters
+  int hint_idx;           // slot of an earlier solve of this step whose sweep count plans
+                          // the passes (the same substep's previous correction); < 0 none
+};
+struct JacobiGroup {
+  int nx, ny, nsys;
+  int maxiter;
+  int block;              // sweeps per pass at most
+  int form;               // kSysRecip, kSysDiv, kSysCsr (swm_strip.cuh)
+  unsigned long long thresh[3];  // tol * n in residual units (limbs)
+  const int* rowstart;    // CSR pattern, 1-based (finitevolume.f90:230,267)
+  const int* cols;
   JacobiCtl* ctl;
-  int block;              // sweeps per pass (stencil)
-  int recip;              // stencil (split form): S..N hold Mass/Diagonal, cD holds b/Diagonal
   long long spin_limit;   // grid-barrier watchdog
+  JacobiSys sys[kMaxSys];
 };
 
 struct DtArgs {
@@ -241,8 +274,12 @@ size_t rhs_smem_bytes(int mode);
 cudaError_t launch_dt(const DtArgs& a, cudaStream_t s);
 cudaError_t launch_assemble(const AssembleArgs& a, bool csr, cudaStream_t s);
 cudaError_t launch_assemble_multi(const AssembleMultiArgs& a, cudaStream_t s);
-cudaError_t launch_jacobi(const JacobiArgs& a, bool csr, int grid_blocks, cudaStream_t s);
-int jacobi_grid_blocks(bool csr, int block, int device, bool recip = false);
+// Resident blocks of the Jacobi kernel's two forms (swm_strip.cuh).
+struct JacobiGrid {
+  int tile_blocks, strip_blocks;
+};
+cudaError_t launch_jacobi(const JacobiGroup& a, const JacobiGrid& g, cudaStream_t s);
+int jacobi_grid_blocks(int form, bool tiles, int device);
 cudaError_t launch_ghosted_to_planes(const double* G, int nx, int ny, double* h, double* hu,
                                      double* hv, cudaStream_t s);
 cudaError_t launch_planes_to_ghosted(const double* h, const double* hu, const double* hv, int nx,

@@ -17,7 +17,7 @@
 
 namespace {
 
-using swm::JacobiArgs;
+using swm::JacobiGroup;
 using swm::JacobiCtl;
 
 constexpr size_t kNoAllocMaxCells = size_t(1) << 20;  // 1,048,576 cells, e.g. 1024 x 1024
@@ -32,7 +32,7 @@ static __device__ __align__(256) double g_jacobi_scratch[kNoAllocMaxCells + kCtl
 struct DeviceSetup {
   bool ready = false;
   double* scratch = nullptr;  // device address of g_jacobi_scratch on that device
-  int blocks[swm::kMaxBlock + 1] = {};
+  swm::JacobiGrid grid{};     // resident CTAs of the kernel
 };
 DeviceSetup g_setup[kMaxDevices];
 std::mutex g_setup_mutex;
@@ -102,10 +102,12 @@ int swm_jacobi_noalloc(int nx, int ny, const double* cS, const double* cW, const
       ds.scratch = static_cast<double*>(p);
       ds.ready = true;
     }
-    if (ds.blocks[block] == 0) {
-      int nb = swm::jacobi_grid_blocks(false, block, dev);
-      if (nb < 1) return noalloc_fail(SWM_ERR_CUDA, "Jacobi kernel cannot be resident");
-      ds.blocks[block] = nb;
+    if (ds.grid.strip_blocks == 0) {
+      const swm::JacobiGrid g{swm::jacobi_grid_blocks(swm::kSysDiv, true, dev),
+                              swm::jacobi_grid_blocks(swm::kSysDiv, false, dev)};
+      if (g.tile_blocks < 1 || g.strip_blocks < 1)
+        return noalloc_fail(SWM_ERR_CUDA, "Jacobi kernel cannot be resident");
+      ds.grid = g;
     }
   }
   const DeviceSetup& ds = g_setup[dev];
@@ -116,25 +118,29 @@ int swm_jacobi_noalloc(int nx, int ny, const double* cS, const double* cW, const
   cudaError_t e = cudaMemsetAsync(ctl, 0, sizeof(JacobiCtl), st);
   if (e != cudaSuccess) return noalloc_fail(SWM_ERR_CUDA, cudaGetErrorString(e));
 
-  JacobiArgs ja{};
+  JacobiGroup ja{};
   ja.nx = nx;
   ja.ny = ny;
-  ja.solve_idx = 0;
+  ja.nsys = 1;
   ja.maxiter = maxiter;
-  swm::residual_limbs_host(tol * (double)nx * (double)ny, ja.thresh);
-  ja.b = rhs;
-  ja.cS = cS;
-  ja.cW = cW;
-  ja.cE = cE;
-  ja.cN = cN;
-  ja.cD = cD;
-  ja.xa = ds.scratch;  // second iterate buffer from the static scratch
-  ja.xb = sol;         // the caller's output doubles as the first
-  ja.out = sol;
-  ja.ctl = ctl;
   ja.block = block;
+  ja.form = swm::kSysDiv;
+  swm::residual_limbs_host(tol * (double)nx * (double)ny, ja.thresh);
+  ja.ctl = ctl;
   ja.spin_limit = swm::kDefaultSpinLimit;
-  e = swm::launch_jacobi(ja, false, ds.blocks[block], st);
+  swm::JacobiSys& y = ja.sys[0];
+  y.b = rhs;
+  y.cS = cS;
+  y.cW = cW;
+  y.cE = cE;
+  y.cN = cN;
+  y.cD = cD;
+  y.xa = ds.scratch;  // second iterate buffer from the static scratch
+  y.xb = sol;         // the caller's output doubles as the first
+  y.out = sol;
+  y.solve_idx = 0;
+  y.hint_idx = -1;
+  e = swm::launch_jacobi(ja, ds.grid, st);
   if (e != cudaSuccess) return noalloc_fail(SWM_ERR_CUDA, cudaGetErrorString(e));
   int res[2] = {0, 0};  // iters[0], status
   e = cudaMemcpyAsync(&res[0], &ctl->iters[0], sizeof(int), cudaMemcpyDeviceToHost, st);
