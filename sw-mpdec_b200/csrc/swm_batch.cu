@@ -1,17 +1,14 @@
 // swm_batch.cu -- ensembles of independent problems on uneven grids.
 //
-// A whole mPDeC5 step of every problem is one cooperative persistent launch (the
-// ensemble step kernel, swm_ensemble.cuh): per-problem TimeStep, the RHS of every
-// (problem, tile), and per correction the assembly of its three substeps into three
-// independent Patankar systems per problem and one batched Jacobi solve of all of
-// them, each system with its own stop rule, phases separated by bounded grid
-// barriers.  The step (three memsets and that launch) is captured once into a CUDA
-// graph.  jacobi_block = 0 lets the first step time the candidate schedules -- Jacobi
-// temporal block (sweeps per pass, which sets the haloed tile shape 64+2T x 16+2T)
-// and CTAs per SM -- on the initial state and keep the fastest (results do not depend
-// on it: every candidate produces the same iterates).  The earlier form, one launch
-// per phase (40 per step), stays selectable for comparison
-// (swm_batch_debug_set_launches).
+// A whole mPDeC5 step of every problem is captured once into a CUDA graph, in one of two
+// forms with identical results: one cooperative persistent launch (the ensemble step
+// kernel, swm_ensemble.cuh), or a kernel per phase (TimeStep, the RHS of every (problem,
+// tile), and per correction the assembly of its three substeps into three independent
+// Patankar systems per problem and one batched solve of all of them by strips, each
+// system with its own stop rule).  jacobi_block = 0 lets the first step time the
+// candidate schedules -- the step form, Jacobi sweeps per pass and, for the persistent
+// form, CTAs per SM -- on the initial state and keep the fastest.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -43,7 +40,7 @@ int bfail(int code, const std::string& msg) {
 
 const int kSolves = 13;    // mPDeC5: 3 substeps x 4 corrections + 1
 const int kRhsSets = 7;    // U^n, and Ua(m) for m = 2..4 at both correction parities
-const int kCandidates[3] = {2, 4, 8};
+const int kCandidates[3] = {4, 2, 8};
 const int kSubsteps = 3;   // systems per problem solved together (substeps m = 2..4)
 
 struct BProblem {
@@ -111,7 +108,12 @@ struct swm_batch {
   JacBatchState* d_st = nullptr;
   JacBatchCtl* d_ctl = nullptr;
   int* d_iters = nullptr;          // [kSolves][n]
-  int jac_blocks[9] = {};
+  // per-phase form: chunks of strips, their systems' states, the solves' control block
+  int4* d_items = nullptr;
+  int nitems = 0;
+  StripBatchState* d_sst = nullptr;
+  StripBatchCtl* d_sctl = nullptr;
+  int jac_blocks = 0;
   cudaGraphExec_t graph = nullptr;
   // host mirrors
   std::vector<double> h_dt;
@@ -357,7 +359,8 @@ static int batch_enqueue_phases(swm_batch* b, int block, cudaEvent_t* marks = nu
     return marks ? cudaEventRecord(marks[mk++], b->stream) : cudaSuccess;
   };
   BCK(mark());
-  BCK(cudaMemsetAsync(b->d_ctl, 0, sizeof(JacBatchCtl), b->stream));
+  BCK(cudaMemsetAsync(b->d_sctl, 0, sizeof(StripBatchCtl), b->stream));
+  BCK(cudaMemsetAsync(b->d_sst, 0, sizeof(StripBatchState) * kSubsteps * b->n, b->stream));
   BCK(launch_dt_batch(b->d_dtd, b->d_cells, b->ncellblk, b->n, b->d_lam, b->d_bad, b->d_dt,
                       b->stream));
   BCK(mark());
@@ -375,19 +378,22 @@ static int batch_enqueue_phases(swm_batch* b, int block, cudaEvent_t* marks = nu
                                   b->ncellblk, b->fast, b->stream));
     }
     BCK(mark());
-    JacobiBatchArgs ja{};
+    StripBatchArgs ja{};
     ja.descs = b->d_jac5 + (size_t)(k - 1) * kSubsteps * b->n;
-    ja.tiles = b->d_tiles;
-    ja.ntiles = b->ntiles;
+    ja.items = b->d_items;
+    ja.nitems = b->nitems;
     ja.nprob = b->n;
     ja.nsets = nsub;
-    ja.st = b->d_st;
-    ja.ctl = b->d_ctl;
+    ja.correction = k - 1;
+    ja.st = b->d_sst;
+    ja.ctl = b->d_sctl;
     ja.iters = b->d_iters + (size_t)solve * b->n;
+    // the same substeps' previous solves: three back, and for the last correction's one
+    // system (substep 4) one back
+    ja.hint = k == 1 ? nullptr : ja.iters - (size_t)(k == 5 ? 1 : kSubsteps) * b->n;
     ja.block = block;
     ja.spin_limit = b->spin_limit;
-    ja.work = b->d_work + 10;  // reset by the solve itself
-    BCK(launch_jacobi_batch(ja, b->jac_blocks[block], b->fast, b->stream));
+    BCK(launch_jacobi_batch(ja, b->jac_blocks, b->fast, b->stream));
     BCK(mark());
     solve += nsub;
     if (k < 5) {
@@ -492,10 +498,10 @@ static int batch_copy_state(swm_batch* b, bool to_save) {
 
 // Autotuner: time one step per candidate schedule on the initial state, restore the
 // state after each, keep the fastest.  Candidates: the step form (the persistent launch,
-// or a kernel per phase, unless the caller fixed it), the Jacobi temporal block 2, 4, 8
-// (the haloed tile of a pass is 64+2T x 16+2T cells) and, for the persistent step, the
-// co-resident grid or half of it (one CTA per SM instead of two).  Every schedule gives
-// the same results.
+// or a kernel per phase, unless the caller fixed it), the Jacobi sweeps per pass (2, 4 or
+// 8 in the persistent form, whose haloed tile is 64+2T x 16+2T cells; 2 or 4 by strips)
+// and, for the persistent step, the co-resident grid or half of it (one CTA per SM
+// instead of two).  Every schedule gives the same results.
 static int batch_tune(swm_batch* b) {
   NvtxRange range("ensemble autotune");
   for (auto& q : b->pr)
@@ -512,13 +518,12 @@ static int batch_tune(swm_batch* b) {
     bool persistent;
     int block, grid;
   };
-  std::vector<Cand> cands;
-  for (int form = 0; form < 2; ++form) {
-    const bool pers = form == 0;
+  std::vector<Cand> cands;  // each form's usually best schedule first
+  for (bool pers : {false, true}) {
     if (b->mode_fixed && pers != b->persistent) continue;
     for (int c : kCandidates) {
-      if (!pers) {
-        cands.push_back({false, c, 0});
+      if (!pers) {  // the strips sweep at most 4 times per pass
+        if (c <= 4) cands.push_back({false, c, 0});
         continue;
       }
       cands.push_back({true, c, b->ens_max[c]});
@@ -530,7 +535,12 @@ static int batch_tune(swm_batch* b) {
   BCK(cudaEventCreate(&e1));
   float best = 1e30f;
   Cand pick = cands[0];
+  // A form whose first schedule takes a fifth longer than the best so far is not tried
+  // further (256-problem split ensemble: 42 ms a step per phase, 60 ms for the persistent
+  // form's best schedule): the trials are paid by the first step.
+  bool skip[2] = {false, false};
   for (const auto& c : cands) {
+    if (skip[c.persistent]) continue;
     for (int rep = 0; rep < 2; ++rep) {  // first repetition warms the kernels
       BCK(cudaEventRecord(e0, b->stream));
       if ((rc = batch_enqueue(b, c.persistent, c.block, c.grid))) return rc;
@@ -540,6 +550,7 @@ static int batch_tune(swm_batch* b) {
     }
     float ms = 0.f;
     BCK(cudaEventElapsedTime(&ms, e0, e1));
+    if (ms > 1.2f * best) skip[c.persistent] = true;
     if (ms < best) {
       best = ms;
       pick = c;
@@ -647,10 +658,31 @@ int swm_batch_create(int n, const swm_params* p, swm_batch_handle* out) {
       cudaMemcpy(b->d_dtd, dd.data(), sizeof(DtBatchDesc) * n, cudaMemcpyHostToDevice))
     return cleanup(bfail(SWM_ERR_CUDA, "table upload failed"));
   if ((rc = batch_tables(b))) return cleanup(rc);
-  for (int c = 1; c <= kMaxBlock; c *= 2) {
-    b->jac_blocks[c] = jacobi_batch_grid_blocks(c, b->device, b->fast);
-    if (b->jac_blocks[c] < 1) return cleanup(bfail(SWM_ERR_CUDA, "Jacobi kernel cannot be resident"));
+  b->jac_blocks = jacobi_batch_grid_blocks(b->device, b->fast);
+  if (b->jac_blocks < 1) return cleanup(bfail(SWM_ERR_CUDA, "Jacobi kernel cannot be resident"));
+  // Chunks of the batched solves: rows so that one correction's three systems give every
+  // resident warp about one chunk, within 8 (the 2 x 4 rows of overlap) and 32 rows.  A
+  // large ensemble has several chunks per warp, and its last passes few systems: on the
+  // 256-problem split ensemble a step's solves took 10.4 / 9.9 / 10.7 / 13.2 / 17.2 ms with
+  // at most 16 / 32 / 64 / 128 / 256 rows.
+  long long rows_all = 0;
+  for (const BProblem& q : b->pr) rows_all += (long long)kSubsteps * jacobi_batch_strips(q.nx) * q.ny;
+  const long long warps = (long long)b->jac_blocks * kJacobiBatchWarps;
+  const int most = (int)std::min(32LL, std::max(8LL, (rows_all + warps - 1) / warps + 1));
+  std::vector<int4> items;
+  for (int i = 0; i < n; ++i) {
+    const BProblem& q = b->pr[i];
+    const int ch = (q.ny + most - 1) / most, rows = (q.ny + ch - 1) / ch;
+    for (int j0 = 0; j0 < q.ny; j0 += rows)
+      for (int st = 0; st < jacobi_batch_strips(q.nx); ++st)
+        items.push_back(make_int4(i, st, j0, std::min(rows, q.ny - j0)));
   }
+  b->nitems = (int)items.size();
+  if ((rc = b->alloc(&b->d_items, items.size())) ||
+      (rc = b->alloc(&b->d_sst, (size_t)kSubsteps * n)) || (rc = b->alloc(&b->d_sctl, 1)))
+    return cleanup(rc);
+  if (cudaMemcpy(b->d_items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice))
+    return cleanup(bfail(SWM_ERR_CUDA, "table upload failed"));
   // co-resident CTAs of the ensemble step kernel per temporal block (cooperative launch)
   for (int c = 2; c <= kMaxBlock; c *= 2) {
     const void* fn = ens_kernel(b, c);
@@ -707,20 +739,21 @@ int swm_batch_step(swm_batch_handle b, double* dt_out) {
   if (b->autotune && (rc = batch_tune(b))) return rc;
   if ((rc = batch_graph(b))) return rc;
   BCK(cudaGraphLaunch(b->graph, b->stream));
-  JacBatchCtl ctl;
+  int status = 0;
+  const int* d_status = b->persistent ? &b->d_ctl->status : &b->d_sctl->status;
   BCK(cudaMemcpyAsync(b->h_dt.data(), b->d_dt, sizeof(double) * b->n, cudaMemcpyDeviceToHost, b->stream));
   BCK(cudaMemcpyAsync(b->h_iters.data(), b->d_iters, sizeof(int) * b->h_iters.size(),
                       cudaMemcpyDeviceToHost, b->stream));
   BCK(cudaMemcpyAsync(b->h_bad.data(), b->d_bad, sizeof(int) * b->n, cudaMemcpyDeviceToHost, b->stream));
-  BCK(cudaMemcpyAsync(&ctl, b->d_ctl, sizeof(JacBatchCtl), cudaMemcpyDeviceToHost, b->stream));
+  BCK(cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
   BCK(cudaStreamSynchronize(b->stream));
   if (dt_out)
     for (int i = 0; i < b->n; ++i) dt_out[i] = b->h_dt[i];
   for (int v : b->h_iters) b->iters_total += v;
   for (int v : b->h_bad)
     if (v) return bfail(SWM_ERR_NAN, "non-finite or negative depth in an ensemble member");
-  if (ctl.status < 0) return bfail(SWM_ERR_WATCHDOG, "Jacobi grid barrier watchdog expired");
-  if (ctl.status == 1) return SWM_WARN_JACOBI_MAXITER;
+  if (status < 0) return bfail(SWM_ERR_WATCHDOG, "Jacobi grid barrier watchdog expired");
+  if (status == 1) return SWM_WARN_JACOBI_MAXITER;
   return SWM_OK;
 }
 

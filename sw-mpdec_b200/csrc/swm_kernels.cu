@@ -332,21 +332,6 @@ __device__ __forceinline__ bool arrive_and_wait(unsigned int* ctr, unsigned int 
   return ok;
 }
 
-// State of one system between passes, held identically by every CTA.
-struct SysState {
-  const double* xin;
-  double* xout;
-  int k;            // sweeps done
-  int Tp;           // sweeps of the coming pass
-  int active;       // still iterating
-  int first;        // the coming pass is the first
-  int rollback;     // the coming pass redoes the last one with Tp sweeps
-  int zero;         // converged before the first sweep: the reference returns 0
-  int maxhit;
-  int exact;        // a sum fell inside the band: solve_exact goes on from xin
-  float r_prev;     // residual sum of the last sweep of the previous pass (planning)
-};
-
 // 1 stop, 0 go on, -1 inside the band (NaN and infinite sums go on, as in exact sums).
 __device__ __forceinline__ int stop_decision(double s, double thresh, double n) {
   const double slack = n * 0x1p-100;
@@ -360,16 +345,19 @@ __device__ __forceinline__ int even_pass(int left, int blk) {
   return np > 0 ? (left + np - 1) / np : blk;
 }
 
-// sum: the pass's residual sums; hint: sweeps of the same substep's previous solve, or 0.
-__device__ __forceinline__ void sys_decide(const JacobiGroup& a, const JacobiSys& y, SysState& S,
-                                           const double* sum, int hint, int blk, double thresh) {
-  const double n = (double)a.nx * a.ny;
+// What a pass's outcome means for a system.  n: its cells; sum: the pass's residual
+// sums; hint: sweeps of the same substep's previous solve, or 0; out: the destination, or
+// b where a pass must not write it directly.
+template <bool RECIP>
+__device__ __forceinline__ void sys_decide(SysState& S, double n, int maxiter, double thresh,
+                                           const double* b, double* xa, double* xb, double* out,
+                                           const double* sum, int hint, int blk) {
   if (S.rollback) {  // the redone pass delivered the final iterate
     S.active = 0;
     S.xin = S.xout;
     return;
   }
-  if (a.form != kSysRecip && !(sum[1] < 0.5 * kBadSum)) {
+  if (!RECIP && !(sum[1] < 0.5 * kBadSum)) {
     S.exact = 1;  // an operand the fast divisions do not take
     S.active = 0;
     return;
@@ -408,7 +396,7 @@ __device__ __forceinline__ void sys_decide(const JacobiGroup& a, const JacobiSys
     return;
   }
   S.k += S.Tp;
-  if (S.k >= a.maxiter) {
+  if (S.k >= maxiter) {
     S.active = 0;
     S.maxhit = 1;
     S.xin = S.xout;
@@ -429,13 +417,30 @@ __device__ __forceinline__ void sys_decide(const JacobiGroup& a, const JacobiSys
   if (left < 1) left = 1;
   int Tp = left > blk ? blk : left;
   if (hint > S.k) Tp = even_pass(left, blk);
-  if (a.maxiter - S.k < Tp) Tp = a.maxiter - S.k;
+  if (maxiter - S.k < Tp) Tp = maxiter - S.k;
   S.Tp = Tp;
   // the next pass writes the other ping-pong buffer or, when it is expected to be the
   // last, the destination (unless that is the rhs or the pass's input)
   S.xin = S.xout;
-  S.xout = (S.xin == y.xa) ? y.xb : y.xa;
-  if (left <= Tp && y.out != y.b && y.out != S.xin) S.xout = y.out;
+  S.xout = (S.xin == xa) ? xb : xa;
+  if (left <= Tp && out != b && out != S.xin) S.xout = out;
+}
+
+
+// A system's first pass.
+__device__ __forceinline__ SysState sys_start(int maxiter, const double* b, double* xa, double* out,
+                                              int hint, int blk) {
+  SysState S;
+  S.Tp = hint > 0 ? even_pass(hint, blk) : blk;
+  if (S.Tp > maxiter) S.Tp = maxiter;
+  S.xin = b;
+  S.xout = (hint > 0 && hint <= S.Tp && out != b) ? out : xa;
+  S.k = 0;
+  S.active = 1;
+  S.first = 1;
+  S.rollback = S.zero = S.maxhit = S.exact = 0;
+  S.r_prev = -1.f;
+  return S;
 }
 
 // Work split of a pass over `nact` systems: chunks per strip so that the slowest warp's
@@ -460,42 +465,58 @@ __device__ __forceinline__ int strip_chunks(int nact, int strips, int ny, int Tp
   return (int)pick;
 }
 
-// One row of a system, the CSR rows through the pattern.
-template <int FORM>
-__device__ double row_update(const JacobiGroup& a, const JacobiSys& y, const double* xin, int row) {
+// What solve_exact needs of a grid and its system's arrays.
+struct ExactGrid {
+  int nx, ny, pitch, maxiter;
+  const unsigned long long* thresh;
+  const int* rowstart;  // CSR pattern, 1-based
+  const int* cols;
+  unsigned long long (*acc)[2][3];  // ring of limb sums, zero between solves' passes
+  unsigned int* bar;
+  int* status;
+  long long spin_limit;
+};
+
+// One cell of a system, the CSR rows through the pattern.
+template <int FORM, typename Sys>
+__device__ __forceinline__ double cell_update(const ExactGrid& g, const Sys& y, const double* xin,
+                                              int i, int j) {
   double p = 0.;
   if constexpr (FORM == kSysCsr) {
-    const int n = a.nx * a.ny;
-    for (int sp = a.rowstart[row]; sp <= a.rowstart[row + 1] - 1; ++sp)
-      if (SWM_IN_RANGE(sp - 1, 5LL * n, kChkCsr) && SWM_IN_RANGE(a.cols[sp - 1] - 1, n, kChkCsr))
-        p = __dadd_rn(p, __dmul_rn(y.mass[sp - 1], __ldcg(&xin[a.cols[sp - 1] - 1])));
+    const int n = g.nx * g.ny, row = j * g.nx + i;
+    for (int sp = g.rowstart[row]; sp <= g.rowstart[row + 1] - 1; ++sp)
+      if (SWM_IN_RANGE(sp - 1, 5LL * n, kChkCsr) && SWM_IN_RANGE(g.cols[sp - 1] - 1, n, kChkCsr))
+        p = __dadd_rn(p, __dmul_rn(y.mass[sp - 1], __ldcg(&xin[g.cols[sp - 1] - 1])));
     return __ddiv_rn(__dsub_rn(y.b[row], p), y.diag[row]);
+  } else {
+    const int im = i == 0 ? g.nx - 1 : i - 1, ip = i == g.nx - 1 ? 0 : i + 1;
+    const int jm = j == 0 ? g.ny - 1 : j - 1, jp = j == g.ny - 1 ? 0 : j + 1;
+    const size_t r = (size_t)j * g.pitch, c = r + i;
+    p = __dmul_rn(y.cS[c], __ldcg(&xin[(size_t)jm * g.pitch + i]));
+    p = __dadd_rn(p, __dmul_rn(y.cW[c], __ldcg(&xin[r + im])));
+    p = __dadd_rn(p, __dmul_rn(y.cE[c], __ldcg(&xin[r + ip])));
+    p = __dadd_rn(p, __dmul_rn(y.cN[c], __ldcg(&xin[(size_t)jp * g.pitch + i])));
+    if constexpr (FORM == kSysRecip)
+      return __dsub_rn(y.cD[c], p);
+    else
+      return __ddiv_rn(__dsub_rn(y.b[c], p), y.cD[c]);
   }
-  const int i = row % a.nx, j = row / a.nx, base = row - i;
-  const int im = i == 0 ? a.nx - 1 : i - 1, ip = i == a.nx - 1 ? 0 : i + 1;
-  const int jm = j == 0 ? a.ny - 1 : j - 1, jp = j == a.ny - 1 ? 0 : j + 1;
-  p = __dmul_rn(y.cS[row], __ldcg(&xin[jm * a.nx + i]));
-  p = __dadd_rn(p, __dmul_rn(y.cW[row], __ldcg(&xin[base + im])));
-  p = __dadd_rn(p, __dmul_rn(y.cE[row], __ldcg(&xin[base + ip])));
-  p = __dadd_rn(p, __dmul_rn(y.cN[row], __ldcg(&xin[jp * a.nx + i])));
-  if (FORM == kSysRecip) return __dsub_rn(y.cD[row], p);
-  return __ddiv_rn(__dsub_rn(y.b[row], p), y.cD[row]);
 }
 
-// The rest of a solve one sweep at a time, residuals summed exactly in integer limbs.
-// Returns false when a barrier wait gave up.
-template <int FORM>
-__device__ __noinline__ bool solve_exact(const JacobiGroup& a, const JacobiSys& y, SysState& S,
-                                         int* pass, unsigned int* nbar) {
+// The rest of a solve one sweep at a time with IEEE divisions, residuals summed exactly
+// in integer limbs; every block of the grid takes part.  pass, nbar: the block's position
+// in the ring of limb sums and its count of grid barriers (shared memory).  Returns false
+// when a barrier wait gave up.
+template <int FORM, typename Sys>
+__device__ __noinline__ bool solve_exact(const ExactGrid& g, const Sys& y, SysState& S, int* pass,
+                                         unsigned int* nbar) {
   __shared__ unsigned long long s_acc[2][3];
   __shared__ unsigned long long s_tot[2][3];
   __shared__ int s_ok;
-  unsigned int* bar = &a.ctl->bar[a.sys[0].solve_idx];
-  const int n = a.nx * a.ny, stride = gridDim.x * blockDim.x;
+  const int n = g.nx * g.ny, stride = gridDim.x * blockDim.x;
   const double* xin = S.xin;
   int k = S.k, stop = -1;
-  const bool first0 = S.first != 0;
-  bool first = first0;
+  bool first = S.first != 0;
   for (;;) {
     double* xout = (xin == y.xa) ? y.xb : y.xa;
     if (threadIdx.x < 6) (&s_acc[0][0])[threadIdx.x] = 0ull;
@@ -508,12 +529,14 @@ __device__ __noinline__ bool solve_exact(const JacobiGroup& a, const JacobiSys& 
         acc_reduce<1>(acc, s_acc);
         since = 1;
       }
-      const int row = base + threadIdx.x;
-      if (row < n) {
-        const double v = row_update<FORM>(a, y, xin, row);
-        xout[row] = v;
-        acc_put<1>(acc, fabs(__dsub_rn(v, __ldcg(&xin[row]))));
-        if (first) acc_put<0>(acc, fabs(0. - y.b[row]));
+      const int cell = base + threadIdx.x;
+      if (cell < n) {
+        const int i = cell % g.nx, j = cell / g.nx;
+        const size_t c = (size_t)j * g.pitch + i;
+        const double v = cell_update<FORM>(g, y, xin, i, j);
+        xout[c] = v;
+        acc_put<1>(acc, fabs(__dsub_rn(v, __ldcg(&xin[c]))));
+        if (first) acc_put<0>(acc, fabs(0. - y.b[c]));
       }
     }
     acc_reduce<1>(acc, s_acc);
@@ -521,31 +544,31 @@ __device__ __noinline__ bool solve_exact(const JacobiGroup& a, const JacobiSys& 
     const int slot = *pass % kResSlots;
     if (threadIdx.x < 6) {
       const unsigned long long v = (&s_acc[0][0])[threadIdx.x];
-      if (v) atomicAdd(&(&a.ctl->acc[slot][0][0])[threadIdx.x], v);
+      if (v) atomicAdd(&(&g.acc[slot][0][0])[threadIdx.x], v);
     }
     __syncthreads();
-    if (threadIdx.x == 0) s_ok = arrive_and_wait(bar, ++*nbar, a.spin_limit, &a.ctl->status);
+    if (threadIdx.x == 0) s_ok = arrive_and_wait(g.bar, ++*nbar, g.spin_limit, g.status);
     __syncthreads();
     if (!s_ok) return false;
-    if (threadIdx.x < 6) (&s_tot[0][0])[threadIdx.x] = __ldcg(&(&a.ctl->acc[slot][0][0])[threadIdx.x]);
+    if (threadIdx.x < 6) (&s_tot[0][0])[threadIdx.x] = __ldcg(&(&g.acc[slot][0][0])[threadIdx.x]);
     if (blockIdx.x == 0 && threadIdx.x < 6) {
-      (&a.ctl->acc[(*pass + 2) % kResSlots][0][0])[threadIdx.x] = 0ull;
+      (&g.acc[(*pass + 2) % kResSlots][0][0])[threadIdx.x] = 0ull;
       __threadfence();
     }
     __syncthreads();
     if (threadIdx.x == 0) ++*pass;
-    if (first && limbs_le(s_tot[0][0], s_tot[0][1], s_tot[0][2], a.thresh)) {
+    if (first && limbs_le(s_tot[0][0], s_tot[0][1], s_tot[0][2], g.thresh)) {
       stop = 0;
       break;
     }
     first = false;
     ++k;
     xin = xout;
-    if (limbs_le(s_tot[1][0], s_tot[1][1], s_tot[1][2], a.thresh)) {
+    if (limbs_le(s_tot[1][0], s_tot[1][1], s_tot[1][2], g.thresh)) {
       stop = k;
       break;
     }
-    if (k >= a.maxiter) break;
+    if (k >= g.maxiter) break;
     __syncthreads();
   }
   __syncthreads();
@@ -600,18 +623,9 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
     pass = *((volatile int*)&ctl->pass_next);
     if (lane < a.nsys) {
       const JacobiSys& y = a.sys[lane];
-      SysState& S = st[lane];
       const int hint = y.hint_idx >= 0 ? __ldcg(&ctl->iters[y.hint_idx]) : 0;
       s_hint[lane] = hint;
-      S.Tp = hint > 0 ? even_pass(hint, blk) : blk;
-      if (S.Tp > a.maxiter) S.Tp = a.maxiter;
-      S.xin = y.b;
-      S.xout = (hint > 0 && hint <= S.Tp && y.out != y.b) ? y.out : y.xa;
-      S.k = 0;
-      S.active = 1;
-      S.first = 1;
-      S.rollback = S.zero = S.maxhit = S.exact = 0;
-      S.r_prev = -1.f;
+      st[lane] = sys_start(a.maxiter, y.b, y.xa, y.out, hint, blk);
     }
     if (lane == 0) {
       s_xpass = *((volatile int*)&ctl->exact_next);
@@ -707,8 +721,11 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
           __threadfence();
         }
         __syncwarp();
-        if (lane < a.nsys && st[lane].active)
-          sys_decide(a, a.sys[lane], st[lane], s_tot[lane], s_hint[lane], blk, thresh);
+        if (lane < a.nsys && st[lane].active) {
+          const JacobiSys& y = a.sys[lane];
+          sys_decide<FORM == kSysRecip>(st[lane], (double)a.nx * a.ny, a.maxiter, thresh, y.b, y.xa,
+                                        y.xb, y.out, s_tot[lane], s_hint[lane], blk);
+        }
         __syncwarp();
         plan();
         ++pass;
@@ -717,8 +734,10 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
     __syncthreads();
     if (!s_ok) return;
   }
+  const ExactGrid eg{a.nx,   a.ny,     a.nx,       a.maxiter, a.thresh, a.rowstart, a.cols,
+                     ctl->acc, &ctl->bar[a.sys[0].solve_idx], &ctl->status, a.spin_limit};
   for (int q = 0; q < a.nsys; ++q)
-    if (st[q].exact && !solve_exact<FORM>(a, a.sys[q], st[q], &s_xpass, &s_nbar)) return;
+    if (st[q].exact && !solve_exact<FORM>(eg, a.sys[q], st[q], &s_xpass, &s_nbar)) return;
   // deliver the final iterates (haVec of the reference) to their destinations
   const int n = a.nx * a.ny;
   for (int q = 0; q < a.nsys; ++q) {
@@ -804,60 +823,203 @@ cudaError_t launch_jacobi(const JacobiGroup& a, const JacobiGrid& g, cudaStream_
   return cudaLaunchKernelExC(&cfg, l.fn, args);
 }
 
-template <int TB, bool RECIP>
-__global__ void __launch_bounds__(JNT, 2) jacobi_batch_kernel(const JacobiBatchArgs a) {
-  extern __shared__ __align__(16) double jsm[];
-  jacobi_batch_solve<TB, RECIP>(a, jsm);
+// Ensembles: one cooperative launch solves a.nsets x a.nprob systems of any sizes, each
+// with its own stop rule, by strips.  A pass visits the chunks of every system still
+// iterating (a warp takes its first by its number, the others from a counter whose next
+// value it fetches while it works); then each block decides for its share of the systems.
+template <int FORM>
+__global__ void __launch_bounds__(kStripNT, FORM == kSysRecip ? 3 : 2)
+    jacobi_batch_kernel(const StripBatchArgs a) {
+  constexpr int T = kPassT;
+  static_assert(T + 1 <= kBatchSums, "sums of a pass");
+  constexpr bool RECIP = FORM == kSysRecip;
+  extern __shared__ __align__(16) unsigned char jring[];
+  __shared__ int s_ok, s_xpass, s_nact, s_nexact;
+  __shared__ unsigned int s_nbar;
+  __shared__ SysState s_st;
+  __shared__ __align__(16) JacobiArgs s_d;
+  StripBatchCtl* ctl = a.ctl;
+  unsigned int* bar = &ctl->bar[a.correction];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int blk = a.block < 1 ? 1 : (a.block > T ? T : a.block);
+  const int warps = gridDim.x * kStripWarps, me = warp * gridDim.x + blockIdx.x;
+  const int nsys = a.nsets * a.nprob, nwork = a.nsets * a.nitems;
+  double2* ring = reinterpret_cast<double2*>(jring + warp * Strip<FORM>::warp_bytes);
+  if (threadIdx.x == 0) {
+    s_nbar = 0;
+    s_xpass = *((volatile int*)&ctl->exact_next);
+  }
+  auto direct = [](const JacobiArgs& d) {  // where a pass may write the destination
+    return d.pitch == d.nx ? d.out : const_cast<double*>(d.b);
+  };
+  auto start = [&](const JacobiArgs& d, int sys) {
+    return sys_start(d.maxiter, d.b, d.xa, direct(d), a.hint ? __ldg(&a.hint[sys]) : 0, blk);
+  };
+  __syncthreads();
+  for (int pass = 0;; ++pass) {
+    for (int w = me; w < nwork;) {
+      unsigned int nw = 0;
+      if (lane == 0) nw = (unsigned int)warps + atomicAdd(&ctl->work, 1u);
+      const int set = w / a.nitems;
+      const int4 it = a.items[w - set * a.nitems];
+      const int sys = set * a.nprob + it.x;
+      const JacobiArgs& d = a.descs[sys];
+      int Tp, first, active = 1;
+      const double* xin;
+      double* xout;
+      if (pass == 0) {  // the states are written by the first decisions
+        const SysState S = start(d, sys);
+        Tp = S.Tp;
+        first = 1;
+        xin = S.xin;
+        xout = S.xout;
+      } else {
+        const SysState* S = &a.st[sys].s;
+        active = __ldcg(&S->active);
+        Tp = __ldcg(&S->Tp);
+        first = __ldcg(&S->first);
+        xin = reinterpret_cast<const double*>(__ldcg(reinterpret_cast<const unsigned long long*>(&S->xin)));
+        xout = reinterpret_cast<double*>(__ldcg(reinterpret_cast<const unsigned long long*>(&S->xout)));
+      }
+      if (active && SWM_IN_RANGE(it.x, a.nprob, kChkEnsItem)) {
+        const int nx = d.nx, ny = d.ny, pitch = d.pitch;
+        const unsigned long long al =
+            (unsigned long long)xin | (unsigned long long)xout | (unsigned long long)d.b |
+            (unsigned long long)d.cS | (unsigned long long)d.cW | (unsigned long long)d.cE |
+            (unsigned long long)d.cN | (unsigned long long)d.cD;
+        double sum[T + 1];
+        strip_pass<FORM>(d, xin, xout, nx, ny, pitch, pitch, Tp, first != 0, it.y, it.z, it.w,
+                         (al & 15ull) == 0, ring, sum);
+#pragma unroll
+        for (int t = 0; t <= T; ++t) {
+          if (t > Tp) break;
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) sum[t] += __shfl_xor_sync(0xffffffffu, sum[t], o);
+          if (lane == t && sum[t] != 0.) atomicAdd(&a.st[sys].sum[t], sum[t]);
+        }
+      }
+      w = (int)__shfl_sync(0xffffffffu, nw, 0);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) s_ok = arrive_and_wait(bar, ++s_nbar, a.spin_limit, &ctl->status);
+    __syncthreads();
+    if (!s_ok) return;
+    // decisions: system p by thread p / gridDim.x of block p % gridDim.x
+    for (int p = blockIdx.x + gridDim.x * threadIdx.x; p < nsys; p += gridDim.x * blockDim.x) {
+      const JacobiArgs& d = a.descs[p];
+      StripBatchState& B = a.st[p];
+      SysState S = pass == 0 ? start(d, p) : B.s;
+      if (!S.active) continue;
+      double sum[T + 1];
+#pragma unroll
+      for (int t = 0; t <= T; ++t) {
+        sum[t] = __ldcg(&B.sum[t]);
+        B.sum[t] = 0.;
+      }
+      const double thresh = limbs_value(d.thresh[0], d.thresh[1], d.thresh[2]);
+      sys_decide<RECIP>(S, (double)d.nx * d.ny, d.maxiter, thresh, d.b, d.xa, d.xb, direct(d), sum,
+                        a.hint ? __ldg(&a.hint[p]) : 0, blk);
+      B.s = S;
+      if (S.active) atomicAdd(&ctl->nact[pass % 3], 1);
+      if (S.exact) atomicAdd(&ctl->nexact, 1);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      ctl->work = 0u;
+      ctl->nact[(pass + 1) % 3] = 0;  // read by everyone before the barrier above
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s_ok = arrive_and_wait(bar, ++s_nbar, a.spin_limit, &ctl->status);
+      s_nact = __ldcg(&ctl->nact[pass % 3]);
+      s_nexact = __ldcg(&ctl->nexact);
+    }
+    __syncthreads();
+    if (!s_ok) return;
+    if (s_nact == 0) break;
+  }
+  if (blockIdx.x == 0 && threadIdx.x < 3) ctl->nact[threadIdx.x] = 0;  // the next launch's
+  if (s_nexact > 0) {
+    for (int p = 0; p < nsys; ++p) {
+      if (!__ldcg(&a.st[p].s.exact)) continue;
+      if (threadIdx.x == 0) {
+        s_st = a.st[p].s;
+        s_d = a.descs[p];
+      }
+      __syncthreads();
+      const ExactGrid eg{s_d.nx,  s_d.ny,  s_d.pitch, s_d.maxiter,  s_d.thresh,   nullptr,
+                         nullptr, ctl->acc, bar,       &ctl->status, a.spin_limit};
+      if (!solve_exact<FORM>(eg, s_d, s_st, &s_xpass, &s_nbar)) return;
+      if (blockIdx.x == 0 && threadIdx.x == 0) {
+        s_st.exact = 0;
+        a.st[p].s = s_st;
+      }
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) s_ok = arrive_and_wait(bar, ++s_nbar, a.spin_limit, &ctl->status);
+    __syncthreads();
+    if (!s_ok) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      ctl->nexact = 0;
+      *((volatile int*)&ctl->exact_next) = s_xpass;
+    }
+  }
+  // deliver the iterates that the last pass did not write to their destinations, chunk by
+  // chunk, and the sweep counts
+  for (int w = me; w < nwork; w += warps) {
+    const int set = w / a.nitems;
+    const int4 it = a.items[w - set * a.nitems];
+    const int sys = set * a.nprob + it.x;
+    const JacobiArgs& d = a.descs[sys];
+    const SysState* S = &a.st[sys].s;
+    const double* x =
+        reinterpret_cast<const double*>(__ldcg(reinterpret_cast<const unsigned long long*>(&S->xin)));
+    const int zero = __ldcg(&S->zero);
+    if (!zero && x == d.out) continue;
+    const int i0 = it.y * Strip<FORM>::U, i1 = min(i0 + Strip<FORM>::U, d.nx);
+    for (int j = it.z; j < it.z + it.w; ++j)
+      for (int i = i0 + lane; i < i1; i += 32)
+        d.out[(size_t)j * d.nx + i] = zero ? 0. : __ldcg(&x[(size_t)j * d.pitch + i]);
+  }
+  for (int p = blockIdx.x + gridDim.x * threadIdx.x; p < nsys; p += gridDim.x * blockDim.x) {
+    const SysState* S = &a.st[p].s;
+    a.iters[p] = __ldcg(&S->zero) ? 0 : __ldcg(&S->k);
+    if (__ldcg(&S->maxhit)) atomicCAS(&ctl->status, 0, 1);
+  }
 }
 
-template <bool RECIP>
-static const void* pick_batch(int block, size_t* smem) {
-  if (block <= 1) {
-    *smem = JTile<1>::bytes;
-    return reinterpret_cast<const void*>(&jacobi_batch_kernel<1, RECIP>);
-  }
-  if (block <= 2) {
-    *smem = JTile<2>::bytes;
-    return reinterpret_cast<const void*>(&jacobi_batch_kernel<2, RECIP>);
-  }
-  if (block <= 4) {
-    *smem = JTile<4>::bytes;
-    return reinterpret_cast<const void*>(&jacobi_batch_kernel<4, RECIP>);
-  }
-  *smem = JTile<8>::bytes;
-  return reinterpret_cast<const void*>(&jacobi_batch_kernel<8, RECIP>);
+static const void* batch_fn(bool recip) {
+  return recip ? reinterpret_cast<const void*>(&jacobi_batch_kernel<kSysRecip>)
+               : reinterpret_cast<const void*>(&jacobi_batch_kernel<kSysDiv>);
 }
 
-int jacobi_batch_grid_blocks(int block, int device, bool recip) {
-  size_t smem = 0;
-  const void* fn = recip ? pick_batch<true>(block, &smem) : pick_batch<false>(block, &smem);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+int jacobi_batch_strips(int nx) { return (nx + Strip<kSysDiv>::U - 1) / Strip<kSysDiv>::U; }
+
+int jacobi_batch_grid_blocks(int device, bool recip) {
+  const size_t smem = recip ? Strip<kSysRecip>::bytes : Strip<kSysDiv>::bytes;
+  const void* fn = batch_fn(recip);
   int per_sm = 0, sms = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, JNT, smem) != cudaSuccess)
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kStripNT, smem) != cudaSuccess)
     return -1;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   return per_sm < 1 ? -1 : per_sm * sms;
 }
 
-cudaError_t launch_jacobi_batch(const JacobiBatchArgs& a, int grid_blocks, bool recip,
+cudaError_t launch_jacobi_batch(const StripBatchArgs& a, int grid_blocks, bool recip,
                                 cudaStream_t s) {
-  size_t smem = 0;
-  const void* fn = recip ? pick_batch<true>(a.block, &smem) : pick_batch<false>(a.block, &smem);
-  int blocks = grid_blocks < a.ntiles ? grid_blocks : a.ntiles;
-  if (blocks < 1) blocks = 1;
+  const long long need = ((long long)a.nsets * a.nitems + kStripWarps - 1) / kStripWarps;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(JNT);
-  cfg.dynamicSmemBytes = smem;
+  cfg.gridDim = dim3((unsigned)(need < grid_blocks ? (need < 1 ? 1 : need) : grid_blocks));
+  cfg.blockDim = dim3(kStripNT);
+  cfg.dynamicSmemBytes = recip ? Strip<kSysRecip>::bytes : Strip<kSysDiv>::bytes;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  void* args[] = {const_cast<JacobiBatchArgs*>(&a)};
-  return cudaLaunchKernelExC(&cfg, fn, args);
+  void* args[] = {const_cast<StripBatchArgs*>(&a)};
+  return cudaLaunchKernelExC(&cfg, batch_fn(recip), args);
 }
 
 // Batched TimeStep: block b covers 128 cells of problem blk[b].x from blk[b].y.

@@ -188,6 +188,48 @@ struct JacobiBatchArgs {
   // it (reset to 0 before every pass) instead of striding by CTA
   unsigned int* work;
 };
+// ---- the same solves by strips (the per-phase form; swm_strip.cuh) ----
+// State of one system between passes.
+struct SysState {
+  const double* xin;
+  double* xout;
+  int k;            // sweeps done
+  int Tp;           // sweeps of the coming pass
+  int active;       // still iterating
+  int first;        // the coming pass is the first
+  int rollback;     // the coming pass redoes the last one with Tp sweeps
+  int zero;         // converged before the first sweep: the reference returns 0
+  int maxhit;
+  int exact;        // left to solve_exact, which goes on from xin
+  float r_prev;     // residual sum of the last sweep of the previous pass (planning)
+};
+constexpr int kJacobiBatchWarps = 4;  // warps per block of the batched solve
+constexpr int kBatchSums = 8;  // residual sums of a pass, padded
+struct StripBatchState {
+  SysState s;
+  double sum[kBatchSums];  // zero between passes
+};
+struct StripBatchCtl {
+  unsigned int bar[5];          // barrier arrivals of each correction's launch
+  int nact[3];                  // systems still iterating after a pass (ring)
+  int nexact;                   // systems left to solve_exact in this launch
+  int status;                   // 0 ok, 1 some problem hit maxIter, -4 watchdog
+  int exact_next;
+  unsigned int work;            // next work item of the pass
+  unsigned long long acc[kResSlots][2][3];  // solve_exact's limbs
+};
+struct StripBatchArgs {
+  const JacobiArgs* descs;  // [nsets * nprob], as JacobiBatchArgs
+  const int4* items;        // (problem, strip, first row, rows) of every chunk of a set
+  int nitems, nprob, nsets;
+  int correction;           // 0..4: which barrier counter
+  StripBatchState* st;      // [nsets * nprob], zeroed before the step
+  StripBatchCtl* ctl;       // zeroed before the step
+  int* iters;               // [nsets * nprob] sweeps of each system's solve
+  const int* hint;          // nullable: sweeps of the same substeps' previous solves
+  int block;                // sweeps per pass at most
+  long long spin_limit;
+};
 struct DtBatchDesc {
   int nx, ny;
   double g, cfl, dx, dy;
@@ -262,9 +304,12 @@ cudaError_t launch_assemble_multi_batch(const AssembleMultiArgs* descs, const in
                                         cudaStream_t s);
 cudaError_t launch_assemble_batch(const AssembleArgs* descs, const int2* blk, int nblk, bool fast,
                                   cudaStream_t s);
-cudaError_t launch_jacobi_batch(const JacobiBatchArgs& a, int grid_blocks, bool recip,
+cudaError_t launch_jacobi_batch(const StripBatchArgs& a, int grid_blocks, bool recip,
                                 cudaStream_t s);
-int jacobi_batch_grid_blocks(int block, int device, bool recip);
+int jacobi_batch_grid_blocks(int device, bool recip);
+// Work items of one problem's set of a batched solve: strips x chunks of at most `rows`
+// rows, evenly.
+int jacobi_batch_strips(int nx);
 cudaError_t launch_dt_batch(const DtBatchDesc* d, const int2* blk, int nblk, int nprob,
                             unsigned long long* lam, int* bad, double* dt, cudaStream_t s);
 cudaError_t launch_rhs_fast(int mode, const RhsArgs& a, const RhsTma& tm, cudaStream_t s);

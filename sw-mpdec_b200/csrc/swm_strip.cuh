@@ -25,7 +25,7 @@
 
 namespace swm {
 
-constexpr int kStripWarps = 4;                   // warps of a CTA (independent of each other)
+constexpr int kStripWarps = kJacobiBatchWarps;   // warps of a CTA (independent of each other)
 constexpr int kStripNT = 32 * kStripWarps;
 constexpr int kStripSlots = 4;                   // ring rows: three copies ahead of the sweeps
 constexpr int kStripCols = 64;                   // columns a warp loads
@@ -98,8 +98,8 @@ __device__ __forceinline__ void pair_store(double* row, const StripLane& L, doub
 
 // Copy of row gj of the system and of the iterate into ring words dst[0 .. PL) (stride 32
 // words: one per lane).
-template <int FORM>
-__device__ __forceinline__ void strip_copy(const JacobiSys& y, const double* xin, int nx, int pitch,
+template <int FORM, typename Sys>
+__device__ __forceinline__ void strip_copy(const Sys& y, const double* xin, int nx, int pitch,
                                            int gj, const StripLane& L, double2* dst) {
   using G = Strip<FORM>;
   const size_t row = (size_t)gj * pitch;
@@ -222,8 +222,8 @@ __device__ __forceinline__ StripRow<FORM> strip_row(const double2* w, bool& bad)
 // NL sweeps are formed first: few dependent operations per sweep are left in series.
 // Steps before a sweep's first row compute on the zeros and unit rows set below and
 // deliver nothing.
-template <int FORM, int NL>
-__device__ __forceinline__ void strip_chunk(const JacobiSys& y, const double* xin, double* xout,
+template <int FORM, int NL, typename Sys>
+__device__ __forceinline__ void strip_chunk(const Sys& y, const double* xin, double* xout,
                                             int nx, int ny, int pitch, int opitch, int Tp,
                                             bool first, int strip, int j0, int rows, bool aligned,
                                             double2* ring, double (&sum)[kPassT + 1]) {
@@ -305,8 +305,8 @@ __device__ __forceinline__ void strip_chunk(const JacobiSys& y, const double* xi
 
 // Tp sweeps over one chunk by the code of the next even number of sweeps, the lane's
 // sums in sum.
-template <int FORM>
-__device__ __forceinline__ void strip_pass(const JacobiSys& y, const double* xin, double* xout,
+template <int FORM, typename Sys>
+__device__ __forceinline__ void strip_pass(const Sys& y, const double* xin, double* xout,
                                            int nx, int ny, int pitch, int opitch, int Tp,
                                            bool first, int strip, int j0, int rows, bool aligned,
                                            double2* ring, double (&sum)[kPassT + 1]) {
