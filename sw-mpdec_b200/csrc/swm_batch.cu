@@ -223,6 +223,7 @@ static RhsArgs batch_rhs_desc(const BProblem& q, const double* h, const double* 
   a.src_cols = q.src_cols;
   a.src_rows = q.src_rows;
   a.bgrad = q.bgrad;
+  a.over_len = q.p.precision == SWM_PREC_FP64 ? 1 : 0;
   return a;
 }
 

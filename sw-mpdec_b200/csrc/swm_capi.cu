@@ -238,6 +238,7 @@ static RhsArgs make_rhs_args(swm_solver* s, const double* h, const double* hu, c
   a.src_cols = s->src_cols;
   a.src_rows = s->src_rows;
   a.bgrad = s->bgrad;
+  a.over_len = fast_patankar(s->p) ? 0 : 1;
   a.status = &s->ctl->status;
   return a;
 }
@@ -526,13 +527,13 @@ static int enqueue_patankar(swm_solver* s) {
   }
   int solve = 0, last_solve[5] = {-1, -1, -1, -1, -1};  // by substep: its latest solve
   // the three substeps of an mPDeC5 correction iteration depend only on the previous
-  // iteration: the split and FMA forms assemble them in one launch (stencil layout), and
-  // they are solved together unless the grid is large (kGroupCells)
-  const bool fused = !csr && ms == 4 && fast_patankar(s->p);
+  // iteration: they are assembled in one launch and solved together, unless the grid is
+  // large (kGroupCells; the split and FMA forms have the planes to assemble all three)
+  const bool fused = ms == 4 && (s->grouped || fast_patankar(s->p));
   for (int k = 1; k <= kc; ++k) {
     const int mlo = (k == kc) ? ms : 2;
     const bool last = (k == kc);
-    const bool fuse_k = fused && !last, group_k = s->grouped && ms == 4 && !last;
+    const bool fuse_k = fused && !last, group_k = s->grouped && !last;
     JacobiGroup ja{};
     ja.nx = s->nx;
     ja.ny = s->ny;
@@ -545,7 +546,7 @@ static int enqueue_patankar(swm_solver* s) {
     ja.ctl = s->ctl;
     ja.spin_limit = s->spin_limit;
     for (int m = mlo; m <= ms; ++m) {
-      const int set = (fuse_k || group_k) ? m - 2 : 0;  // substep m's system
+      const int set = fuse_k ? m - 2 : 0;  // substep m's system
       AssembleArgs aa{};
       aa.nx = s->nx;
       aa.ny = s->ny;
@@ -600,9 +601,11 @@ static int enqueue_patankar(swm_solver* s) {
           ma.cE[q] = s->cset[q][2];
           ma.cN[q] = s->cset[q][3];
           ma.cD[q] = s->cset[q][4];
+          ma.csr_mass[q] = s->csr_mass[q];
+          ma.csr_diag[q] = s->csr_diag[q];
         }
         prof_mark(s, 1);
-        CK(launch_assemble_multi(ma, s->stream));
+        CK(launch_assemble_multi(ma, csr, s->stream));
         prof_mark(s, -1);
       }
       const int xs = group_k ? set : 0;

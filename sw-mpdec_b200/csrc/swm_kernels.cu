@@ -171,15 +171,28 @@ __global__ void __launch_bounds__(128, 4) assemble_multi_kernel(const AssembleMu
   assemble_multi_cell(a, i, j);
 }
 
-cudaError_t launch_assemble_multi(const AssembleMultiArgs& a, cudaStream_t s) {
-  if (a.nm != kMaxFusedStages || a.base.msteps != 4 || !a.base.fast) return cudaErrorInvalidValue;
+// The same for the exact forms (FP64; any form with the CSR solver).
+__global__ void __launch_bounds__(128, 4)
+    assemble_multi_exact_kernel(const __grid_constant__ AssembleMultiArgs a, bool csr) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y;
+  if (i >= a.base.nx || j >= a.base.ny) return;
+  assemble_multi_exact_cell(a, csr, i, j);
+}
+
+cudaError_t launch_assemble_multi(const AssembleMultiArgs& a, bool csr, cudaStream_t s) {
+  if (a.nm != kMaxFusedStages || a.base.msteps != 4) return cudaErrorInvalidValue;
   dim3 blk(128), grd((a.base.nx + 127) / 128, a.base.ny);
-  assemble_multi_kernel<<<grd, blk, 0, s>>>(a);
+  if (a.base.fast && !csr)
+    assemble_multi_kernel<<<grd, blk, 0, s>>>(a);
+  else
+    assemble_multi_exact_kernel<<<grd, blk, 0, s>>>(a, csr);
   return cudaGetLastError();
 }
 
 template <bool FAST, int MS>
-__global__ void __launch_bounds__(128) assemble_kernel(const AssembleArgs a, bool csr) {
+__global__ void __launch_bounds__(128) assemble_kernel(const __grid_constant__ AssembleArgs a,
+                                                       bool csr) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y;
   if (i >= a.nx || j >= a.ny) return;

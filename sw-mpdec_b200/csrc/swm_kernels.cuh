@@ -53,8 +53,8 @@ struct AssembleArgs {
   const double* hv_n;
   const double* fu[4];    // FUp(r, 2) planes
   const double* fv[4];    // FUp(r, 3)
-  const double* fxm[4];   // mass fluxes of stage r: [ny][nx+1]
-  const double* fym[4];   // [ny+1][nx]
+  const double* fxm[4];   // mass fluxes of stage r [ny][nx+1] (over dx unless fast)
+  const double* fym[4];   // [ny+1][nx] (over dy unless fast)
   const double* hp[4];    // Up(r, 1) for r = 1..msteps (hp(m,.) is hp[m-1])
   double* hu_out;         // Ua(m, 2:3)
   double* hv_out;
@@ -90,6 +90,8 @@ struct AssembleMultiArgs {
   double* cE[kMaxFusedStages];
   double* cN[kMaxFusedStages];
   double* cD[kMaxFusedStages];
+  double* csr_mass[kMaxFusedStages];  // CSR solver
+  double* csr_diag[kMaxFusedStages];
 };
 
 struct JacobiArgs {
@@ -318,7 +320,7 @@ size_t rhs_smem_bytes(int mode);
 
 cudaError_t launch_dt(const DtArgs& a, cudaStream_t s);
 cudaError_t launch_assemble(const AssembleArgs& a, bool csr, cudaStream_t s);
-cudaError_t launch_assemble_multi(const AssembleMultiArgs& a, cudaStream_t s);
+cudaError_t launch_assemble_multi(const AssembleMultiArgs& a, bool csr, cudaStream_t s);
 // Resident blocks of the Jacobi kernel's two forms (swm_strip.cuh).
 struct JacobiGrid {
   int tile_blocks, strip_blocks;

@@ -42,6 +42,9 @@ struct RhsArgs {
   double* ut_h;         // nullable: mass RHS Ut(1) (build without PATANKAR, explicit schemes)
   double* fxm;          // mass flux at x faces [ny][nx+1] (face f = left face of cell f)
   double* fym;          // mass flux at y faces [ny+1][nx]
+  // 1: fxm, fym hold the fluxes divided by dx, dy: the production and destruction entries
+  // of the exact assembly, which reads each of them in up to three substeps
+  int over_len;
   double* fx_full;      // nullable: [3][ny][nx+1]
   double* fy_full;      // nullable: [3][ny+1][nx]
   double* s_full;       // nullable: [3][ny][nx]
@@ -720,10 +723,17 @@ __device__ __forceinline__ void rhs_tile(const RhsArgs& a, const RhsTma* tm, con
       else
         a.ut_h[kc] = s[0] - (fxr[0] - fxl[0]) * gr.rdx - (fyt[0] - fyb[0]) * gr.rdy;
     }
-    a.fxm[kx] = fxl[0];
-    a.fym[ky] = fyb[0];
-    if (gi == nx - 1) a.fxm[kx + 1] = fxr[0];
-    if (gj == ny - 1) a.fym[ky + nx] = fyt[0];
+    if (a.over_len) {  // correctly rounded quotients (finitevolume.f90:500-523)
+      a.fxm[kx] = div_rn(fxl[0], gr.dx, gr.rdx);
+      a.fym[ky] = div_rn(fyb[0], gr.dy, gr.rdy);
+      if (gi == nx - 1) a.fxm[kx + 1] = div_rn(fxr[0], gr.dx, gr.rdx);
+      if (gj == ny - 1) a.fym[ky + nx] = div_rn(fyt[0], gr.dy, gr.rdy);
+    } else {
+      a.fxm[kx] = fxl[0];
+      a.fym[ky] = fyb[0];
+      if (gi == nx - 1) a.fxm[kx + 1] = fxr[0];
+      if (gj == ny - 1) a.fym[ky + nx] = fyt[0];
+    }
     if (a.fx_full) {
 #pragma unroll
       for (int v = 0; v < 3; ++v) {

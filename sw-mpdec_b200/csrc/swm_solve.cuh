@@ -94,8 +94,8 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 // Stage combination + Patankar assembly for substep m
 //   Ua(m,2:3) = Ua(1,2:3) + sum_r dt theta(m,r) FUp(r,2:3)   timediscretization.f90:539-543
 //   Mass/Diagonal of MODIFIED_PATANKAR_MATRIX_INVERSION       timediscretization.f90:795-885
-// P/D entries are rebuilt from the stored mass fluxes with the same operations
-// UpdateTimeDerivative uses (finitevolume.f90:500-523).
+// P/D entries are the stored mass fluxes over dx, dy, the quotients that
+// UpdateTimeDerivative forms (finitevolume.f90:500-523).
 // ---------------------------------------------------------------------------
 // PATANKAR_DIV(p, h) = 0 if h < MIN_DEPTH, else 2 h p / den(h) with
 // den(h) = h^2 + max(h^2, MIN_DEPTH) (timediscretization.f90:913-924).
@@ -159,13 +159,12 @@ __device__ __forceinline__ void load_cell(const AssembleArgs& a, int i, int j, s
 
 // Outputs of one substep m: Ua(m, 2:3) and its Patankar system (stencil or CSR).
 struct StageOut {
-  double *hu, *hv, *cS, *cW, *cE, *cN, *cD;
+  double *hu, *hv, *cS, *cW, *cE, *cN, *cD, *mass, *diag;
 };
 
 // Combination + assembly of substep m (1-based) for one cell from its loaded inputs.
-//  exact: the reference's branches and operation order; each quotient correctly
-//         rounded (div_rn) from RN(1/len) and one RN(1/den(h)) per depth, i.e. equal
-//         to the division it replaces;
+//  exact: the reference's operation order; each quotient correctly rounded (div_rn) from
+//         one RN(1/den(h)) per depth, i.e. equal to the division it replaces;
 //  FAST : weights w(h) = 2h/den(h) from one reciprocal per depth, 1/len folded into
 //         them, dt theta_r formed once and every term added by a fused
 //         multiply-add (split and FMA forms; the batched assembly shares this code,
@@ -184,8 +183,72 @@ __device__ __forceinline__ void load_hp(const AssembleArgs& a, int m1, int i, in
   hL[3] = hp_read(a, m, i, jp);
 }
 
+// Row of the Patankar matrix in the reference's order (timediscretization.f90:795-885).
+// fl holds the face fluxes over the cell's extent (RhsArgs::over_len), oriented into the
+// cell: p > 0 is the production P_KL, -p the destruction D_KL of p < 0.  Either is weighted
+// by the depth it leaves (the neighbour's for th > 0 and production, th < 0 and
+// destruction), which selects the operands of one division.  The quotients are div_mk's,
+// which needs no branch, so that all of a row's divisions overlap; returns true when an
+// operand was outside its range (a zero numerator +0 is right too), and the caller then
+// takes the SAFE form (div_rn) for the cell.
+template <int MS, bool SAFE>
+__device__ __forceinline__ bool patankar_exact(double dt, const double (&fl)[4][MS], double hK,
+                                               const double (&hL)[4], const double* theta,
+                                               double (&M)[4], double& D) {
+  const double denK = patankar_den(hK), rdenK = __drcp_rn(denK), hK2 = 2. * hK;
+  bool bad = !mk_range(denK);
+  D = 1.;
+#pragma unroll
+  for (int nb = 0; nb < 4; ++nb) {
+    const double h = hL[nb], denL = patankar_den(h), rdenL = __drcp_rn(denL), hL2 = 2. * h;
+    bad |= !mk_range(denL);
+    double m = 0.;
+#pragma unroll
+    for (int r = 0; r < MS; ++r) {
+      const double p = fl[nb][r], th = theta[r];
+      const bool pos = p > 0., other = pos == (th > 0.);  // other: the neighbour's depth
+      const double num = (other ? hL2 : hK2) * fabs(p);
+      const double den = other ? denL : denK, rden = other ? rdenL : rdenK;
+      double pd;
+      if constexpr (SAFE) {
+        pd = div_rn(num, den, rden);
+      } else {
+        pd = div_mk(num, den, rden);
+        bad |= !mk_range(num) && (__double2hiint(num) | __double2loint(num)) != 0;
+      }
+      if ((other ? h : hK) < kMinDepth) pd = 0.;
+      const double t = dt * th * pd;
+      // production takes t off, destruction (p < 0) adds it; neither for p = 0 or NaN
+      const double u = pos ? -t : (p < 0. ? t : 0.);
+      if (other)
+        m = __dadd_rn(m, u);
+      else
+        D = __dadd_rn(D, u);
+    }
+    M[nb] = m;
+  }
+  return bad;
+}
+// The SAFE form out of line, from the arrays (so that the caller's operands need no
+// addresses); m1 is the substep, 1-based.
+struct PatankarRow {
+  double M[4], D;
+};
+template <int MS>
+static __device__ __noinline__ PatankarRow patankar_exact_safe(const AssembleArgs& a,
+                                                               const double* theta, int m1, int i,
+                                                               int j) {
+  PatankarRow o;
+  CellIn<MS> c;
+  double hK, hL[4];
+  load_cell<false, MS>(a, i, j, (size_t)j * a.nx + i, (size_t)j * (a.nx + 1) + i, c);
+  load_hp(a, m1, i, j, hK, hL);
+  patankar_exact<MS, true>(c.dt, c.fl, hK, hL, theta, o.M, o.D);
+  return o;
+}
+
 template <bool FAST, int MS>
-__device__ __forceinline__ void assemble_stage(const AssembleArgs& a, bool csr, int i, int j,
+__device__ __forceinline__ void assemble_stage(const AssembleArgs& a, bool csr, int m1, int i, int j,
                                                const CellIn<MS>& c, const double hK,
                                                const double (&hL)[4], const double* theta,
                                                const StageOut& o) {
@@ -238,46 +301,22 @@ __device__ __forceinline__ void assemble_stage(const AssembleArgs& a, bool csr, 
     o.hu[k] = au;
     o.hv[k] = av;
     // ---- Patankar weights (timediscretization.f90:795-885) ----
-    const double denK = patankar_den(hK), rdenK = __drcp_rn(denK);
-  #pragma unroll
-    for (int nb = 0; nb < 4; ++nb) {
-      const bool ydir = (nb == 0 || nb == 3);
-      const double len = ydir ? a.dy : a.dx, ilen = ydir ? a.inv_dy : a.inv_dx;
-      const double h = hL[nb], denL = patankar_den(h), rdenL = __drcp_rn(denL);
-  #pragma unroll
-      for (int r = 0; r < MS; ++r) {
-        const double f = c.fl[nb][r], th = theta[r];
-        if (f > 0.) {  // production P_KL = f/len
-          const double P = div_rn(f, len, ilen);
-          if (th > 0.) {
-            const double pd = h < kMinDepth ? 0. : div_rn(2. * h * P, denL, rdenL);
-            M[nb] = M[nb] - dt * th * pd;
-          } else {
-            const double pd = hK < kMinDepth ? 0. : div_rn(2. * hK * P, denK, rdenK);
-            D = D - dt * th * pd;
-          }
-        } else if (f < 0.) {  // destruction D_KL = -f/len
-          const double Q = div_rn(-f, len, ilen);
-          if (th > 0.) {
-            const double pd = hK < kMinDepth ? 0. : div_rn(2. * hK * Q, denK, rdenK);
-            D = D + dt * th * pd;
-          } else {
-            const double pd = h < kMinDepth ? 0. : div_rn(2. * h * Q, denL, rdenL);
-            M[nb] = M[nb] + dt * th * pd;
-          }
-        }
-      }
+    if (patankar_exact<MS, false>(dt, c.fl, hK, hL, theta, M, D)) {
+      const PatankarRow safe = patankar_exact_safe<MS>(a, theta, m1, i, j);
+#pragma unroll
+      for (int nb = 0; nb < 4; ++nb) M[nb] = safe.M[nb];
+      D = safe.D;
     }
   }
   if (csr) {
     // CSR slots S, W, C, E, N of row K (finitevolume.f90:234-261)
-    double* mv = a.csr_mass + 5 * k;
+    double* mv = o.mass + 5 * k;
     mv[0] = M[0];
     mv[1] = M[1];
     mv[2] = 0.;
     mv[3] = M[2];
     mv[4] = M[3];
-    a.csr_diag[k] = D;
+    o.diag[k] = D;
   } else if constexpr (FAST) {
     // the fast stencil solver iterates x = b/D - sum (M/D) x: the row divided by its
     // Diagonal, the rhs b = hp(1,.) (timediscretization.f90:887) in the D plane
@@ -307,11 +346,29 @@ __device__ __forceinline__ void assemble_cell(const AssembleArgs& a, bool csr, c
   load_cell<FAST, MS>(a, i, j, k, kx, c);
   double hK, hL[4];
   load_hp(a, a.m, i, j, hK, hL);
-  const StageOut o{a.hu_out, a.hv_out, a.cS, a.cW, a.cE, a.cN, a.cD};
-  assemble_stage<FAST, MS>(a, csr, i, j, c, hK, hL, a.theta, o);
+  const StageOut o{a.hu_out, a.hv_out, a.cS, a.cW, a.cE, a.cN, a.cD, a.csr_mass, a.csr_diag};
+  assemble_stage<FAST, MS>(a, csr, a.m, i, j, c, hK, hL, a.theta, o);
   if (a.rhs_out) {  // rhs = hp(1,.) (timediscretization.f90:887), in the planes' layout
     const size_t kj = a.jpitch > 0 ? (size_t)j * a.jpitch + i : k;
     a.rhs_out[kj] = hp_read(a, 0, i, j);
+  }
+}
+
+// One cell of the exact forms' assembly of the kMaxFusedStages substeps of a correction:
+// the flux quotients and stage momenta are read once and stay in registers while the
+// substeps follow one another (unrolled, their reciprocals and sums would take 220).
+__device__ __forceinline__ void assemble_multi_exact_cell(const AssembleMultiArgs& am, bool csr,
+                                                          const int i, const int j) {
+  const size_t kk = (size_t)j * am.base.nx + i, kx = (size_t)j * (am.base.nx + 1) + i;
+  CellIn<4> cin;
+  load_cell<false, 4>(am.base, i, j, kk, kx, cin);
+#pragma unroll 1
+  for (int q = 0; q < kMaxFusedStages; ++q) {
+    double hK, hL[4];
+    load_hp(am.base, am.m[q], i, j, hK, hL);
+    const StageOut o{am.hu_out[q], am.hv_out[q], am.cS[q], am.cW[q], am.cE[q],
+                     am.cN[q],     am.cD[q],     am.csr_mass[q], am.csr_diag[q]};
+    assemble_stage<false, 4>(am.base, csr, am.m[q], i, j, cin, hK, hL, am.theta[q], o);
   }
 }
 
@@ -328,8 +385,9 @@ __device__ __forceinline__ void assemble_multi_cell(const AssembleMultiArgs& am,
   for (int q = 0; q < kMaxFusedStages; ++q) load_hp(am.base, am.m[q], i, j, hK[q], hL[q]);
 #pragma unroll
   for (int q = 0; q < kMaxFusedStages; ++q) {
-    const StageOut o{am.hu_out[q], am.hv_out[q], am.cS[q], am.cW[q], am.cE[q], am.cN[q], am.cD[q]};
-    assemble_stage<true, 4>(am.base, false, i, j, cin, hK[q], hL[q], am.theta[q], o);
+    const StageOut o{am.hu_out[q], am.hv_out[q], am.cS[q], am.cW[q], am.cE[q],
+                     am.cN[q],     am.cD[q],     nullptr,  nullptr};
+    assemble_stage<true, 4>(am.base, false, am.m[q], i, j, cin, hK[q], hL[q], am.theta[q], o);
   }
   if (am.base.rhs_out) {
     const size_t kj = am.base.jpitch > 0 ? (size_t)j * am.base.jpitch + i : kk;
