@@ -296,6 +296,50 @@ static cudaError_t launch_rhs(swm_solver* s, const RhsArgs& a) {
   return launch_rhs_fast(s->p.precision == SWM_PREC_SPLIT ? 1 : 0, a, tm, s->stream);
 }
 
+// Event pair around one launch when profiling (class 0 RHS, 1 assembly, 2 Jacobi).
+static void prof_mark(swm_solver* s, int cls) {
+  if (!s->profiling) return;
+  cudaEvent_t e;
+  cudaEventCreate(&e);
+  cudaEventRecord(e, s->stream);
+  s->prof_ev.push_back(e);
+  s->prof_cls.push_back(cls);
+}
+
+// The RHS of n <= kRhsGroup states of the grid: one launch for all of them while they are
+// few tiles (fewer launches and part-filled last rounds), in 8 x 8 tiles while even the
+// 16 x 16 tiles of all states would fill less than half of the SMs.  Measured per mPDeC5
+// step (one RHS, then four times three; B200), separate / one launch / one launch of 8 x 8
+// tiles: FP64 50^2 487 / 198 / 124 us, 100^2 490 / 205 / 221, 512^2 2251 / 2153 / 3456;
+// split 50^2 191 / 74 / 54, 512^2 668 / 600 / 1143, 1024^2 2282 / 2254 / -.  A group
+// launch stages its state's arguments in shared memory and loads tiles without TMA, which
+// costs 2.8% of a large grid's RHS.
+constexpr long long kRhsSmallTiles = 64, kRhsGroupTiles = 3 * 4096;
+
+static int launch_rhs_states(swm_solver* s, const RhsArgs* a, int n) {
+  const long long tiles = (long long)((s->nx + RHS_TX - 1) / RHS_TX) *
+                          ((s->ny + RHS_TY - 1) / RHS_TY) * n;
+  const bool small = tiles <= kRhsSmallTiles;
+  if (small || (n > 1 && tiles <= kRhsGroupTiles)) {
+    RhsGroup g;
+    for (int q = 0; q < n; ++q) g.a[q] = a[q];
+    for (int q = n; q < kRhsGroup; ++q) g.a[q] = a[0];
+    prof_mark(s, 0);
+    if (s->p.precision == SWM_PREC_FP64)
+      CK(launch_rhs_group_exact(g, n, small, s->stream));
+    else
+      CK(launch_rhs_group_fast(s->p.precision == SWM_PREC_SPLIT ? 1 : 0, g, n, small, s->stream));
+    prof_mark(s, -1);
+    return SWM_OK;
+  }
+  for (int q = 0; q < n; ++q) {
+    prof_mark(s, 0);
+    CK(launch_rhs(s, a[q]));
+    prof_mark(s, -1);
+  }
+  return SWM_OK;
+}
+
 // One RHS outside a step, waited for: a tile whose TMA load gave up is reported.
 static int run_rhs_sync(swm_solver* s, const RhsArgs& a) {
   CK(cudaMemsetAsync(&s->ctl->status, 0, sizeof(int), s->stream));
@@ -310,16 +354,6 @@ static int run_rhs_sync(swm_solver* s, const RhsArgs& a) {
 static void fill_thresh(const swm_solver* s, unsigned long long t[3]) {
   // stop when sum|dx| <= tol * n  (jacobi_iteration.f90:71,77)
   residual_limbs_host(s->p.jacobi_tol * (double)s->N, t);
-}
-
-// Event pair around one launch when profiling (class 0 RHS, 1 assembly, 2 Jacobi).
-static void prof_mark(swm_solver* s, int cls) {
-  if (!s->profiling) return;
-  cudaEvent_t e;
-  cudaEventCreate(&e);
-  cudaEventRecord(e, s->stream);
-  s->prof_ev.push_back(e);
-  s->prof_cls.push_back(cls);
 }
 
 // Enqueue one complete mPDeC step on s->stream (dt read from s->dt_dev).
@@ -340,10 +374,7 @@ static int explicit_rhs(swm_solver* s, const Planes& X, const Planes& R) {
   a.ut_h = R[0];
   a.ut_hu = R[1];
   a.ut_hv = R[2];
-  prof_mark(s, 0);
-  CK(launch_rhs(s, a));
-  prof_mark(s, -1);
-  return SWM_OK;
+  return launch_rhs_states(s, &a, 1);
 }
 
 static int combo(swm_solver* s, int form, std::initializer_list<std::pair<double, Planes>> xs,
@@ -521,9 +552,8 @@ static int enqueue_patankar(swm_solver* s) {
   // RHS at U^n (timediscretization.f90:519), stored in slot 1 and used for all r at k=1
   {
     NvtxRange r("rhs");
-    prof_mark(s, 0);
-    CK(launch_rhs(s, make_rhs_args(s, s->h, s->hu, s->hv, 0)));
-    prof_mark(s, -1);
+    const RhsArgs ra = make_rhs_args(s, s->h, s->hu, s->hv, 0);
+    if (int rc = launch_rhs_states(s, &ra, 1)) return rc;
   }
   int solve = 0, last_solve[5] = {-1, -1, -1, -1, -1};  // by substep: its latest solve
   // the three substeps of an mPDeC5 correction iteration depend only on the previous
@@ -635,13 +665,11 @@ static int enqueue_patankar(swm_solver* s) {
       }
     }
     if (k < kc) {  // RHS at Ua(m) (timediscretization.f90:550-557)
-      for (int m = 2; m <= ms; ++m) {
-        NvtxRange r("rhs");
-        prof_mark(s, 0);
-        CK(launch_rhs(s, make_rhs_args(s, s->hbuf[m - 1][k & 1], s->hum[m - 1], s->hvm[m - 1],
-                                       m - 1)));
-        prof_mark(s, -1);
-      }
+      NvtxRange r("rhs");
+      RhsArgs ra[kRhsGroup];
+      for (int m = 2; m <= ms; ++m)
+        ra[m - 2] = make_rhs_args(s, s->hbuf[m - 1][k & 1], s->hum[m - 1], s->hvm[m - 1], m - 1);
+      if (int rc = launch_rhs_states(s, ra, ms - 1)) return rc;
     }
   }
   s->n_solves = solve;

@@ -66,7 +66,7 @@ __device__ __forceinline__ double ens_dt_of(const DtBatchDesc& d, unsigned long 
 // phases and the tile code get their registers allocated separately.
 template <int MODE>
 static __device__ __noinline__ void ens_tile(const RhsArgs& a, int i0, int j0) {
-  rhs_tile<MODE>(a, nullptr, i0, j0);
+  rhs_tile<MODE, JNT>(a, nullptr, i0, j0);
 }
 
 // The RHS of descriptor sets set0 .. set0 + nsets - 1 for every (problem, tile).  CTAs

@@ -316,6 +316,9 @@ cudaError_t launch_dt_batch(const DtBatchDesc* d, const int2* blk, int nblk, int
                             unsigned long long* lam, int* bad, double* dt, cudaStream_t s);
 cudaError_t launch_rhs_fast(int mode, const RhsArgs& a, const RhsTma& tm, cudaStream_t s);
 cudaError_t launch_rhs_exact(const RhsArgs& a, const RhsTma& tm, cudaStream_t s);
+// n states of one grid in one launch; small: 8 x 8 tiles
+cudaError_t launch_rhs_group_fast(int mode, const RhsGroup& g, int n, bool small, cudaStream_t s);
+cudaError_t launch_rhs_group_exact(const RhsGroup& g, int n, bool small, cudaStream_t s);
 size_t rhs_smem_bytes(int mode);
 
 cudaError_t launch_dt(const DtArgs& a, cudaStream_t s);

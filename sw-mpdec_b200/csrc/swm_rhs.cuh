@@ -73,11 +73,18 @@ struct RhsArgs {
 constexpr int RHS_TX = 16;
 constexpr int RHS_TY = 16;
 constexpr int RHS_NT = 256;
+// Grids of few tiles use 8 x 8 tiles (rhs_group_kernel): four times the blocks, and one
+// round of a block's threads where a 16 x 16 tile takes four or five.
+constexpr int RHS_SMALL = 8;
+constexpr int kRhsGroup = 3;  // states of one grid a group launch covers
+struct RhsGroup {
+  RhsArgs a[kRhsGroup];
+};
 
 // Shared-memory plan (element counts).
-template <typename T>
+template <typename T, int TX_ = RHS_TX, int TY_ = RHS_TY>
 struct RhsSmem {
-  static constexpr int TX = RHS_TX, TY = RHS_TY;
+  static constexpr int TX = TX_, TY = TY_;
   static constexpr int VX = TX + 6, VY = TY + 6;                  // V tile incl. 3-cell halo
   static constexpr int nV = 3 * VY * VX;                          // double
   static constexpr int F1X = (TY + 4) * (TX + 2);                 // x first sweeps
@@ -168,13 +175,12 @@ __device__ __forceinline__ void store_mp(unsigned long long* p, int pitch, f2 wm
 // MODE: 0 FP64 (EXACT per translation unit), 1 SPLIT.  One CTA, tile origin (i0, j0).
 // tm (nullable): tensor maps of the input planes; tiles whose haloed box lies inside
 // the grid are then staged by TMA, the others (at the periodic seams) by wrapped loads.
-template <int MODE>
+template <int MODE, int NT = RHS_NT, int TX = RHS_TX, int TY = RHS_TY>
 __device__ __forceinline__ void rhs_tile(const RhsArgs& a, const RhsTma* tm, const int i0,
                                          const int j0) {
   using T = typename std::conditional<MODE == 1, float, double>::type;
   constexpr bool EX = (MODE == 0) && SWM_EXACT;
-  constexpr int TX = RHS_TX, TY = RHS_TY, NT = RHS_NT;
-  using SM = RhsSmem<T>;
+  using SM = RhsSmem<T, TX, TY>;
   constexpr int VX = SM::VX, VY = SM::VY;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   double* sV = reinterpret_cast<double*>(smem_raw);  // [3][VY][VX]
@@ -192,9 +198,10 @@ __device__ __forceinline__ void rhs_tile(const RhsArgs& a, const RhsTma* tm, con
   // ---- load the haloed tile, V = ConsToPrim(U) (equation.f90:778-782) ----
   constexpr int NLD = (VY * VX + NT - 1) / NT;  // cells per thread; all loads issued first
   double lh[NLD], lhu[NLD], lhv[NLD];
-  static_assert(kTmaBoxX >= VX + 1 && kTmaBoxY == VY, "TMA box covers the haloed tile");
-  static_assert(3 * kTmaBoxX * kTmaBoxY + 16 <= SM::nW, "TMA staging fits the face-value area");
-  if (tm != nullptr && tm->enabled && i0 >= 4 && i0 - 4 + kTmaBoxX <= nx && j0 >= 3 &&
+  constexpr bool kTmaTile = TX == RHS_TX && TY == RHS_TY;  // the maps' boxes are its size
+  static_assert(!kTmaTile || (kTmaBoxX >= VX + 1 && kTmaBoxY == VY), "TMA box covers the haloed tile");
+  static_assert(!kTmaTile || 3 * kTmaBoxX * kTmaBoxY + 16 <= SM::nW, "TMA staging fits the face-value area");
+  if (kTmaTile && tm != nullptr && tm->enabled && i0 >= 4 && i0 - 4 + kTmaBoxX <= nx && j0 >= 3 &&
       j0 - 3 + kTmaBoxY <= ny) {
     // Interior tile: one thread copies the three 24 x 22 boxes (columns i0-4..i0+19,
     // rows j0-3..j0+18) into the face-value area, unused until the x second sweeps,
@@ -752,6 +759,31 @@ template <int MODE>
 __global__ void __launch_bounds__(RHS_NT, 2)
     rhs_kernel(const RhsArgs a, const __grid_constant__ RhsTma tm) {
   rhs_tile<MODE>(a, &tm, blockIdx.x * RHS_TX, blockIdx.y * RHS_TY);
+}
+
+// Up to kRhsGroup states of one grid, block z of the grid state z, in tiles of TX x TX.
+template <int MODE, int TX>
+__global__ void __launch_bounds__(RHS_NT, 2) rhs_group_kernel(const __grid_constant__ RhsGroup g) {
+  static_assert(sizeof(RhsArgs) % 8 == 0 && sizeof(RhsArgs) / 8 <= RHS_NT, "descriptor copy");
+  __shared__ __align__(16) RhsArgs sa;
+  if (threadIdx.x < sizeof(RhsArgs) / 8)
+    reinterpret_cast<unsigned long long*>(&sa)[threadIdx.x] =
+        reinterpret_cast<const unsigned long long*>(&g.a[blockIdx.z])[threadIdx.x];
+  __syncthreads();
+  rhs_tile<MODE, RHS_NT, TX, TX>(sa, nullptr, blockIdx.x * TX, blockIdx.y * TX);
+}
+
+template <int MODE, int TX>
+static cudaError_t launch_group(const RhsGroup& g, int n, cudaStream_t s) {
+  using T = typename std::conditional<MODE == 1, float, double>::type;
+  constexpr int bytes = (int)RhsSmem<T, TX, TX>::bytes;
+  cudaError_t e = cudaFuncSetAttribute(rhs_group_kernel<MODE, TX>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return e;
+  const Grid& gr = g.a[0].gr;
+  dim3 grd((gr.nx + TX - 1) / TX, (gr.ny + TX - 1) / TX, n);
+  rhs_group_kernel<MODE, TX><<<grd, RHS_NT, bytes, s>>>(g);
+  return cudaGetLastError();
 }
 
 // Ensembles: CTA b computes tile (work[b].y, work[b].z) of problem work[b].x, whose

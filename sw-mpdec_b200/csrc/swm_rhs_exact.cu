@@ -26,6 +26,11 @@ cudaError_t launch_rhs_exact(const RhsArgs& a, const RhsTma& tm, cudaStream_t s)
   return cudaGetLastError();
 }
 
+cudaError_t launch_rhs_group_exact(const RhsGroup& g, int n, bool small, cudaStream_t s) {
+  return small ? rhs_exact::launch_group<0, RHS_SMALL>(g, n, s)
+               : rhs_exact::launch_group<0, RHS_TX>(g, n, s);
+}
+
 cudaError_t launch_rhs_batch_exact(const RhsArgs* descs, const int4* work, int nwork,
                                    cudaStream_t s) {
   if (nwork < 1) return cudaSuccess;

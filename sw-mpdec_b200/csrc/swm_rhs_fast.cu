@@ -41,6 +41,14 @@ cudaError_t launch_rhs_fast(int mode, const RhsArgs& a, const RhsTma& tm, cudaSt
   return cudaGetLastError();
 }
 
+cudaError_t launch_rhs_group_fast(int mode, const RhsGroup& g, int n, bool small, cudaStream_t s) {
+  if (mode == 1)
+    return small ? rhs_fast::launch_group<1, RHS_SMALL>(g, n, s)
+                 : rhs_fast::launch_group<1, RHS_TX>(g, n, s);
+  return small ? rhs_fast::launch_group<0, RHS_SMALL>(g, n, s)
+               : rhs_fast::launch_group<0, RHS_TX>(g, n, s);
+}
+
 cudaError_t launch_rhs_batch_fast(int mode, const RhsArgs* descs, const int4* work, int nwork,
                                   cudaStream_t s) {
   if (nwork < 1) return cudaSuccess;
