@@ -514,11 +514,19 @@ template <bool LAM32 = false>
 __device__ __forceinline__ void rusanov(double g, double hL, double nL, double tL, double hR,
                                         double nR, double tR, double& F0, double& F1, double& F2) {
   double FL0 = hL * nL;
-  double FL1 = hL * (nL * nL) + 0.5 * g * (hL * hL);
   double FL2 = hL * nL * tL;
   double FR0 = hR * nR;
-  double FR1 = hR * (nR * nR) + 0.5 * g * (hR * hR);
   double FR2 = hR * nR * tR;
+  double FL1, FR1;
+  if (LAM32) {
+    // the contraction of the expressions below, written out: which of the two products
+    // is fused must not depend on where the compiler inlines this
+    FL1 = fma(0.5 * g, __dmul_rn(hL, hL), __dmul_rn(hL, __dmul_rn(nL, nL)));
+    FR1 = fma(0.5 * g, __dmul_rn(hR, hR), __dmul_rn(hR, __dmul_rn(nR, nR)));
+  } else {
+    FL1 = hL * (nL * nL) + 0.5 * g * (hL * hL);
+    FR1 = hR * (nR * nR) + 0.5 * g * (hR * hR);
+  }
   double lam;
   if (LAM32) {
     float fl = (float)nL + sqrt_approx((float)(g * hL)),
@@ -568,6 +576,21 @@ __device__ __forceinline__ void limit_h(const Grid& gr, double Vc, double wm[4],
 // >= MIN_DEPTH up to FP64 rounding for every face value d >= mmin.
 __device__ __forceinline__ void limit_h_dev(const Grid& gr, double Vc, const float dm[4],
                                             const float dp[4], double wm[4], double wp[4]) {
+  // No deviation beyond the cell's depth over MIN_DEPTH: nothing limits.  The minimum
+  // below is one of the deviations or csi, which is at most a fifth of the largest, so
+  // its quotient is >= 1 at every Gauss point.
+  const double ta = Vc - kMinDepth;
+  float most = 0.f;
+#pragma unroll
+  for (int g = 0; g < 4; ++g) most = fmaxf(most, fmaxf(fabsf(dm[g]), fabsf(dp[g])));
+  if (fabs(ta) >= (double)most) {
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      wp[g] = Vc + (double)dp[g];
+      wm[g] = Vc + (double)dm[g];
+    }
+    return;
+  }
   float alpha = 0.f, beta = 0.f;
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
@@ -575,7 +598,6 @@ __device__ __forceinline__ void limit_h_dev(const Grid& gr, double Vc, const flo
     beta = fmaf(gr.qwf[g], dp[g], beta);
   }
   const float csi = -((float)kWLobatto * alpha + (float)kWLobatto * beta) * (float)kCsiRcp;
-  const double ta = Vc - kMinDepth;
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     const double mmin = (double)fminf(csi, fminf(dm[g], dp[g]));

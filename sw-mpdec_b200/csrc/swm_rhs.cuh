@@ -69,7 +69,7 @@ struct RhsArgs {
 };
 
 // 16 x 16 tiles: less vertical halo than 32 x 8 (the FP64 form is 4% faster, the split
-// form the same) at 105 KB of shared memory, two CTAs per SM
+// form the same); two CTAs per SM in the FP64 forms (97 KB), three in the split form
 constexpr int RHS_TX = 16;
 constexpr int RHS_TY = 16;
 constexpr int RHS_NT = 256;
@@ -92,16 +92,24 @@ struct RhsSmem {
   static constexpr int nF1 = 2 * 3 * (F1X > F1Y ? F1X : F1Y);     // T
   static constexpr int WX = TY * (TX + 2);                        // x face-value cells
   static constexpr int WY = (TY + 2) * TX;                        // y face-value cells
-  static constexpr int nW = 2 * 3 * 4 * (WX > WY ? WX : WY);      // double
+  static constexpr int nWC = WX > WY ? WX : WY;
+  static constexpr bool kSplit = std::is_same<T, float>::value;
+  // face values: FP64 [2][3][4][cells]; the split form keeps the depth's so and the
+  // velocities' as the FP32 deviations from the cell value that they are formed from
+  // (V + d is formed again, the same sum, where a face reads it)
+  static constexpr int nW = 2 * (kSplit ? 1 : 3) * 4 * nWC;       // double
+  static constexpr int nWD = kSplit ? 2 * 2 * 4 * nWC : 0;        // float
   static constexpr int nFX = 3 * TY * (TX + 1);                   // double
   static constexpr int nFY = 3 * (TY + 1) * TX;                   // double
   // split form: V also as interleaved FP32 (hi, lo) pairs (hi = fl32(V), lo = fl32(V - hi))
-  static constexpr int nVF = std::is_same<T, float>::value ? 2 * nV : 0;  // float
-  // split form: the source term's y sweeps [4][TY][TX+4] in a buffer of their own, so
-  // they can run in the x second-sweep phase (the FP64 form reuses the first-sweep area)
-  static constexpr int nVt = std::is_same<T, float>::value ? 4 * TY * (TX + 4) : 0;  // float
-  static constexpr size_t bytes = sizeof(double) * (nV + nW + nFX + nFY) + sizeof(T) * nF1 +
-                                  sizeof(float) * (nVF + nVt);
+  static constexpr int nVF = kSplit ? 2 * nV : 0;                 // float
+  // the split form's y fluxes lie over the velocities' pairs, which the y second sweeps
+  // read last, and its source sweeps over the y first sweeps: three tiles fit an SM
+  static constexpr int nVt = 4 * TY * (TX + 4);                   // T
+  static_assert(!kSplit || 2 * VY * VX >= nFY, "y fluxes over the velocity pairs");
+  static_assert(nVt <= nF1, "source sweeps over the first sweeps");
+  static constexpr size_t bytes = sizeof(double) * (nV + nW + nFX + (kSplit ? 0 : nFY)) +
+                                  sizeof(T) * nF1 + sizeof(float) * (nVF + nWD);
 };
 
 }  // namespace swm
@@ -162,7 +170,7 @@ __device__ __forceinline__ void face_pass(const Grid& gr, Flux&& flux, Store&& s
   }
 }
 
-// Split form: the first sweeps of two rows (wm, wp packed by row) stored as the (m, p)
+// Split form: the y first sweeps of two rows (wm, wp packed by row) stored as the (m, p)
 // pairs of row 0 at p[0] and of row 1 at p[pitch].
 __device__ __forceinline__ void store_mp(unsigned long long* p, int pitch, f2 wm, f2 wp) {
   float m0, m1, p0, p1;
@@ -184,12 +192,15 @@ __device__ __forceinline__ void rhs_tile(const RhsArgs& a, const RhsTma* tm, con
   constexpr int VX = SM::VX, VY = SM::VY;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   double* sV = reinterpret_cast<double*>(smem_raw);  // [3][VY][VX]
-  double* sW = sV + SM::nV;                          // [2][3][4][cells]
-  double* sFX = sW + SM::nW;                         // [3][TY][TX+1]
-  double* sFY = sFX + SM::nFX;                       // [3][TY+1][TX]
-  T* sF1 = reinterpret_cast<T*>(sFY + SM::nFY);      // [2][3][...]
+  double* sW = sV + SM::nV;                          // [2][3][4][cells]; split [2][4][cells]
+  float* sWD = reinterpret_cast<float*>(sW + SM::nW);  // split: [2][2][4][cells]
+  double* sFX = reinterpret_cast<double*>(sWD + SM::nWD);  // [3][TY][TX+1]
   // split: [3][VY][VX] (hi, lo) pairs, one 8-byte load each
-  unsigned long long* sVhl = reinterpret_cast<unsigned long long*>(sF1 + SM::nF1);
+  unsigned long long* sVhl = reinterpret_cast<unsigned long long*>(sFX + SM::nFX);
+  double* sFY = MODE == 1 ? reinterpret_cast<double*>(sVhl + VY * VX)  // [3][TY+1][TX]
+                          : sFX + SM::nFX;
+  T* sF1 = MODE == 1 ? reinterpret_cast<T*>(sVhl + SM::nV)  // [2][3][...]
+                     : reinterpret_cast<T*>(sFY + SM::nFY);
 
   const Grid& gr = a.gr;
   const int nx = gr.nx, ny = gr.ny;
@@ -200,7 +211,8 @@ __device__ __forceinline__ void rhs_tile(const RhsArgs& a, const RhsTma* tm, con
   double lh[NLD], lhu[NLD], lhv[NLD];
   constexpr bool kTmaTile = TX == RHS_TX && TY == RHS_TY;  // the maps' boxes are its size
   static_assert(!kTmaTile || (kTmaBoxX >= VX + 1 && kTmaBoxY == VY), "TMA box covers the haloed tile");
-  static_assert(!kTmaTile || 3 * kTmaBoxX * kTmaBoxY + 16 <= SM::nW, "TMA staging fits the face-value area");
+  static_assert(!kTmaTile || 3 * kTmaBoxX * kTmaBoxY + 16 <= SM::nW + SM::nWD / 2,
+                "TMA staging fits the face-value area");
   if (kTmaTile && tm != nullptr && tm->enabled && i0 >= 4 && i0 - 4 + kTmaBoxX <= nx && j0 >= 3 &&
       j0 - 3 + kTmaBoxY <= ny) {
     // Interior tile: one thread copies the three 24 x 22 boxes (columns i0-4..i0+19,
@@ -291,15 +303,77 @@ __device__ __forceinline__ void rhs_tile(const RhsArgs& a, const RhsTma* tm, con
     return dh + dl;
   };
 
-  // source term's y sweeps of h at the 4 y Gauss points (split form: own buffer)
+  // split form: deviation of one (hi, lo) pair from another, and two neighbouring 8-byte
+  // words by one 16-byte load
+  auto dev_of = [](unsigned long long a, unsigned long long c) -> float {
+    float dh, dl;
+    f2_unpack(sub2(f2{a}, f2{c}), dh, dl);
+    return dh + dl;
+  };
+  auto ld2 = [](const unsigned long long* p, unsigned long long& a, unsigned long long& b) {
+    const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(p);
+    a = w.x;
+    b = w.y;
+  };
+  // split form: face values of the neighbouring cells c, c + 1 (c even) of WC, from their
+  // (m, p) deviations w[cell][gauss]; lim: the cell's depth is limited
+  auto put_pair = [&](int v, int WC, int c, const f2 (&w)[2][4], const double (&Vc)[2],
+                      const bool (&lim)[2]) {
+    float dm[2][4], dp[2][4];
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int g = 0; g < 4; ++g) f2_unpack(w[e][g], dm[e][g], dp[e][g]);
+    if (v == 0) {
+      double hm[2][4], hp[2][4];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        if (lim[e]) {
+          limit_h_dev(gr, Vc[e], dm[e], dp[e], hm[e], hp[e]);
+        } else {
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            hm[e][g] = Vc[e] + (double)dm[e][g];
+            hp[e][g] = Vc[e] + (double)dp[e][g];
+          }
+        }
+      }
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        *reinterpret_cast<double2*>(&sW[g * WC + c]) = make_double2(hm[0][g], hm[1][g]);
+        *reinterpret_cast<double2*>(&sW[(4 + g) * WC + c]) = make_double2(hp[0][g], hp[1][g]);
+      }
+    } else {
+      float* d = sWD + (v - 1) * 4 * WC + c;
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        *reinterpret_cast<float2*>(&d[g * WC]) = make_float2(dm[0][g], dm[1][g]);
+        *reinterpret_cast<float2*>(&d[(8 + g) * WC]) = make_float2(dp[0][g], dp[1][g]);
+      }
+    }
+  };
+
+  // split form: flux at Gauss point g between cells L and R of WC whose velocities are
+  // (uL, vL) and (uR, vR), for x (dir 0) or y faces: normal and tangential components
+  auto split_flux = [&](int WC, int g, int L, int R, double uL, double vL, double uR, double vR,
+                        int dir, double& F0, double& Fn, double& Ft) {
+    const double hL = sW[(4 + g) * WC + L], hR = sW[g * WC + R];
+    const double a = uL + (double)sWD[(8 + g) * WC + L], b = vL + (double)sWD[(12 + g) * WC + L];
+    const double c = uR + (double)sWD[g * WC + R], d = vR + (double)sWD[(4 + g) * WC + R];
+    if (dir == 0)
+      rusanov<true>(gr.g, hL, a, b, hR, c, d, F0, Fn, Ft);
+    else
+      rusanov<true>(gr.g, hL, b, a, hR, d, c, F0, Fn, Ft);
+  };
+
+  // source term's y sweeps of h at the 4 y Gauss points
   const bool has_src = gr.bathy > 0;
   constexpr int SW_ = TX + 4;  // y-sweep columns i0-2..i0+TX+1
-  T* sVt = (MODE == 1) ? reinterpret_cast<T*>(sVhl + SM::nV) : sF1;  // [4][TY][TX+4]
+  T* sVt = sF1;                // [4][TY][TX+4], over the y first sweeps
   auto src_sweeps_split = [&]() {
     if constexpr (MODE == 1) {
     static_assert(TY % 2 == 0, "row pairs");
-    static_assert(SM::nVt == 4 * TY * SW_, "source sweep buffer");
-    for (int it = NT - 1 - tid; it < (TY / 2) * SW_; it += NT) {  // reversed: fills the last round
+    for (int it = NT - 1 - tid; it < (TY / 2) * SW_; it += NT) {  // reversed: balances the y faces
       int cc = it % SW_, rr = 2 * (it / SW_);
       // U(1) = V(1) = h; rows (j0+rr)-2..+2 -> tile rows rr+1..rr+5; col i0-2+cc -> cc+1
       f2 q[5], w[4];
@@ -324,22 +398,30 @@ __device__ __forceinline__ void rhs_tile(const RhsArgs& a, const RhsTma* tm, con
     T* sTP = sF1 + 3 * FH * FW;
     unsigned long long* sTMP = reinterpret_cast<unsigned long long*>(sF1);  // split: (m, p) pairs
     if constexpr (MODE == 1) {
-      // two rows per item (packed pairs), deviations from each stencil's centre
-      static_assert(FH % 2 == 0, "row pairs");
-      constexpr int FH2 = FH / 2;
-      for (int it = tid; it < 3 * FH2 * FW; it += NT) {
-        int cc = it % FW, rest = it / FW, rp = rest % FH2, v = rest / FH2;
-        const int rr = 2 * rp;
+      // two neighbouring columns per item (packed pairs): their stencils share four of
+      // six values, in three 16-byte loads; deviations from each stencil's centre, which
+      // is an exact zero
+      static_assert(FW % 2 == 0 && VX % 2 == 0, "column pairs");
+      constexpr int FW2 = FW / 2;
+      for (int it = tid; it < 3 * FH * FW2; it += NT) {
+        const int cc = 2 * (it % FW2), rest = it / FW2, rr = rest % FH, v = rest / FH;
+        const unsigned long long* p = &sVhl[(v * VY + rr + 1) * VX + cc];
+        unsigned long long h[6];
+#pragma unroll
+        for (int k = 0; k < 6; k += 2) ld2(p + k, h[k], h[k + 1]);
         f2 q[5];
 #pragma unroll
-        for (int k = 0; k < 5; ++k)  // k = 2 is each stencil's centre: an exact zero
-          if (k != 2)
-            q[k] = f2_pack(dev(v, rr + 1, cc + k, rr + 1, cc + 2),
-                           dev(v, rr + 2, cc + k, rr + 2, cc + 2));
-        q[2] = f2_splat(0.f);
+        for (int k = 0; k < 5; ++k)
+          q[k] = (k == 2) ? f2_splat(0.f) : f2_pack(dev_of(h[k], h[2]), dev_of(h[k + 1], h[3]));
         f2 wm, wp;
         weno5_first_x2<true>(q[0], q[1], q[2], q[3], q[4], wm, wp);
-        store_mp(sTMP + (v * FH + rr) * FW + cc, FW, wm, wp);
+        float m0, m1, p0, p1;
+        f2_unpack(wm, m0, m1);
+        f2_unpack(wp, p0, p1);
+        ulonglong2 o;
+        o.x = f2_pack(m0, p0).v;
+        o.y = f2_pack(m1, p1).v;
+        *reinterpret_cast<ulonglong2*>(&sTMP[(v * FH + rr) * FW + cc]) = o;
       }
     } else {
       for (int it = tid; it < 3 * FH * FW; it += NT) {
@@ -354,60 +436,60 @@ __device__ __forceinline__ void rhs_tile(const RhsArgs& a, const RhsTma* tm, con
     __syncthreads();
     // second sweeps along y; cells: cols i0-1..i0+TX (cc), rows j0..j0+TY-1 (rr)
     constexpr int WC = TY * FW;
-    for (int it = tid; it < 3 * WC; it += NT) {
-      int cc = it % FW, rest = it / FW, rr = rest % TY, v = rest / TY;
-      double wmv[4], wpv[4];
-      const double Vc = SV(v, rr + 3, cc + 2);
-      if constexpr (MODE == 1) {
-        float dm[4], dp[4];
-        f2 q[5], w[4];
+    if constexpr (MODE == 1) {
+      // two neighbouring columns per item: 16-byte loads of both and 16- or 8-byte stores
+      constexpr int FW2 = FW / 2;
+      for (int it = tid; it < 3 * TY * FW2; it += NT) {
+        const int cc = 2 * (it % FW2), rest = it / FW2, rr = rest % TY, v = rest / TY;
+        unsigned long long t[5][2], h[5][2];
 #pragma unroll
-        for (int k = 0; k < 5; ++k) {  // k = 2 is the centre row: no offset
-          const f2 t = f2{sTMP[(v * FH + rr + k) * FW + cc]};
-          q[k] = (k == 2) ? t : add2(f2_splat(dev(v, rr + 1 + k, cc + 2, rr + 3, cc + 2)), t);
+        for (int k = 0; k < 5; ++k) {
+          ld2(&sTMP[(v * FH + rr + k) * FW + cc], t[k][0], t[k][1]);
+          ld2(&sVhl[(v * VY + rr + 1 + k) * VX + cc + 2], h[k][0], h[k][1]);
         }
-        weno5_second_x2(q[0], q[1], q[2], q[3], q[4], w);
+        const double2 Vc2 = *reinterpret_cast<const double2*>(&SV(v, rr + 3, cc + 2));
+        f2 w[2][4];
 #pragma unroll
-        for (int g = 0; g < 4; ++g) f2_unpack(w[g], dm[g], dp[g]);
-        const int gc = i0 - 1 + cc;
-        if (v == 0 && gc != nx) {
-          limit_h_dev(gr, Vc, dm, dp, wmv, wpv);
-        } else {
+        for (int e = 0; e < 2; ++e) {
+          f2 q[5];
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            wmv[g] = Vc + (double)dm[g];
-            wpv[g] = Vc + (double)dp[g];
-          }
+          for (int k = 0; k < 5; ++k)  // k = 2 is the centre row: no offset
+            q[k] = (k == 2) ? f2{t[k][e]}
+                            : add2(f2_splat(dev_of(h[k][e], h[2][e])), f2{t[k][e]});
+          weno5_second_x2(q[0], q[1], q[2], q[3], q[4], w[e]);
         }
-      } else {
+        const double Vc[2] = {Vc2.x, Vc2.y};
+        const bool lim[2] = {i0 - 1 + cc != nx, i0 + cc != nx};
+        put_pair(v, WC, rr * FW + cc, w, Vc, lim);
+      }
+    } else {
+      for (int it = tid; it < 3 * WC; it += NT) {
+        int cc = it % FW, rest = it / FW, rr = rest % TY, v = rest / TY;
+        double wmv[4], wpv[4];
+        const double Vc = SV(v, rr + 3, cc + 2);
         const T* cm = &sTM[(v * FH + rr) * FW + cc];
         const T* cp = &sTP[(v * FH + rr) * FW + cc];
-        T tm[4], tp[4];
-        weno5_second<T, EX>(cm[0], cm[FW], cm[2 * FW], cm[3 * FW], cm[4 * FW], tm);
-        weno5_second<T, EX>(cp[0], cp[FW], cp[2 * FW], cp[3 * FW], cp[4 * FW], tp);
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          wmv[g] = tm[g];
-          wpv[g] = tp[g];
-        }
+        weno5_second<T, EX>(cm[0], cm[FW], cm[2 * FW], cm[3 * FW], cm[4 * FW], wmv);
+        weno5_second<T, EX>(cp[0], cp[FW], cp[2 * FW], cp[3 * FW], cp[4 * FW], wpv);
         const int gc = i0 - 1 + cc;
         if (v == 0 && gc != nx) limit_h(gr, Vc, wmv, wpv);
-      }
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        sW[((0 * 3 + v) * 4 + g) * WC + rr * FW + cc] = wmv[g];
-        sW[((1 * 3 + v) * 4 + g) * WC + rr * FW + cc] = wpv[g];
+        for (int g = 0; g < 4; ++g) {
+          sW[((0 * 3 + v) * 4 + g) * WC + rr * FW + cc] = wmv[g];
+          sW[((1 * 3 + v) * 4 + g) * WC + rr * FW + cc] = wpv[g];
+        }
       }
-    }
-    if constexpr (MODE == 1) {  // fills the last, partial round of the second sweeps
-      if (has_src) src_sweeps_split();
     }
     __syncthreads();
     // Rusanov at faces f = i0 .. i0+TX (ff), rows rr; left = WP(cell f-1) (cc = ff), right = WM(f)
     auto xface = [&](int f, int g, double& F0, double& F1, double& F2) {
       const int ff = f % (TX + 1), rr = f / (TX + 1);
       const int L = rr * FW + ff, R = rr * FW + ff + 1;
-      rusanov<MODE == 1>(gr.g, sW[((1 * 3 + 0) * 4 + g) * WC + L], sW[((1 * 3 + 1) * 4 + g) * WC + L],
+      if constexpr (MODE == 1)
+        split_flux(WC, g, L, R, SV(1, rr + 3, ff + 2), SV(2, rr + 3, ff + 2), SV(1, rr + 3, ff + 3),
+                   SV(2, rr + 3, ff + 3), 0, F0, F1, F2);
+      else
+        rusanov(gr.g, sW[((1 * 3 + 0) * 4 + g) * WC + L], sW[((1 * 3 + 1) * 4 + g) * WC + L],
               sW[((1 * 3 + 2) * 4 + g) * WC + L], sW[((0 * 3 + 0) * 4 + g) * WC + R],
               sW[((0 * 3 + 1) * 4 + g) * WC + R], sW[((0 * 3 + 2) * 4 + g) * WC + R], F0, F1, F2);
     };
@@ -462,48 +544,51 @@ __device__ __forceinline__ void rhs_tile(const RhsArgs& a, const RhsTma* tm, con
     __syncthreads();
     // second sweeps along x; cells: cols i0..i0+TX-1 (cc), rows j0-1..j0+TY (rr)
     constexpr int WC = FH * TX;
-    for (int it = tid; it < 3 * WC; it += NT) {
-      int cc = it % TX, rest = it / TX, rr = rest % FH, v = rest / FH;
-      double wmv[4], wpv[4];
-      const double Vc = SV(v, rr + 2, cc + 3);
-      const int gr_row = j0 - 1 + rr;
-      if constexpr (MODE == 1) {
-        float dm[4], dp[4];
-        f2 q[5], w[4];
+    if constexpr (MODE == 1) {
+      // two neighbouring columns per item, whose stencils share four of six values
+      static_assert(TX % 2 == 0 && FW % 2 == 0, "column pairs");
+      constexpr int TX2 = TX / 2;
+      for (int it = tid; it < 3 * FH * TX2; it += NT) {
+        const int cc = 2 * (it % TX2), rest = it / TX2, rr = rest % FH, v = rest / FH;
+        unsigned long long t[6], h[6];
+        const unsigned long long* pt = &sTMP[(v * FH + rr) * FW + cc];
+        const unsigned long long* ph = &sVhl[(v * VY + rr + 2) * VX + cc + 1];
 #pragma unroll
-        for (int k = 0; k < 5; ++k) {  // k = 2 is the centre column: no offset
-          const f2 t = f2{sTMP[(v * FH + rr) * FW + cc + k]};
-          q[k] = (k == 2) ? t : add2(f2_splat(dev(v, rr + 2, cc + 1 + k, rr + 2, cc + 3)), t);
+        for (int k = 0; k < 6; k += 2) ld2(pt + k, t[k], t[k + 1]);
+        h[0] = ph[0];
+        ld2(ph + 1, h[1], h[2]);
+        ld2(ph + 3, h[3], h[4]);
+        h[5] = ph[5];
+        f2 w[2][4];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          f2 q[5];
+#pragma unroll
+          for (int k = 0; k < 5; ++k)  // k = 2 is the centre column: no offset
+            q[k] = (k == 2) ? f2{t[k + e]}
+                            : add2(f2_splat(dev_of(h[k + e], h[2 + e])), f2{t[k + e]});
+          weno5_second_x2(q[0], q[1], q[2], q[3], q[4], w[e]);
         }
-        weno5_second_x2(q[0], q[1], q[2], q[3], q[4], w);
-#pragma unroll
-        for (int g = 0; g < 4; ++g) f2_unpack(w[g], dm[g], dp[g]);
-        if (v == 0 && gr_row != ny) {
-          limit_h_dev(gr, Vc, dm, dp, wmv, wpv);
-        } else {
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            wmv[g] = Vc + (double)dm[g];
-            wpv[g] = Vc + (double)dp[g];
-          }
-        }
-      } else {
+        const double Vc[2] = {SV(v, rr + 2, cc + 3), SV(v, rr + 2, cc + 4)};
+        const bool limited = j0 - 1 + rr != ny;
+        const bool lim[2] = {limited, limited};
+        put_pair(v, WC, rr * TX + cc, w, Vc, lim);
+      }
+    } else {
+      for (int it = tid; it < 3 * WC; it += NT) {
+        int cc = it % TX, rest = it / TX, rr = rest % FH, v = rest / FH;
+        double wmv[4], wpv[4];
+        const double Vc = SV(v, rr + 2, cc + 3);
         const T* cm = &sTM[(v * FH + rr) * FW + cc];
         const T* cp = &sTP[(v * FH + rr) * FW + cc];
-        T tm[4], tp[4];
-        weno5_second<T, EX>(cm[0], cm[1], cm[2], cm[3], cm[4], tm);
-        weno5_second<T, EX>(cp[0], cp[1], cp[2], cp[3], cp[4], tp);
+        weno5_second<T, EX>(cm[0], cm[1], cm[2], cm[3], cm[4], wmv);
+        weno5_second<T, EX>(cp[0], cp[1], cp[2], cp[3], cp[4], wpv);
+        if (v == 0 && j0 - 1 + rr != ny) limit_h(gr, Vc, wmv, wpv);
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
-          wmv[g] = tm[g];
-          wpv[g] = tp[g];
+          sW[((0 * 3 + v) * 4 + g) * WC + rr * TX + cc] = wmv[g];
+          sW[((1 * 3 + v) * 4 + g) * WC + rr * TX + cc] = wpv[g];
         }
-        if (v == 0 && gr_row != ny) limit_h(gr, Vc, wmv, wpv);
-      }
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        sW[((0 * 3 + v) * 4 + g) * WC + rr * TX + cc] = wmv[g];
-        sW[((1 * 3 + v) * 4 + g) * WC + rr * TX + cc] = wpv[g];
       }
     }
     __syncthreads();
@@ -512,7 +597,11 @@ __device__ __forceinline__ void rhs_tile(const RhsArgs& a, const RhsTma* tm, con
     auto yface = [&](int f, int g, double& F0, double& F2, double& F1) {
       const int cc = f % TX, fr = f / TX;
       const int L = fr * TX + cc, R = (fr + 1) * TX + cc;
-      rusanov<MODE == 1>(gr.g, sW[((1 * 3 + 0) * 4 + g) * WC + L], sW[((1 * 3 + 2) * 4 + g) * WC + L],
+      if constexpr (MODE == 1)
+        split_flux(WC, g, L, R, SV(1, fr + 2, cc + 3), SV(2, fr + 2, cc + 3), SV(1, fr + 3, cc + 3),
+                   SV(2, fr + 3, cc + 3), 1, F0, F1, F2);
+      else
+        rusanov(gr.g, sW[((1 * 3 + 0) * 4 + g) * WC + L], sW[((1 * 3 + 2) * 4 + g) * WC + L],
               sW[((1 * 3 + 1) * 4 + g) * WC + L], sW[((0 * 3 + 0) * 4 + g) * WC + R],
               sW[((0 * 3 + 2) * 4 + g) * WC + R], sW[((0 * 3 + 1) * 4 + g) * WC + R], F0, F1, F2);
     };
@@ -528,8 +617,8 @@ __device__ __forceinline__ void rhs_tile(const RhsArgs& a, const RhsTma* tm, con
   }
 
   // ======================= source term (depth only) =======================
-  // (the split form's y sweeps ran in the x second-sweep phase)
   if (has_src) {
+    src_sweeps_split();
     if constexpr (MODE == 0) {
       for (int it = NT - 1 - tid; it < TY * SW_; it += NT) {  // reversed: balances the y faces
         int cc = it % SW_, rr = it / SW_;
@@ -755,15 +844,22 @@ __device__ __forceinline__ void rhs_tile(const RhsArgs& a, const RhsTma* tm, con
 #undef SV
 }
 
+// Split form: bound by instruction issue (56%), the reciprocal and conversion unit (52%)
+// and shared-memory wavefronts (58%) in turn from phase to phase, so what helped was more
+// blocks to overlap phases and fewer loads: three blocks per SM (75 KB and 80 registers;
+// two of 103 KB before), the velocities' face values as FP32 deviations, two columns per
+// item (16-byte loads, shared stencil values) and the limiter left early where no
+// deviation can limit.  2048^2 island, one launch: 666 -> 553 us (256 threads; 288 or 320
+// at three blocks spill: 680, 667).
 template <int MODE>
-__global__ void __launch_bounds__(RHS_NT, 2)
+__global__ void __launch_bounds__(RHS_NT, MODE == 1 ? 3 : 2)
     rhs_kernel(const RhsArgs a, const __grid_constant__ RhsTma tm) {
   rhs_tile<MODE>(a, &tm, blockIdx.x * RHS_TX, blockIdx.y * RHS_TY);
 }
 
 // Up to kRhsGroup states of one grid, block z of the grid state z, in tiles of TX x TX.
 template <int MODE, int TX>
-__global__ void __launch_bounds__(RHS_NT, 2) rhs_group_kernel(const __grid_constant__ RhsGroup g) {
+__global__ void __launch_bounds__(RHS_NT, MODE == 1 ? 3 : 2) rhs_group_kernel(const __grid_constant__ RhsGroup g) {
   static_assert(sizeof(RhsArgs) % 8 == 0 && sizeof(RhsArgs) / 8 <= RHS_NT, "descriptor copy");
   __shared__ __align__(16) RhsArgs sa;
   if (threadIdx.x < sizeof(RhsArgs) / 8)
@@ -789,7 +885,7 @@ static cudaError_t launch_group(const RhsGroup& g, int n, cudaStream_t s) {
 // Ensembles: CTA b computes tile (work[b].y, work[b].z) of problem work[b].x, whose
 // descriptor is staged in shared memory; one launch covers every problem's tiles.
 template <int MODE>
-__global__ void __launch_bounds__(RHS_NT, 2)
+__global__ void __launch_bounds__(RHS_NT, MODE == 1 ? 3 : 2)
     rhs_batch_kernel(const RhsArgs* __restrict__ descs, const int4* __restrict__ work) {
   static_assert(sizeof(RhsArgs) % 8 == 0 && sizeof(RhsArgs) / 8 <= RHS_NT, "descriptor copy");
   __shared__ __align__(16) RhsArgs sa;
