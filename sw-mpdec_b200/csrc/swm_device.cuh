@@ -131,6 +131,33 @@ __device__ __forceinline__ double div_mk(double x, double y, double r) {
   e = fma(-q, y, x);
   return fma(e, r, q);
 }
+// RN(1/y) without a branch, for y in mk_range whose significand is not all ones
+// (mk_plain): the hardware's approximation (relative error below 2^-20), one third-order
+// step r (1 + e + e^2), e = 1 - y r, which leaves it within one ulp, and Markstein's final
+// step r + r (1 - y r), which from there rounds correctly (same references; the all-ones
+// significand is its one exception).  __drcp_rn gives the same value, but with a branch
+// each time, which kept the WENO's seven reciprocals per stencil apart.
+__device__ __forceinline__ double rcp_mk(double y) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(y));
+  double e = fma(-y, r, 1.0);
+  e = fma(e, e, e);
+  r = fma(r, e, r);
+  e = fma(-y, r, 1.0);
+  return fma(r, e, r);
+}
+// false for some y whose significand's low 32 bits are all ones, and for all whose
+// significand is
+__device__ __forceinline__ bool mk_plain(double y) { return __double2loint(y) != -1; }
+// x / y from r = RN(1/y) and rl = r (1 - y r), its residual part (mk_low): x (r + rl) is
+// within 0.5 ulp + 2^-48 ulp of the quotient, from where one residual correction rounds
+// correctly (as div_mk's second does).  One operation fewer per quotient than div_mk, for
+// two per reciprocal.
+__device__ __forceinline__ double mk_low(double y, double r) { return fma(-y, r, 1.0) * r; }
+__device__ __forceinline__ double div_mk2(double x, double y, double r, double rl) {
+  const double q = fma(x, r, x * rl);
+  return fma(fma(-q, y, x), r, q);
+}
 // The IEEE division, kept out of line: it only serves operands outside mk_range.
 static __device__ __noinline__ double div_ieee(double x, double y) { return x / y; }
 // x / y for any operands; a zero numerator gives x * r, the correctly signed zero
@@ -154,10 +181,22 @@ __device__ __forceinline__ float weno_eps<float>() { return kWenoEpsF; }
 // 3*(13/12 (a-2b+c)^2 + 1/4 (a-4b+3c)^2): non-negative by construction and free of
 // the cancellation of the expanded form, which in FP32 can drive eps+beta to zero
 // (and the weights to inf/inf) on nearly constant stencils.
-template <typename T, bool EXACT>
+template <typename T, bool EXACT, bool FUSE>
 __device__ __forceinline__ void weno_d(T qm2, T qm1, T q0, T qp1, T qp2, T& d1, T& d2, T& d3) {
   T beta1, beta2, beta3;
-  if (EXACT) {
+  if constexpr (EXACT && FUSE) {
+    // 4 a a -+ x as one fused operation on a a: the factor 4 is exact, so the same value
+    // (for a a normal; a subnormal one is far below eps)
+    const T third = T(1.0) / T(3.0), c10 = T(10.0) * q0 * q0, c13 = T(13.0) * q0;
+    beta1 = third * (fma(T(4.0), qm2 * qm2, -(T(19.0) * qm2 * qm1)) + T(25.0) * qm1 * qm1 +
+                     T(11.0) * qm2 * q0 - T(31.0) * qm1 * q0 + c10);
+    beta2 = third * fma(T(4.0), qp1 * qp1,
+                        fma(T(4.0), qm1 * qm1, -(T(13.0) * qm1 * q0)) + c13 * q0 +
+                            T(5.0) * qm1 * qp1 - c13 * qp1);
+    beta3 = third * fma(T(4.0), qp2 * qp2,
+                        c10 - T(31.0) * q0 * qp1 + T(25.0) * qp1 * qp1 + T(11.0) * q0 * qp2 -
+                            T(19.0) * qp1 * qp2);
+  } else if constexpr (EXACT) {
     beta1 = (T(1.0) / T(3.0)) * (T(4.0) * qm2 * qm2 - T(19.0) * qm2 * qm1 + T(25.0) * qm1 * qm1 +
                                  T(11.0) * qm2 * q0 - T(31.0) * qm1 * q0 + T(10.0) * q0 * q0);
     beta2 = (T(1.0) / T(3.0)) * (T(4.0) * qm1 * qm1 - T(13.0) * qm1 * q0 + T(13.0) * q0 * q0 +
@@ -190,13 +229,28 @@ enum { kDivRcp = 0, kDivMk = 1, kDivIeee = 2 };
 //         [2^-400, 2^400), alpha_k and their sum lie in [2^-405, 2^402], so every
 //         quotient (>= 2^-807) and residual stays normal and div_mk is exact.
 //  else : the same weights as products with the reciprocals.
-template <typename T, int DIV>
-__device__ __forceinline__ T weno_point(T g1, T g2, T g3, T d1, T d2, T d3, T i1, T i2, T i3, T W1,
-                                        T W2, T W3) {
+template <typename T>
+struct WenoRcp {  // i_k = RN(1/d_k); kDivMk second sweeps: their residual parts
+  T i1, i2, i3, l1, l2, l3;
+};
+template <typename T, int DIV, bool LOW>
+__device__ __forceinline__ T weno_point(T g1, T g2, T g3, T d1, T d2, T d3, const WenoRcp<T>& c,
+                                        T W1, T W2, T W3, bool& ok) {
+  const T i1 = c.i1, i2 = c.i2, i3 = c.i3;
   if constexpr (DIV == kDivMk) {
-    T a1 = div_mk(g1, d1, i1), a2 = div_mk(g2, d2, i2), a3 = div_mk(g3, d3, i3);
-    const T s = a1 + a2 + a3, rs = rcp_(s);
-    return div_mk(a1, s, rs) * W1 + div_mk(a2, s, rs) * W2 + div_mk(a3, s, rs) * W3;
+    T a1, a2, a3;
+    if constexpr (LOW) {
+      a1 = div_mk2(g1, d1, i1, c.l1);
+      a2 = div_mk2(g2, d2, i2, c.l2);
+      a3 = div_mk2(g3, d3, i3, c.l3);
+    } else {
+      a1 = div_mk(g1, d1, i1);
+      a2 = div_mk(g2, d2, i2);
+      a3 = div_mk(g3, d3, i3);
+    }
+    const T s = a1 + a2 + a3, rs = rcp_mk(s), ls = mk_low(s, rs);
+    ok = ok && mk_plain(s);
+    return div_mk2(a1, s, rs, ls) * W1 + div_mk2(a2, s, rs, ls) * W2 + div_mk2(a3, s, rs, ls) * W3;
   } else if constexpr (DIV == kDivIeee) {
     T a1 = g1 / d1, a2 = g2 / d2, a3 = g3 / d3;
     return a1 / (a1 + a2 + a3) * W1 + a2 / (a1 + a2 + a3) * W2 + a3 / (a1 + a2 + a3) * W3;
@@ -206,40 +260,54 @@ __device__ __forceinline__ T weno_point(T g1, T g2, T g3, T d1, T d2, T d3, T i1
   }
 }
 
+// The reciprocals of the smoothness indicators; kDivMk: false when one is outside what
+// rcp_mk and div_mk take.
 template <int DIV>
-__device__ __forceinline__ bool div_ok(double d1, double d2, double d3) {
-  return DIV != kDivMk || (mk_range(d1) && mk_range(d2) && mk_range(d3));
-}
-template <int DIV>
-__device__ __forceinline__ bool div_ok(float, float, float) {
-  return true;
-}
-
-// WENO5_FirstSweep (reconstruction.f90:673-755): cell-face means at x_{i-1/2},
-// x_{i+1/2}.  Returns false (nothing written) when kDivMk's range check fails.
-template <typename T, bool EXACT, int DIV>
-__device__ __forceinline__ bool weno5_first_div(T qm2, T qm1, T q0, T qp1, T qp2, T& wm, T& wp) {
-  T d1, d2, d3;
-  weno_d<T, EXACT>(qm2, qm1, q0, qp1, qp2, d1, d2, d3);
-  if (!div_ok<DIV>(d1, d2, d3)) return false;
-  T i1 = T(0), i2 = T(0), i3 = T(0);
-  if constexpr (DIV != kDivIeee) {
+__device__ __forceinline__ bool weno_rcp(double d1, double d2, double d3, double& i1, double& i2,
+                                         double& i3) {
+  if constexpr (DIV == kDivMk) {
+    i1 = rcp_mk(d1);
+    i2 = rcp_mk(d2);
+    i3 = rcp_mk(d3);
+    return mk_range(d1) && mk_range(d2) && mk_range(d3) && mk_plain(d1) && mk_plain(d2) &&
+           mk_plain(d3);
+  } else if constexpr (DIV == kDivRcp) {
     i1 = rcp_(d1);
     i2 = rcp_(d2);
     i3 = rcp_(d3);
   }
+  return true;
+}
+template <int DIV>
+__device__ __forceinline__ bool weno_rcp(float d1, float d2, float d3, float& i1, float& i2,
+                                         float& i3) {
+  i1 = rcp_(d1);
+  i2 = rcp_(d2);
+  i3 = rcp_(d3);
+  return true;
+}
+
+// WENO5_FirstSweep (reconstruction.f90:673-755): cell-face means at x_{i-1/2},
+// x_{i+1/2}.  Returns false when kDivMk does not apply (the results are then not valid);
+// no branch before that, so that a stencil's divisions overlap.
+template <typename T, bool EXACT, int DIV>
+__device__ __forceinline__ bool weno5_first_div(T qm2, T qm1, T q0, T qp1, T qp2, T& wm, T& wp) {
+  T d1, d2, d3;
+  weno_d<T, EXACT, DIV == kDivMk>(qm2, qm1, q0, qp1, qp2, d1, d2, d3);
+  WenoRcp<T> c{};
+  bool ok = weno_rcp<DIV>(d1, d2, d3, c.i1, c.i2, c.i3);
   const T s6 = T(1.0) / T(6.0);
   T W1 = s6 * (-qm2 + T(5.0) * qm1 + T(2.0) * q0);
   T W2 = s6 * (T(2.0) * qm1 + T(5.0) * q0 - qp1);
   T W3 = s6 * (T(11.0) * q0 - T(7.0) * qp1 + T(2.0) * qp2);
-  wm = weno_point<T, DIV>(T(3.0) / T(10.0), T(3.0) / T(5.0), T(1.0) / T(10.0), d1, d2, d3, i1, i2,
-                          i3, W1, W2, W3);
+  wm = weno_point<T, DIV, false>(T(3.0) / T(10.0), T(3.0) / T(5.0), T(1.0) / T(10.0), d1, d2, d3, c,
+                          W1, W2, W3, ok);
   W1 = s6 * (T(2.0) * qm2 - T(7.0) * qm1 + T(11.0) * q0);
   W2 = s6 * (-qm1 + T(5.0) * q0 + T(2.0) * qp1);
   W3 = s6 * (T(2.0) * q0 + T(5.0) * qp1 - qp2);
-  wp = weno_point<T, DIV>(T(1.0) / T(10.0), T(3.0) / T(5.0), T(3.0) / T(10.0), d1, d2, d3, i1, i2,
-                          i3, W1, W2, W3);
-  return true;
+  wp = weno_point<T, DIV, false>(T(1.0) / T(10.0), T(3.0) / T(5.0), T(3.0) / T(10.0), d1, d2, d3, c,
+                          W1, W2, W3, ok);
+  return ok;
 }
 
 // WENO5_SecondSweep (reconstruction.f90:999-1136): values at the 4 Gauss nodes.
@@ -249,36 +317,36 @@ __device__ __forceinline__ bool weno5_first_div(T qm2, T qm1, T q0, T qp1, T qp2
 template <typename T, bool EXACT, int DIV>
 __device__ __forceinline__ bool weno5_second_div(T qm2, T qm1, T q0, T qp1, T qp2, T w[4]) {
   T d1, d2, d3;
-  weno_d<T, EXACT>(qm2, qm1, q0, qp1, qp2, d1, d2, d3);
-  if (!div_ok<DIV>(d1, d2, d3)) return false;
-  T i1 = T(0), i2 = T(0), i3 = T(0);
-  if constexpr (DIV != kDivIeee) {
-    i1 = rcp_(d1);
-    i2 = rcp_(d2);
-    i3 = rcp_(d3);
+  weno_d<T, EXACT, DIV == kDivMk>(qm2, qm1, q0, qp1, qp2, d1, d2, d3);
+  WenoRcp<T> c{};
+  bool ok = weno_rcp<DIV>(d1, d2, d3, c.i1, c.i2, c.i3);
+  if constexpr (DIV == kDivMk) {
+    c.l1 = mk_low(d1, c.i1);
+    c.l2 = mk_low(d2, c.i2);
+    c.l3 = mk_low(d3, c.i3);
   }
   T W1, W2, W3;
   W1 = T(-0.1642562761719537) * qm2 + T(0.7590807081409336) * qm1 + T(0.4051755680310201) * q0;
   W2 = T(0.2663118796250726) * qm1 + T(0.8979443965468811) * q0 - T(0.1642562761719537) * qp1;
   W3 = T(1.6968800354220990) * q0 - T(0.9631919150471715) * qp1 + T(0.2663118796250726) * qp2;
-  w[0] = weno_point<T, DIV>(T(0.2658420974778319), T(0.6112504900322486), T(0.1229074124899195),
-                            d1, d2, d3, i1, i2, i3, W1, W2, W3);
+  w[0] = weno_point<T, DIV, true>(T(0.2658420974778319), T(0.6112504900322486), T(0.1229074124899195),
+                            d1, d2, d3, c, W1, W2, W3, ok);
   W1 = T(-0.1122135388132497) * qm2 + T(0.3944175994189276) * qm1 + T(0.7177959393943222) * q0;
   W2 = T(0.0577769829791784) * qm1 + T(1.0544365558340714) * q0 - T(0.1122135388132497) * qp1;
   W3 = T(1.2277675047716066) * q0 - T(0.2855444877507849) * qp1 + T(0.0577769829791784) * qp2;
-  w[1] = weno_point<T, DIV>(T(0.1281641584355059), T(0.5219691498503563), T(0.3498666917141379),
-                            d1, d2, d3, i1, i2, i3, W1, W2, W3);
+  w[1] = weno_point<T, DIV, true>(T(0.1281641584355059), T(0.5219691498503563), T(0.3498666917141379),
+                            d1, d2, d3, c, W1, W2, W3, ok);
   W1 = T(0.0577769829791784) * qm2 - T(0.2855444877507849) * qm1 + T(1.2277675047716066) * q0;
   W2 = T(-0.1122135388132497) * qm1 + T(1.0544365558340714) * q0 + T(0.0577769829791784) * qp1;
   W3 = T(0.7177959393943222) * q0 + T(0.3944175994189276) * qp1 - T(0.1122135388132497) * qp2;
-  w[2] = weno_point<T, DIV>(T(0.3498666917141379), T(0.5219691498503563), T(0.1281641584355059),
-                            d1, d2, d3, i1, i2, i3, W1, W2, W3);
+  w[2] = weno_point<T, DIV, true>(T(0.3498666917141379), T(0.5219691498503563), T(0.1281641584355059),
+                            d1, d2, d3, c, W1, W2, W3, ok);
   W1 = T(0.2663118796250726) * qm2 - T(0.9631919150471715) * qm1 + T(1.6968800354220990) * q0;
   W2 = T(-0.1642562761719537) * qm1 + T(0.8979443965468811) * q0 + T(0.2663118796250726) * qp1;
   W3 = T(0.4051755680310201) * q0 + T(0.7590807081409336) * qp1 - T(0.1642562761719537) * qp2;
-  w[3] = weno_point<T, DIV>(T(0.1229074124899195), T(0.6112504900322486), T(0.2658420974778319),
-                            d1, d2, d3, i1, i2, i3, W1, W2, W3);
-  return true;
+  w[3] = weno_point<T, DIV, true>(T(0.1229074124899195), T(0.6112504900322486), T(0.2658420974778319),
+                            d1, d2, d3, c, W1, W2, W3, ok);
+  return ok;
 }
 
 // Out-of-line IEEE versions for EXACT reconstructions whose indicators leave mk_range
@@ -544,6 +612,28 @@ __device__ __forceinline__ void rusanov(double g, double hL, double nL, double t
 // Positivity limiter on the 4 face values of h of one cell
 // (finitevolume.f90:671-691, identical for x and y).
 __device__ __forceinline__ void limit_h(const Grid& gr, double Vc, double wm[4], double wp[4]) {
+  // No face value further from the cell's depth than MIN_DEPTH is: nothing limits.  The
+  // minimum below is one of the face values or csi, whose distance from Vc is at most a
+  // fifth of the largest face value's plus rounding (a few ulp of Vc), so every quotient
+  // is >= 1 and theta exactly 1.  Compared on the high words, 2^-19 on the safe side.
+  const double ta0 = Vc - kMinDepth;
+  const int hta = __double2hiint(ta0) & 0x7fffffff;
+  double dm[4], dp[4];
+  int most = 0;
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    dm[g] = wm[g] - Vc;
+    dp[g] = wp[g] - Vc;
+    most = max(most, max(__double2hiint(dm[g]) & 0x7fffffff, __double2hiint(dp[g]) & 0x7fffffff));
+  }
+  if (hta >= most + 2 && hta >= (__double2hiint(Vc) & 0x7fffffff) - (30 << 20)) {
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      wp[g] = Vc + dp[g];
+      wm[g] = Vc + dm[g];
+    }
+    return;
+  }
   double alpha = 0., beta = 0.;
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
