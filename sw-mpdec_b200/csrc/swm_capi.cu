@@ -904,9 +904,8 @@ int swm_create(const swm_params* p, swm_handle* out) {
         cudaSuccess)
       return cleanup(fail(SWM_ERR_CUDA, "bathymetry table upload failed"));
   }
-  s->jac_grid = {jacobi_grid_blocks(jacobi_form(s->p), true, s->device),
-                 jacobi_grid_blocks(jacobi_form(s->p), false, s->device)};
-  if (s->jac_grid.tile_blocks < 1 || s->jac_grid.strip_blocks < 1)
+  s->jac_grid = jacobi_grid(jacobi_form(s->p), s->device);
+  if (s->jac_grid.tile_blocks < 1)
     return cleanup(fail(SWM_ERR_CUDA, "Jacobi kernel cannot be resident"));
   // the RHS kernels' shared-memory attribute is set on first launch
   if (cudaDeviceSynchronize() != cudaSuccess)

@@ -595,14 +595,16 @@ __device__ __noinline__ bool solve_exact(const ExactGrid& g, const Sys& y, SysSt
   return true;
 }
 
-// TILES: a block per tile (small grids), else a warp per chunk of a strip.
-template <int FORM, bool TILES>
+// TILES: a block per tile and passes of up to TILES sweeps (small grids); 0: a warp per
+// chunk of a strip, passes of up to kPassT.
+template <int FORM, int TILES>
 __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
                                   TILES ? 1 : (FORM == kSysRecip ? 3 : 2))
     jacobi_kernel(const __grid_constant__ JacobiGroup a) {
   using G = Strip<FORM>;
-  using TG = Tile<FORM>;
-  constexpr int T = kPassT, NW = TILES ? kTileWarps : kStripWarps;
+  constexpr int T = TILES ? TILES : kPassT, NW = TILES ? kTileWarps : kStripWarps;
+  using TG = Tile<FORM, T>;
+  static_assert(T <= kMaxBlock, "residual sums of a pass");
   extern __shared__ __align__(16) unsigned char jring[];
   __shared__ SysState st[kMaxSys];
   __shared__ double s_sum[NW][kMaxSys][T + 1], s_tot[kMaxSys][T + 1];
@@ -612,9 +614,9 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int blk = a.block < 1 ? 1 : (a.block > T ? T : a.block);
   const double thresh = limbs_value(a.thresh[0], a.thresh[1], a.thresh[2]);
-  const int strips = (a.nx + G::U - 1) / G::U, warps = gridDim.x * kStripWarps;
+  const int strips = (a.nx + TG::UX - 1) / TG::UX, warps = gridDim.x * kStripWarps;
   const int tiles = TILES ? strips * ((a.ny + TG::UY - 1) / TG::UY) : 0;
-  static_assert(G::U == TG::UX, "strips and tiles deliver the same columns");
+  static_assert(TILES || G::U == TG::UX, "strips deliver as many columns as tiles");
   double2* ring = reinterpret_cast<double2*>(jring + (TILES ? 0 : warp * G::warp_bytes));
   // the systems still iterating and the pass's split, by warp 0
   auto plan = [&]() {
@@ -656,15 +658,6 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
     for (int q = lane; q < kMaxSys * (T + 1); q += 32) (&s_sum[warp][0][0])[q] = 0.;
     __syncwarp();
     const int nact = s_nact;
-    auto flush = [&](int q, int Tp, double (&sum)[T + 1]) {
-#pragma unroll
-      for (int t = 0; t <= T; ++t) {
-        if (t > Tp) break;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum[t] += __shfl_down_sync(0xffffffffu, sum[t], o);
-        if (lane == 0) s_sum[warp][q][t] += sum[t];
-      }
-    };
     auto aligned = [&](const JacobiSys& y, const SysState& S) {
       unsigned long long al = (unsigned long long)S.xin | (unsigned long long)S.xout |
                               (unsigned long long)y.b;
@@ -681,16 +674,14 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
         const JacobiSys& y = a.sys[q];
         const SysState& S = st[q];
         const int Tp = S.Tp, strip = tile % strips, j0 = (tile / strips) * TG::UY;
-        const StripLane L = strip_lane<FORM>(a.nx, a.nx, strip, aligned(y, S));
+        const StripLane L = strip_lane<T>(a.nx, a.nx, strip, aligned(y, S));
         if (held != q * tiles + tile) {  // a block with one tile keeps its rows of the system
           held = q * tiles + tile;
           held_bad = false;
           tile_rows<FORM>(y, a.nx, a.ny, a.nx, wrap(j0 + warp * TG::RW - T, a.ny), L, cf, held_bad);
         }
-        double sum[T + 1];
-        tile_pass<FORM>(S.xin, S.xout, a.nx, a.ny, a.nx, Tp, S.first != 0, j0, L, cf, held_bad,
-                        ring, sum);
-        flush(q, Tp, sum);
+        tile_pass<FORM, T>(S.xin, S.xout, a.nx, a.ny, a.nx, Tp, S.first != 0, j0, L, cf, held_bad,
+                           ring, s_sum[warp][q]);
         __syncthreads();  // the edge rows are read
       }
     } else {
@@ -707,7 +698,12 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
         double sum[T + 1];
         strip_pass<FORM>(y, S.xin, S.xout, a.nx, a.ny, a.nx, a.nx, Tp, S.first != 0, strip, j0,
                          rows, aligned(y, S), ring, sum);
-        flush(q, Tp, sum);
+#pragma unroll
+        for (int t = 0; t <= T; ++t) {
+          if (t > Tp) break;
+          const double v = warp_sum(sum[t]);
+          if (lane == 0) s_sum[warp][q][t] += v;
+        }
       }
     }
     __syncthreads();
@@ -776,21 +772,25 @@ struct JacobiLaunch {
   size_t smem;
 };
 
+template <int FORM, int T>
+static JacobiLaunch jacobi_tiles() {
+  using G = Tile<FORM, T>;
+  return {reinterpret_cast<const void*>(&jacobi_kernel<FORM, T>), kTileNT, G::UX, G::UY, G::bytes};
+}
+
 template <int FORM>
-static JacobiLaunch jacobi_launch_of(bool tiles) {
-  if (tiles)
-    return {reinterpret_cast<const void*>(&jacobi_kernel<FORM, true>), kTileNT, Tile<FORM>::UX,
-            Tile<FORM>::UY, Tile<FORM>::bytes};
-  return {reinterpret_cast<const void*>(&jacobi_kernel<FORM, false>), kStripNT, Strip<FORM>::U, 8,
+static JacobiLaunch jacobi_launch_of(int tiles) {
+  if (tiles) return tiles == 8 ? jacobi_tiles<FORM, 8>() : jacobi_tiles<FORM, 4>();
+  return {reinterpret_cast<const void*>(&jacobi_kernel<FORM, 0>), kStripNT, Strip<FORM>::U, 8,
           Strip<FORM>::bytes};
 }
 
-static JacobiLaunch jacobi_pick(int form, bool tiles) {
+static JacobiLaunch jacobi_pick(int form, int tiles) {
   if (form == kSysRecip) return jacobi_launch_of<kSysRecip>(tiles);
   return form == kSysDiv ? jacobi_launch_of<kSysDiv>(tiles) : jacobi_launch_of<kSysCsr>(tiles);
 }
 
-int jacobi_grid_blocks(int form, bool tiles, int device) {
+int jacobi_grid_blocks(int form, int tiles, int device) {
   const JacobiLaunch l = jacobi_pick(form, tiles);
   int per_sm = 0, sms = 0;
   cudaFuncSetAttribute(l.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem);
@@ -801,24 +801,35 @@ int jacobi_grid_blocks(int form, bool tiles, int device) {
   return per_sm < 1 ? -1 : per_sm * sms;
 }
 
-// Tiles while they make at most kTileWaves rounds over the resident blocks, strips beyond.
-// Measured per step (13 solves of 10 to 14 sweeps, B200), tiles against strips: split
-// 256^2 182 / 266 us, 512^2 (300 tiles of a launch's three systems over 148 blocks) 315 /
-// 346, 768^2 (630 tiles) 553 / 479, 2048^2 2675 / 1920; FP64 512^2 (390 tiles) 393 / 458,
-// 768^2 (840 tiles) 745 / 635.
+JacobiGrid jacobi_grid(int form, int device) {
+  const int t8 = jacobi_grid_blocks(form, 8, device), t4 = jacobi_grid_blocks(form, 4, device);
+  const JacobiGrid g{t8 < t4 ? t8 : t4, jacobi_grid_blocks(form, 0, device)};
+  return g.tile_blocks < 1 || g.strip_blocks < 1 ? JacobiGrid{0, 0} : g;
+}
+
+// Which pieces a solve is cut into, by how many rounds they make over the resident blocks.
+// Measured per step (13 solves of 10 to 14 sweeps, B200), 8-sweep tiles / 4-sweep tiles /
+// strips: split 50^2 152 / 182 / 280 us, 320^2 (168 and 126 tiles of a launch's three
+// systems over 148 blocks) 192 / 178 / -, 512^2 (396 and 300) 257 / 305 / 346, 768^2 (864 and
+// 630) 473 / 553 / 448, 2048^2 - / 2675 / 1792; FP64 257^2 mPDeC2 70 / 95 / 163, 600^2 (741
+// and 525) 532 / - / 469.  One round of either length beats two (a block keeps its rows of
+// the system for the whole solve), the longer passes win up to three rounds, strips beyond.
 constexpr int kTileWaves = 3;
 
 cudaError_t launch_jacobi(const JacobiGroup& a, const JacobiGrid& g, cudaStream_t s) {
-  JacobiLaunch l = jacobi_pick(a.form, true);
-  const long long tiles = (long long)a.nsys * ((a.nx + l.width - 1) / l.width) *
-                          ((a.ny + l.height - 1) / l.height);
-  long long blocks = tiles, most = g.tile_blocks;
-  if (tiles > (long long)kTileWaves * g.tile_blocks) {
-    l = jacobi_pick(a.form, false);
-    // no more blocks than chunks of `height` rows give work to
-    const long long items = (long long)a.nsys * ((a.nx + l.width - 1) / l.width) *
-                            ((a.ny + l.height - 1) / l.height);
-    blocks = (items + kStripWarps - 1) / kStripWarps;
+  auto pieces = [&](const JacobiLaunch& l) {  // tiles, or chunks of at least 8 rows
+    return (long long)a.nsys * ((a.nx + l.width - 1) / l.width) * ((a.ny + l.height - 1) / l.height);
+  };
+  const long long t8 = pieces(jacobi_pick(a.form, 8)), t4 = pieces(jacobi_pick(a.form, 4));
+  const long long round = g.tile_blocks;
+  const int tiles = t8 <= round ? 8
+                    : t4 <= round ? 4
+                    : t8 <= kTileWaves * round ? 8
+                    : t4 <= kTileWaves * round ? 4 : 0;
+  const JacobiLaunch l = jacobi_pick(a.form, tiles);
+  long long blocks = tiles == 8 ? t8 : t4, most = round;
+  if (tiles == 0) {
+    blocks = (pieces(l) + kStripWarps - 1) / kStripWarps;
     most = g.strip_blocks;
   }
   if (blocks > most) blocks = most;
@@ -906,8 +917,7 @@ __global__ void __launch_bounds__(kStripNT, FORM == kSysRecip ? 3 : 2)
 #pragma unroll
         for (int t = 0; t <= T; ++t) {
           if (t > Tp) break;
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) sum[t] += __shfl_xor_sync(0xffffffffu, sum[t], o);
+          sum[t] = warp_sum(sum[t]);
           if (lane == t && sum[t] != 0.) atomicAdd(&a.st[sys].sum[t], sum[t]);
         }
       }

@@ -326,10 +326,12 @@ cudaError_t launch_assemble(const AssembleArgs& a, bool csr, cudaStream_t s);
 cudaError_t launch_assemble_multi(const AssembleMultiArgs& a, bool csr, cudaStream_t s);
 // Resident blocks of the Jacobi kernel's two forms (swm_strip.cuh).
 struct JacobiGrid {
-  int tile_blocks, strip_blocks;
+  int tile_blocks, strip_blocks;  // tiles: the fewer of the two pass lengths' kernels
 };
 cudaError_t launch_jacobi(const JacobiGroup& a, const JacobiGrid& g, cudaStream_t s);
-int jacobi_grid_blocks(int form, bool tiles, int device);
+int jacobi_grid_blocks(int form, int tiles, int device);  // tiles: 8 or 4, 0 for strips
+// both, or {0, 0} when a kernel cannot be resident
+JacobiGrid jacobi_grid(int form, int device);
 cudaError_t launch_ghosted_to_planes(const double* G, int nx, int ny, double* h, double* hu,
                                      double* hv, cudaStream_t s);
 cudaError_t launch_planes_to_ghosted(const double* h, const double* hu, const double* hv, int nx,

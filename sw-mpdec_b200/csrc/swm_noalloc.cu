@@ -103,9 +103,8 @@ int swm_jacobi_noalloc(int nx, int ny, const double* cS, const double* cW, const
       ds.ready = true;
     }
     if (ds.grid.strip_blocks == 0) {
-      const swm::JacobiGrid g{swm::jacobi_grid_blocks(swm::kSysDiv, true, dev),
-                              swm::jacobi_grid_blocks(swm::kSysDiv, false, dev)};
-      if (g.tile_blocks < 1 || g.strip_blocks < 1)
+      const swm::JacobiGrid g = swm::jacobi_grid(swm::kSysDiv, dev);
+      if (g.tile_blocks < 1)
         return noalloc_fail(SWM_ERR_CUDA, "Jacobi kernel cannot be resident");
       ds.grid = g;
     }

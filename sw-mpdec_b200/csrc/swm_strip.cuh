@@ -7,7 +7,7 @@
 //          computes row s - t from the rows of x^{t-1} that the previous step and the
 //          previous sweep left in registers.  Rows come through a ring in shared memory
 //          that only their own lane reads, so there is no barrier in the walk;
-//  tiles   a block holds a 64-column tile, a few rows per warp; the warps exchange their
+//  tiles   (passes of up to 4 or 8 sweeps) a block holds a 64-column tile, a few rows per warp; the warps exchange their
 //          edge rows through shared memory after every sweep.
 // In both, west and east neighbours come from the next lanes, and each row of the system
 // is read once per pass (tiles: once per solve when every block has one tile).
@@ -65,16 +65,17 @@ struct StripLane {
   bool wide;        // the pair is one 16-byte word of every array
 };
 
-template <int FORM>
+// H halo columns on each side, U = kStripCols - 2 H delivered.
+template <int H>
 __device__ __forceinline__ StripLane strip_lane(int nx, int pitch, int strip, bool aligned) {
-  using G = Strip<FORM>;
-  const int lane = threadIdx.x & 31, i0 = strip * G::U;
+  constexpr int U = kStripCols - 2 * H;
+  const int lane = threadIdx.x & 31, i0 = strip * U;
   StripLane L;
-  const int q = 2 * lane - G::H;  // first column of the pair relative to the strip's own
+  const int q = 2 * lane - H;  // first column of the pair relative to the strip's own
   L.c0 = wrap(i0 + q, nx);
   L.c1 = L.c0 + 1 == nx ? 0 : L.c0 + 1;
-  L.own0 = q >= 0 && q < G::U && i0 + q < nx;
-  L.own1 = q >= 0 && q < G::U && i0 + q + 1 < nx;
+  L.own0 = q >= 0 && q < U && i0 + q < nx;
+  L.own1 = q >= 0 && q < U && i0 + q + 1 < nx;
   L.wide = aligned && (pitch & 1) == 0 && (L.c0 & 1) == 0 && L.c0 + 1 < nx;
   return L;
 }
@@ -230,7 +231,7 @@ __device__ __forceinline__ void strip_chunk(const Sys& y, const double* xin, dou
   using G = Strip<FORM>;
   constexpr int NS = kStripSlots;
   static_assert(NL % 2 == 0 && NL <= G::T, "row parities are static");
-  const StripLane L = strip_lane<FORM>(nx, pitch, strip, aligned);
+  const StripLane L = strip_lane<G::H>(nx, pitch, strip, aligned);
   double2* mine = ring + (threadIdx.x & 31);
   constexpr int SLOT = G::PL * 32;
   const int total = rows + 2 * Tp;  // input rows j0 - Tp .. j0 + rows - 1 + Tp
@@ -322,16 +323,17 @@ __device__ __forceinline__ void strip_pass(const Sys& y, const double* xin, doub
 }
 
 // ---------------------------------------------------------------------------
-// Tiles: kTileWarps warps of RW rows each, kPassT of the tile's rows and columns halo on
-// each side.  RW is what a thread's registers hold at one block of kTileNT threads per SM.
+// Tiles: kTileWarps warps of RW rows each, T of the tile's rows and columns halo on each
+// side for passes of at most T sweeps.  RW is what a thread's registers hold at one block
+// of kTileNT threads per SM.
 // ---------------------------------------------------------------------------
 constexpr int kTileWarps = 12, kTileNT = 32 * kTileWarps;
 
-template <int FORM>
+template <int FORM, int T>
 struct Tile {
   static constexpr int RW = FORM == kSysRecip ? 5 : 4;
   static constexpr int ROWS = kTileWarps * RW;
-  static constexpr int UX = kStripCols - 2 * kPassT, UY = ROWS - 2 * kPassT;  // delivered
+  static constexpr int UX = kStripCols - 2 * T, UY = ROWS - 2 * T;  // delivered
   // edge rows of x, by sweep parity: [2][warp][top, bottom][lane]
   static constexpr size_t bytes = sizeof(double2) * 2 * kTileWarps * 2 * 32;
 };
@@ -375,16 +377,24 @@ __device__ __forceinline__ void tile_rows(const JacobiSys& y, int nx, int ny, in
   for (int r = 0; r < RW; ++r) strip_rcp<FORM>(cf[r], bad);
 }
 
-// Tp <= kPassT sweeps over the tile at (i0, j0) whose rows of the system are in cf; sums
-// as strip_chunk's.  Every thread of the block takes part.
-template <int FORM>
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Tp <= T sweeps over the tile at (i0, j0) whose rows of the system are in cf; the warp's
+// residual sums are added to sum[0..T] (shared memory) as strip_chunk's.  Every thread of
+// the block takes part.
+template <int FORM, int T>
 __device__ __forceinline__ void tile_pass(const double* xin, double* xout, int nx, int ny,
                                           int pitch, int Tp, bool first, int j0,
-                                          const StripLane& L, const StripRow<FORM> (&cf)[Tile<FORM>::RW],
-                                          bool bad, double2* edge, double (&sum)[kPassT + 1]) {
-  constexpr int RW = Tile<FORM>::RW;
+                                          const StripLane& L,
+                                          const StripRow<FORM> (&cf)[Tile<FORM, T>::RW], bool bad,
+                                          double2* edge, double* sum) {
+  constexpr int RW = Tile<FORM, T>::RW;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r0 = warp * RW - kPassT;  // this warp's first row relative to the tile's own
+  const int r0 = warp * RW - T;  // this warp's first row relative to the tile's own
   const int g0 = wrap(j0 + r0, ny);
   double2 x[RW];
   int gj = g0;
@@ -394,20 +404,22 @@ __device__ __forceinline__ void tile_pass(const double* xin, double* xout, int n
     gj = gj + 1 == ny ? 0 : gj + 1;
   }
   // rows this tile delivers, and counts
-  const unsigned rows = min(Tile<FORM>::UY, ny - j0);
-#pragma unroll
-  for (int t = 0; t <= kPassT; ++t) sum[t] = 0.;
+  const unsigned rows = min(Tile<FORM, T>::UY, ny - j0);
+  auto put = [&](int t, double s) {
+    s = warp_sum(s);
+    if (lane == 0) sum[t] += s;
+  };
   if (first) {
+    double s = 0.;
 #pragma unroll
     for (int r = 0; r < RW; ++r) {
       const bool in = (unsigned)(r0 + r) < rows;
-      if (in && L.own0) sum[0] = __dadd_rn(sum[0], fabs(x[r].x));
-      if (in && L.own1) sum[0] = __dadd_rn(sum[0], fabs(x[r].y));
+      if (in && L.own0) s = __dadd_rn(s, fabs(x[r].x));
+      if (in && L.own1) s = __dadd_rn(s, fabs(x[r].y));
     }
+    put(0, s);
   }
-#pragma unroll
-  for (int t = 1; t <= kPassT; ++t) {
-    if (t > Tp) break;
+  for (int t = 1; t <= Tp; ++t) {
     double2* e = edge + (t & 1) * (kTileWarps * 64);
     e[warp * 64 + lane] = x[0];
     e[warp * 64 + 32 + lane] = x[RW - 1];
@@ -417,6 +429,7 @@ __device__ __forceinline__ void tile_pass(const double* xin, double* xout, int n
     const double2 lo = e[(warp == 0 ? 0 : warp - 1) * 64 + 32 + lane];
     const double2 hi = e[(warp == kTileWarps - 1 ? warp : warp + 1) * 64 + lane];
     double2 south = lo;
+    double s = 0.;
 #pragma unroll
     for (int r = 0; r < RW; ++r) {
       const double2 m = x[r];
@@ -424,11 +437,12 @@ __device__ __forceinline__ void tile_pass(const double* xin, double* xout, int n
                                            __shfl_down_sync(0xffffffffu, m.x, 1));
       const double2 v = pair_full<FORM>(cf[r], part, r + 1 < RW ? x[r + 1 < RW ? r + 1 : r] : hi, bad);
       const bool in = (unsigned)(r0 + r) < rows;
-      if (in && L.own0) sum[t] = __dadd_rn(sum[t], fabs(__dsub_rn(v.x, m.x)));
-      if (in && L.own1) sum[t] = __dadd_rn(sum[t], fabs(__dsub_rn(v.y, m.y)));
+      if (in && L.own0) s = __dadd_rn(s, fabs(__dsub_rn(v.x, m.x)));
+      if (in && L.own1) s = __dadd_rn(s, fabs(__dsub_rn(v.y, m.y)));
       south = m;
       x[r] = v;
     }
+    put(t, s);
   }
   gj = g0;
 #pragma unroll
@@ -436,7 +450,9 @@ __device__ __forceinline__ void tile_pass(const double* xin, double* xout, int n
     if ((unsigned)(r0 + r) < rows) pair_store(xout + (size_t)gj * pitch, L, x[r]);
     gj = gj + 1 == ny ? 0 : gj + 1;
   }
-  if (FORM != kSysRecip && bad) sum[1] = kBadSum;
+  if constexpr (FORM != kSysRecip) {
+    if (__any_sync(0xffffffffu, bad) && lane == 0) sum[1] = kBadSum;
+  }
 }
 
 }  // namespace swm

@@ -1,6 +1,6 @@
 """The Jacobi kernel's forms (tiles, strips, one-sweep exact passes) against the oracle,
-bit for bit, where they can go wrong: the edges of tiles (56 x 40 cells) and strips (56
-columns), grids smaller than a warp's halo, odd widths, and operands that the fast
+bit for bit, where they can go wrong: the edges of tiles (56 x 40 and 48 x 32 cells) and
+strips (56 columns), grids smaller than a warp's halo, odd widths, and operands that the fast
 division does not take."""
 import numpy as np
 import pytest
@@ -27,9 +27,11 @@ def check(o, s, mass, diag, rhs):
     return k, rc
 
 
-# 1100 x 1003: 540 tiles, more than the tile form takes
-@pytest.mark.parametrize("nx,ny", [(3, 3), (5, 90), (56, 40), (57, 41), (64, 48), (113, 39),
-                                   (224, 81), (1100, 1003), (1101, 1000)])
+# 48 x 32 tiles up to 148 of them, 56 x 40 at 700 x 420 (135; 210 of 48 x 32), three rounds of
+# 48 x 32 at 1000 x 620, strips at 1100 x 1003
+@pytest.mark.parametrize("nx,ny", [(3, 3), (5, 90), (48, 32), (49, 33), (64, 48), (97, 65),
+                                   (224, 81), (700, 420), (701, 401), (1000, 620),
+                                   (1100, 1003), (1101, 1000)])
 @pytest.mark.parametrize("solver,block", [("stencil", 0), ("stencil", 3), ("csr", 0)])
 def test_shapes(gpu, nx, ny, solver, block):
     o, s = pair(gpu, nx, ny, solver, block)
