@@ -368,13 +368,20 @@ using Planes = std::array<double*, 3>;
 static Planes state_planes(swm_solver* s) { return {s->h, s->hu, s->hv}; }
 static Planes slot(swm_solver* s, int k) { return {s->ex[k][0], s->ex[k][1], s->ex[k][2]}; }
 
-// RHS of state X into R (all three components), mass fluxes to the slot-0 scratch.
+// RHS of the n states X into R (all three components), mass fluxes to the scratch of slots
+// 0 .. n - 1.
+static int explicit_rhs(swm_solver* s, const Planes* X, const Planes* R, int n) {
+  RhsArgs a[kRhsGroup];
+  for (int q = 0; q < n; ++q) {
+    a[q] = make_rhs_args(s, X[q][0], X[q][1], X[q][2], q);
+    a[q].ut_h = R[q][0];
+    a[q].ut_hu = R[q][1];
+    a[q].ut_hv = R[q][2];
+  }
+  return launch_rhs_states(s, a, n);
+}
 static int explicit_rhs(swm_solver* s, const Planes& X, const Planes& R) {
-  RhsArgs a = make_rhs_args(s, X[0], X[1], X[2], 0);
-  a.ut_h = R[0];
-  a.ut_hu = R[1];
-  a.ut_hv = R[2];
-  return launch_rhs_states(s, &a, 1);
+  return explicit_rhs(s, &X, &R, 1);
 }
 
 static int combo(swm_solver* s, int form, std::initializer_list<std::pair<double, Planes>> xs,
@@ -502,11 +509,10 @@ static int enqueue_explicit(swm_solver* s) {
           }
           CK(launch_combo(c, s->stream));
         }
-        if (kk != 5)
-          for (int ii = 2; ii <= 4; ++ii) {
-            F[ii] = slot(s, 2 + ii);  // FUp(2..4) in slots 4..6
-            XCK(explicit_rhs(s, Ua[ii], F[ii]));
-          }
+        if (kk != 5) {
+          for (int ii = 2; ii <= 4; ++ii) F[ii] = slot(s, 2 + ii);  // FUp(2..4) in slots 4..6
+          XCK(explicit_rhs(s, &Ua[2], &F[2], 3));
+        }
       }
     } break;
     default:

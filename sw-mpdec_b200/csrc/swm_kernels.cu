@@ -496,7 +496,8 @@ __device__ __forceinline__ double cell_update(const ExactGrid& g, const Sys& y, 
                                               int i, int j) {
   double p = 0.;
   if constexpr (FORM == kSysCsr) {
-    const int n = g.nx * g.ny, row = j * g.nx + i;
+    [[maybe_unused]] const int n = g.nx * g.ny;  // (the checked build's bound)
+    const int row = j * g.nx + i;
     for (int sp = g.rowstart[row]; sp <= g.rowstart[row + 1] - 1; ++sp)
       if (SWM_IN_RANGE(sp - 1, 5LL * n, kChkCsr) && SWM_IN_RANGE(g.cols[sp - 1] - 1, n, kChkCsr))
         p = __dadd_rn(p, __dmul_rn(y.mass[sp - 1], __ldcg(&xin[g.cols[sp - 1] - 1])));
@@ -822,9 +823,10 @@ cudaError_t launch_jacobi(const JacobiGroup& a, const JacobiGrid& g, cudaStream_
   };
   const long long t8 = pieces(jacobi_pick(a.form, 8)), t4 = pieces(jacobi_pick(a.form, 4));
   const long long round = g.tile_blocks;
-  const int tiles = t8 <= round ? 8
+  const bool long_pass = a.block > 4;  // else 8-sweep tiles would carry halo for nothing
+  const int tiles = long_pass && t8 <= round ? 8
                     : t4 <= round ? 4
-                    : t8 <= kTileWaves * round ? 8
+                    : long_pass && t8 <= kTileWaves * round ? 8
                     : t4 <= kTileWaves * round ? 4 : 0;
   const JacobiLaunch l = jacobi_pick(a.form, tiles);
   long long blocks = tiles == 8 ? t8 : t4, most = round;

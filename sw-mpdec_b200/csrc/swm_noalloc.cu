@@ -9,6 +9,7 @@
 // keeps its only scratch -- one iterate buffer and the solver's control block --
 // in the file-scope array below, which every GPU that loads this library holds
 // until the process exits.
+#include <cstddef>
 #include <cstdint>
 #include <mutex>
 
@@ -141,15 +142,16 @@ int swm_jacobi_noalloc(int nx, int ny, const double* cS, const double* cW, const
   y.hint_idx = -1;
   e = swm::launch_jacobi(ja, ds.grid, st);
   if (e != cudaSuccess) return noalloc_fail(SWM_ERR_CUDA, cudaGetErrorString(e));
-  int res[2] = {0, 0};  // iters[0], status
-  e = cudaMemcpyAsync(&res[0], &ctl->iters[0], sizeof(int), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&res[1], &ctl->status, sizeof(int), cudaMemcpyDeviceToHost, st);
+  // iters[0] .. status by one copy
+  int res[swm::kMaxSolves + 1] = {};
+  static_assert(offsetof(JacobiCtl, status) ==
+                    offsetof(JacobiCtl, iters) + swm::kMaxSolves * sizeof(int), "one copy");
+  e = cudaMemcpyAsync(res, &ctl->iters[0], sizeof(res), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return noalloc_fail(SWM_ERR_CUDA, cudaGetErrorString(e));
   if (iters) *iters = res[0];
-  if (res[1] < 0) return noalloc_fail(SWM_ERR_WATCHDOG, "Jacobi grid barrier watchdog expired");
-  return res[1] == 1 ? SWM_WARN_JACOBI_MAXITER : SWM_OK;
+  if (res[swm::kMaxSolves] < 0) return noalloc_fail(SWM_ERR_WATCHDOG, "Jacobi grid barrier watchdog expired");
+  return res[swm::kMaxSolves] == 1 ? SWM_WARN_JACOBI_MAXITER : SWM_OK;
 }
 
 }  // extern "C"
