@@ -187,7 +187,7 @@ __device__ __forceinline__ void load_hp(const AssembleArgs& a, int m1, int i, in
 // fl holds the face fluxes over the cell's extent (RhsArgs::over_len), oriented into the
 // cell: p > 0 is the production P_KL, -p the destruction D_KL of p < 0.  Either is weighted
 // by the depth it leaves (the neighbour's for th > 0 and production, th < 0 and
-// destruction), which selects the operands of one division.  The quotients are div_mk's,
+// destruction), which selects the operands of one division.  The quotients are div_mk2's,
 // which needs no branch, so that all of a row's divisions overlap; returns true when an
 // operand was outside its range (a zero numerator +0 is right too), and the caller then
 // takes the SAFE form (div_rn) for the cell.
@@ -195,13 +195,17 @@ template <int MS, bool SAFE>
 __device__ __forceinline__ bool patankar_exact(double dt, const double (&fl)[4][MS], double hK,
                                                const double (&hL)[4], const double* theta,
                                                double (&M)[4], double& D) {
-  const double denK = patankar_den(hK), rdenK = __drcp_rn(denK), hK2 = 2. * hK;
-  bool bad = !mk_range(denK);
+  // SAFE: the rounded reciprocals by __drcp_rn, no residual parts
+  auto rcp = [](double y) { return SAFE ? __drcp_rn(y) : rcp_mk(y); };
+  auto low = [](double y, double r) { return SAFE ? 0. : mk_low(y, r); };
+  const double denK = patankar_den(hK), rdenK = rcp(denK), ldenK = low(denK, rdenK), hK2 = 2. * hK;
+  bool bad = !mk_range(denK) || !mk_plain(denK);
   D = 1.;
 #pragma unroll
   for (int nb = 0; nb < 4; ++nb) {
-    const double h = hL[nb], denL = patankar_den(h), rdenL = __drcp_rn(denL), hL2 = 2. * h;
-    bad |= !mk_range(denL);
+    const double h = hL[nb], denL = patankar_den(h), rdenL = rcp(denL), ldenL = low(denL, rdenL),
+                 hL2 = 2. * h;
+    bad |= !mk_range(denL) || !mk_plain(denL);
     double m = 0.;
 #pragma unroll
     for (int r = 0; r < MS; ++r) {
@@ -213,7 +217,7 @@ __device__ __forceinline__ bool patankar_exact(double dt, const double (&fl)[4][
       if constexpr (SAFE) {
         pd = div_rn(num, den, rden);
       } else {
-        pd = div_mk(num, den, rden);
+        pd = div_mk2(num, den, rden, other ? ldenL : ldenK);
         bad |= !mk_range(num) && (__double2hiint(num) | __double2loint(num)) != 0;
       }
       if ((other ? h : hK) < kMinDepth) pd = 0.;
@@ -280,14 +284,13 @@ __device__ __forceinline__ void assemble_stage(const AssembleArgs& a, bool csr, 
       const double aL = ilen * wL, aK = ilen * wK;
 #pragma unroll
       for (int r = 0; r < MS; ++r) {
-        const double f = c.fl[nb][r], pf = dmax(f, 0.), qf = dmax(-f, 0.);
-        if (theta[r] > 0.) {
-          M[nb] = fma(-(cr[r] * pf), aL, M[nb]);
-          D = fma(cr[r] * qf, aK, D);
-        } else {
-          D = fma(-(cr[r] * pf), aK, D);
-          M[nb] = fma(cr[r] * qf, aL, M[nb]);
-        }
+        // t = dt theta_r f: positive (production for th > 0, destruction for th < 0) it
+        // takes the neighbour's weight off M, negative the cell's off D; the other part is
+        // an exact zero (split by t's sign bit: no FP64 operation, no branch on theta)
+        const double f = c.fl[nb][r], t = cr[r] * (f == f ? f : 0.);
+        const int hi = __double2hiint(t), lo = __double2loint(t), neg = hi >> 31;
+        M[nb] = fma(-__hiloint2double(hi & ~neg, lo & ~neg), aL, M[nb]);
+        D = fma(-__hiloint2double(hi & neg, lo & neg), aK, D);
       }
     }
   } else {

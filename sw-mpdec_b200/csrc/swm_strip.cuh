@@ -147,11 +147,18 @@ __device__ __forceinline__ bool strip_range(double x) {
 __device__ __forceinline__ bool strip_num(double x) {
   return strip_range(x) || (__double2hiint(x) | __double2loint(x)) == 0;
 }
-template <int FORM>
+// RN(1/D) of a row: strips form one per step, without a branch; tiles once per load, by
+// __drcp_rn, whose branches keep the registers of a thread's rows from all being live.
+template <int FORM, bool TILE>
 __device__ __forceinline__ void strip_rcp(StripRow<FORM>& r, bool& bad) {
   if constexpr (FORM != kSysRecip) {
-    r.R = make_double2(__drcp_rn(r.D.x), __drcp_rn(r.D.y));
     bad |= !strip_range(r.D.x) || !strip_range(r.D.y);
+    if constexpr (TILE) {
+      r.R = make_double2(__drcp_rn(r.D.x), __drcp_rn(r.D.y));
+    } else {
+      r.R = make_double2(rcp_mk(r.D.x), rcp_mk(r.D.y));
+      bad |= !mk_plain(r.D.x) || !mk_plain(r.D.y);
+    }
   }
 }
 
@@ -210,7 +217,7 @@ __device__ __forceinline__ StripRow<FORM> strip_row(const double2* w, bool& bad)
     r.D = w[128];
     if constexpr (FORM == kSysDiv) r.B = w[160];
   }
-  strip_rcp<FORM>(r, bad);
+  strip_rcp<FORM, false>(r, bad);
   return r;
 }
 
@@ -374,7 +381,7 @@ __device__ __forceinline__ void tile_rows(const JacobiSys& y, int nx, int ny, in
     gj = gj + 1 == ny ? 0 : gj + 1;
   }
 #pragma unroll
-  for (int r = 0; r < RW; ++r) strip_rcp<FORM>(cf[r], bad);
+  for (int r = 0; r < RW; ++r) strip_rcp<FORM, true>(cf[r], bad);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
