@@ -345,12 +345,12 @@ constexpr double kBand = 0x1p-20;
 
 // Grid barrier number `nth` (1, 2, ..) of a launch on its own arrival counter (zero when
 // the launch starts), by one thread: everything its block wrote before a block barrier is
-// visible to every block after it.  The count only grows, so an arrival is one atomic and
-// a wait one polled word.  False when the wait gave up (status -4).
+// visible to every block after it (the arrival releases, the poll acquires; both are
+// ordered with the block's other threads by the block barriers around this).  The count
+// only grows, so an arrival is one atomic and a wait one polled word.  False when the wait gave up (status -4).
 __device__ __forceinline__ bool arrive_and_wait(unsigned int* ctr, unsigned int nth,
                                                 long long spin_limit, int* status) {
   const unsigned int target = nth * gridDim.x;
-  __threadfence();
   unsigned int c;
   asm volatile("atom.add.acq_rel.gpu.u32 %0, [%1], 1;" : "=r"(c) : "l"(ctr) : "memory");
   bool ok = true;
@@ -366,7 +366,6 @@ __device__ __forceinline__ bool arrive_and_wait(unsigned int* ctr, unsigned int 
       }
     }
   }
-  __threadfence();
   return ok;
 }
 
