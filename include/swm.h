@@ -81,7 +81,7 @@ typedef struct swm_params {
   int solver;            /* SWM_SOLVER_* */
   int jacobi_maxiter;    /* maxIter = 1000 (jacobi_iteration.f90:64) */
   double jacobi_tol;     /* tolerance = 1e-16 (jacobi_iteration.f90:63) */
-  int jacobi_block;      /* stencil solver: Jacobi sweeps per pass (1..8), 0 = auto */
+  int jacobi_block;      /* stencil solver: Jacobi sweeps per pass at most (1..8), 0 = auto */
   int mpdec2_compat;     /* 1: reproduce the hp(2,nx,ny) read of Up(:,1,:,:) of mPDeC2 and mPEuler */
   int use_graph;         /* capture each step into a CUDA graph (1 = default) */
   int device;            /* CUDA device ordinal */
@@ -234,7 +234,7 @@ SWM_API int swm_debug_inject_alloc_failure(long long nth, long long *counted);
  * and loops that must not pay the device-wide synchronisation of cudaMalloc and
  * cudaFree.  Solves one Patankar system (x <- (rhs - S x_S - W x_W - E x_E - N x_N)/D
  * on the periodic nx*ny grid, stop rule of jacobi_iteration.f90:52-87) with the
- * matrix-free stencil kernel, `block` sweeps per pass (1..8).  All arrays are the
+ * matrix-free stencil kernel, at most `block` sweeps per pass (1..8).  All arrays are the
  * caller's device memory, nx*ny doubles each, [ny][nx] row-major; sol is written
  * while the others are read, so it must not overlap rhs or any coefficient plane
  * (SWM_ERR_PARAM otherwise).  Scratch is a static device array sized for at most
@@ -264,14 +264,14 @@ SWM_API int swm_debug_checked_status(int *site, unsigned long long *count);
 typedef struct swm_batch *swm_batch_handle;
 /* n problems of independent size and parameters, stepped together (the
  * reference's time loop, timediscretization.f90:57-95, over an ensemble): a whole
- * mPDeC5 step of every problem is one cooperative persistent launch (TimeStep, the
- * RHS of every tile, and per correction the assembly of its three substeps and one
- * batched Jacobi solve of all their systems, each with its own stop rule), captured
- * with its memsets as a CUDA graph.  All problems share precision and jacobi_block
- * (taken from p[0]); mPDeC5 only, no well-balanced reference; the stencil solver is
- * always used.  jacobi_block = 0 lets the first step time the schedules (2, 4 and 8
- * sweeps per pass, one or two CTAs per SM) on the initial state and keep the
- * fastest; every schedule gives the same results. */
+ * mPDeC5 step of every problem is one cooperative persistent launch, or a kernel per
+ * phase (TimeStep, the RHS of every tile, and per correction the assembly of its three
+ * substeps and one batched Jacobi solve of all their systems, each with its own stop
+ * rule), captured with its memsets as a CUDA graph.  All problems share precision and
+ * jacobi_block (taken from p[0]); mPDeC5 only, no well-balanced reference; the stencil
+ * solver is always used.  jacobi_block = 0 lets the first step time the schedules (the
+ * two forms, sweeps per pass, CTAs per SM) on the initial state and keep the fastest;
+ * every schedule gives the same results. */
 SWM_API int swm_batch_create(int n, const swm_params *p, swm_batch_handle *out);
 SWM_API int swm_batch_destroy(swm_batch_handle b);
 SWM_API int swm_batch_set_planes(swm_batch_handle b, int i, const double *planes);

@@ -399,13 +399,14 @@ __device__ __forceinline__ void assemble_multi_cell(const AssembleMultiArgs& am,
 }
 
 // ---------------------------------------------------------------------------
-// Jacobi (jacobi_iteration.f90:52-87): x^{k+1} = (b - L x^k)/D from x^0 = b,
-// residual mean|x^{k+1}-x^k|, stop when <= tol or at maxIter.
-// One cooperative persistent launch per solve; passes separated by a bounded
-// grid barrier; the stop decision is taken identically by every CTA from the
-// integer residual sums.
+// Jacobi (jacobi_iteration.f90:52-87) in the persistent ensemble step: x^{k+1} =
+// (b - L x^k)/D from x^0 = b, residual mean|x^{k+1}-x^k|, stop when <= tol or at
+// maxIter, in passes over shared-memory tiles separated by bounded grid barriers, the
+// stop decision taken from integer residual sums.  (The single-grid solver and the
+// per-phase ensemble sweep by registers, swm_strip.cuh; the step kernel shares its 128
+// registers with the RHS tile.)
 // ---------------------------------------------------------------------------
-// C: JacobiCtl or JacBatchCtl (bar_count, bar_gen, status).
+// C: JacBatchCtl (bar_count, bar_gen, status).
 template <typename C>
 __device__ bool grid_barrier(C* ctl, long long spin_limit, int* s_ok) {
   __syncthreads();
@@ -719,14 +720,13 @@ __device__ __forceinline__ void tile_load(const JacobiArgs& a, const double* xin
   }
 }
 
-// One stencil pass of Tp <= TB sweeps over every tile of this CTA.  A tile is a
-// JBX x JBY block of cells plus a TB-cell halo in shared memory; sweep t updates
-// the region shrunk by t, so after Tp sweeps the tile interior holds x^{k+Tp},
-// bit-identical to Tp global sweeps.  Warps own rows, lanes own columns.
-template <int TB, bool RECIP, bool ONE_TILE>
-__device__ void stencil_tiles(const JacobiArgs& a, const double* xin, double* xout, int Tp,
-                              bool first, Acc& acc, double* sm, int tile_first,
-                              unsigned long long (*s_acc)[3]) {
+// One pass of Tp <= TB sweeps over one tile: a JBX x JBY block of cells plus a TB-cell
+// halo in shared memory; sweep t updates the region shrunk by t, so after Tp sweeps the
+// tile interior holds x^{k+Tp}, bit-identical to Tp global sweeps.  Warps own rows, lanes
+// own columns.
+template <int TB, bool RECIP>
+__device__ void stencil_tile(const JacobiArgs& a, const double* xin, double* xout, int Tp,
+                             bool first, Acc& acc, double* sm, int tile) {
   using G = JTile<TB>;
   constexpr int HX = G::HX, HY = G::HY, HN = G::HN, NW = JNT / 32;
   double* sB = sm + 5 * HN;
@@ -736,58 +736,45 @@ __device__ void stencil_tiles(const JacobiArgs& a, const double* xin, double* xo
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool small = (nx < HX) || (ny < HY);
   // 16-byte pairs need an even first column (i0 - TB), an even row pitch and 16-byte
-  // aligned arrays (the allocation-free entry takes the caller's pointers as given)
+  // aligned arrays
   const bool pairs = (TB % 2 == 0) && !small && (pitch % 2 == 0) && arrays_aligned16(a, xin);
   // first pass: x^0 = b, already in the b tile (sweep 1 reads it there)
   const bool from_b = xin == a.b;
-  const int tx = (nx + JBX - 1) / JBX, ty = (ny + JBY - 1) / JBY;
-  // ONE_TILE: exactly tile `tile_first` (ensembles); else every CTA-strided tile
-  const int t_end = ONE_TILE ? tile_first + 1 : tx * ty;
-  const int t_step = ONE_TILE ? 1 : gridDim.x;
-  // values a thread adds per sweep and tile: two per pair unit of sweep 1
-  constexpr int kPerTile = 2 * ((((HX - 2) / 2 + 1) * (HY - 2) + JNT - 1) / JNT);
-  int since_flush = 0;
-  for (int tile = tile_first; tile < t_end; tile += t_step) {
-    const int i0 = (tile % tx) * JBX, j0 = (tile / tx) * JBY;
-    const int cx_lim = min(JBX, nx - i0), cy_lim = min(JBY, ny - j0);
-    if (!ONE_TILE && (since_flush += kPerTile) > kAccFlushCells) {
-      acc_reduce<TB>(acc, s_acc);  // keep the per-thread part sums exact
-      since_flush = kPerTile;
-    }
-    // ensembles: a tile cut by the grid's edge loads and sweeps only the box it needs
-    // (their grids are small, edge tiles common); the single-grid kernel keeps one
-    // code path, which measured 2% faster with the partial variant compiled out
-    const bool part = ONE_TILE && (cx_lim < JBX || cy_lim < JBY);
-    if (part)
-      tile_load<TB, RECIP, true>(a, xin, sm, i0, j0, cx_lim, cy_lim, pitch, pairs, small, from_b);
-    else
-      tile_load<TB, RECIP, false>(a, xin, sm, i0, j0, cx_lim, cy_lim, pitch, pairs, small, from_b);
-    __syncthreads();
-    if (first) {  // initial residual mean|0 - b| (jacobi_iteration.f90:69)
-      for (int ly = TB + warp; ly < TB + JBY; ly += NW)
-        for (int lx = TB + lane; lx < TB + JBX; lx += 32)
-          if (i0 + lx - TB < nx && j0 + ly - TB < ny) acc_put<0>(acc, fabs(0. - sB[ly * HX + lx]));
-    }
-    double* xp = from_b ? sB : x0;
-    double* xn = x1;
-    if (part)
-      tile_sweeps<TB, 1, RECIP, true>(sm, xp, xn, Tp, cx_lim, cy_lim, acc);
-    else
-      tile_sweeps<TB, 1, RECIP, false>(sm, xp, xn, Tp, cx_lim, cy_lim, acc);
-    for (int ly = TB + warp; ly < TB + JBY; ly += NW) {
-      const int gj = j0 + ly - TB;
-      if (gj >= ny) continue;
-      for (int lx = TB + lane; lx < TB + JBX; lx += 32) {
-        const int gi = i0 + lx - TB;
-        if (gi < nx) xout[(size_t)gj * pitch + gi] = xp[ly * HX + lx];
-      }
-    }
-    __syncthreads();
+  const int tx = (nx + JBX - 1) / JBX;
+  const int i0 = (tile % tx) * JBX, j0 = (tile / tx) * JBY;
+  const int cx_lim = min(JBX, nx - i0), cy_lim = min(JBY, ny - j0);
+  // a tile cut by the grid's edge loads and sweeps only the box it needs (an ensemble's
+  // grids are small, edge tiles common)
+  const bool part = cx_lim < JBX || cy_lim < JBY;
+  if (part)
+    tile_load<TB, RECIP, true>(a, xin, sm, i0, j0, cx_lim, cy_lim, pitch, pairs, small, from_b);
+  else
+    tile_load<TB, RECIP, false>(a, xin, sm, i0, j0, cx_lim, cy_lim, pitch, pairs, small, from_b);
+  __syncthreads();
+  if (first) {  // initial residual mean|0 - b| (jacobi_iteration.f90:69)
+    for (int ly = TB + warp; ly < TB + JBY; ly += NW)
+      for (int lx = TB + lane; lx < TB + JBX; lx += 32)
+        if (i0 + lx - TB < nx && j0 + ly - TB < ny) acc_put<0>(acc, fabs(0. - sB[ly * HX + lx]));
   }
+  double* xp = from_b ? sB : x0;
+  double* xn = x1;
+  if (part)
+    tile_sweeps<TB, 1, RECIP, true>(sm, xp, xn, Tp, cx_lim, cy_lim, acc);
+  else
+    tile_sweeps<TB, 1, RECIP, false>(sm, xp, xn, Tp, cx_lim, cy_lim, acc);
+  for (int ly = TB + warp; ly < TB + JBY; ly += NW) {
+    const int gj = j0 + ly - TB;
+    if (gj >= ny) continue;
+    for (int lx = TB + lane; lx < TB + JBX; lx += 32) {
+      const int gi = i0 + lx - TB;
+      if (gi < nx) xout[(size_t)gj * pitch + gi] = xp[ly * HX + lx];
+    }
+  }
+  __syncthreads();
 }
 
 // ---------------------------------------------------------------------------
-// Ensembles: one cooperative launch solves the Patankar systems of every problem.
+// The persistent ensemble step's batched solve: the Patankar systems of every problem.
 // Each pass visits the tiles of all still-active problems; residual limbs are
 // flushed per tile into that problem's accumulators; after a grid barrier CTA 0
 // applies the single-problem stop rule to every problem (stop, redo the pass with
@@ -919,7 +906,7 @@ __device__ __forceinline__ bool jacobi_batch_solve(const JacobiBatchArgs& a, dou
   Acc acc;
   acc_zero(acc);
   int loaded = -1;
-  // values a thread adds per sweep slot and tile (as stencil_tiles counts them); the
+  // values a thread adds per sweep slot and tile (two per pair unit of sweep 1); the
   // part sums are flushed before they could exceed kAccFlushCells values
   constexpr int kPerTile =
       2 * ((((JTile<TB>::HX - 2) / 2 + 1) * (JTile<TB>::HY - 2) + JNT - 1) / JNT);
@@ -958,7 +945,7 @@ __device__ __forceinline__ bool jacobi_batch_solve(const JacobiBatchArgs& a, dou
   auto tile = [&](int t) {
     const double* xin = s_cur == 0 ? sd.b : (s_cur == 1 ? sd.xa : (s_cur == 2 ? sd.xb : sd.out));
     double* xout = s_xnext == 1 ? sd.xa : (s_xnext == 2 ? sd.xb : sd.out);
-    stencil_tiles<TB, RECIP, true>(sd, xin, xout, s_Tp, s_first != 0, acc, jsm, t, s_acc);
+    stencil_tile<TB, RECIP>(sd, xin, xout, s_Tp, s_first != 0, acc, jsm, t);
   };
   for (;;) {
     if (a.work) {
