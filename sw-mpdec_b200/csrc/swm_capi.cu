@@ -79,6 +79,13 @@ namespace swm {
 void set_last_error(const char* msg) { g_last_error = msg; }
 }  // namespace swm
 
+// What a step clears before it starts and returns when it ends, in one piece of memory: one
+// memset and one copy.
+struct StepCtl {
+  JacobiCtl ctl;
+  unsigned long long lam[3];  // LambdaMax bit patterns, then the flag (an int)
+};
+
 struct swm_solver {
   swm_params p{};
   int nx = 0, ny = 0;
@@ -133,8 +140,10 @@ struct swm_solver {
   double* stage2 = nullptr;  // the same, shared with set 0
   // pinned host mirrors
   double* h_dt = nullptr;
+  StepCtl* step_ctl = nullptr;          // device: ctl, lam and bad are inside
+  StepCtl* h_step = nullptr;            // its pinned mirror; the next three are inside
   JacobiCtl* h_ctl = nullptr;
-  unsigned long long* h_lam = nullptr;  // pinned mirror of lam and bad (3 words)
+  unsigned long long* h_lam = nullptr;
   int* h_bad = nullptr;
   // graph
   cudaGraphExec_t graph = nullptr;
@@ -524,7 +533,6 @@ static int enqueue_explicit(swm_solver* s) {
 // LambdaMax and the non-finite/negative-depth flag of the state (TimeStep's
 // reduction, equation.f90:791-837), into s->lam / s->bad.
 static int enqueue_dt(swm_solver* s) {
-  CK(cudaMemsetAsync(s->lam, 0, 3 * sizeof(unsigned long long), s->stream));
   DtArgs a{s->nx, s->ny, s->p.g, s->h, s->hu, s->hv, s->lam, s->bad};
   CK(launch_dt(a, s->stream));
   return SWM_OK;
@@ -534,11 +542,14 @@ static int enqueue_patankar(swm_solver* s);
 
 // One step: the scheme's launches, then the reduction of the new state, so that a
 // non-finite value born inside the step is reported by the step itself and the next
-// TimeStep() needs no launch of its own.  The Jacobi control block is cleared first:
+// TimeStep() needs no launch of its own.  dt is copied in from its pinned word and the
+// control block copied out to its pinned mirror as part of the sequence (and so of the
+// graph).  The Jacobi control block is cleared first:
 // every step starts from a clean barrier and residual state, also after a solve
 // that gave up on its grid barrier.
 static int enqueue_step(swm_solver* s) {
-  CK(cudaMemsetAsync(s->ctl, 0, sizeof(JacobiCtl), s->stream));
+  CK(cudaMemcpyAsync(s->dt_dev, s->h_dt, sizeof(double), cudaMemcpyHostToDevice, s->stream));
+  CK(cudaMemsetAsync(s->step_ctl, 0, sizeof(StepCtl), s->stream));
   int rc;
   if (s->p.timescheme <= 4) {
     s->n_solves = 0;
@@ -547,7 +558,9 @@ static int enqueue_step(swm_solver* s) {
     rc = enqueue_patankar(s);
   }
   if (rc) return rc;
-  return enqueue_dt(s);
+  if ((rc = enqueue_dt(s))) return rc;
+  CK(cudaMemcpyAsync(s->h_step, s->step_ctl, sizeof(StepCtl), cudaMemcpyDeviceToHost, s->stream));
+  return SWM_OK;
 }
 
 static int enqueue_patankar(swm_solver* s) {
@@ -839,15 +852,17 @@ int swm_create(const swm_params* p, swm_handle* out) {
     AL(s->swb, 3 * N);
   }
   AL(s->dt_dev, 1);
-  AL(s->lam, 3);
+  AL(s->step_ctl, 1);
+  s->ctl = &s->step_ctl->ctl;
+  s->lam = s->step_ctl->lam;
   s->bad = reinterpret_cast<int*>(s->lam + 2);
-  AL(s->ctl, 1);
   AL(s->summary, 2 + 512);
 #undef AL
   if (lib_malloc_host((void**)&s->h_dt, sizeof(double)) != cudaSuccess ||
-      lib_malloc_host((void**)&s->h_ctl, sizeof(JacobiCtl)) != cudaSuccess ||
-      lib_malloc_host((void**)&s->h_lam, 3 * sizeof(unsigned long long)) != cudaSuccess)
+      lib_malloc_host((void**)&s->h_step, sizeof(StepCtl)) != cudaSuccess)
     return cleanup(fail(SWM_ERR_ALLOC, "cudaMallocHost failed"));
+  s->h_ctl = &s->h_step->ctl;
+  s->h_lam = s->h_step->lam;
   s->h_bad = reinterpret_cast<int*>(s->h_lam + 2);
 
   if (csr) {  // finitevolume.f90:219-267 CSR pattern, 1-based, slot order S, W, C, E, N
@@ -928,8 +943,7 @@ int swm_destroy(swm_handle s) {
   drop_graph(s);
   for (void* ptr : s->allocs) cudaFree(ptr);
   if (s->h_dt) cudaFreeHost(s->h_dt);
-  if (s->h_ctl) cudaFreeHost(s->h_ctl);
-  if (s->h_lam) cudaFreeHost(s->h_lam);
+  if (s->h_step) cudaFreeHost(s->h_step);
   if (s->out_dev) cudaFree(s->out_dev);
   if (s->out_host) cudaFreeHost(s->out_host);
   if (s->stream) cudaStreamDestroy(s->stream);
@@ -1274,6 +1288,7 @@ int swm_timestep(swm_handle s, double* dt_min) {
   if (!s->have_state) return fail(SWM_ERR_STATE, "no state set");
   CK(cudaSetDevice(s->device));
   if (!s->lam_fresh) {  // the state changed since the last step's reduction
+    CK(cudaMemsetAsync(s->lam, 0, 3 * sizeof(unsigned long long), s->stream));
     int rc = enqueue_dt(s);
     if (rc) return rc;
     CK(cudaMemcpyAsync(s->h_lam, s->lam, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
@@ -1308,7 +1323,6 @@ int swm_step(swm_handle s, double t, double dt) {
     return fail(SWM_ERR_STATE, "well_balanced handle without swm_set_wb_state");
   CK(cudaSetDevice(s->device));
   *s->h_dt = dt;
-  CK(cudaMemcpyAsync(s->dt_dev, s->h_dt, sizeof(double), cudaMemcpyHostToDevice, s->stream));
   int rc = build_graph(s);
   if (rc) return rc;
   if (s->graph) {
@@ -1317,9 +1331,6 @@ int swm_step(swm_handle s, double t, double dt) {
     rc = enqueue_step(s);
     if (rc) return rc;
   }
-  CK(cudaMemcpyAsync(s->h_ctl, s->ctl, sizeof(JacobiCtl), cudaMemcpyDeviceToHost, s->stream));
-  CK(cudaMemcpyAsync(s->h_lam, s->lam, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                     s->stream));
   CK(cudaStreamSynchronize(s->stream));
   s->lam_fresh = true;
   if (s->n_solves == 0) {  // graph built without a host pass: count solves
@@ -1361,7 +1372,6 @@ int swm_profile_step(swm_handle s, double t, double dt, float* ms, int* launches
   if (!s->have_state) return fail(SWM_ERR_STATE, "no state set");
   CK(cudaSetDevice(s->device));
   *s->h_dt = dt;
-  CK(cudaMemcpyAsync(s->dt_dev, s->h_dt, sizeof(double), cudaMemcpyHostToDevice, s->stream));
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -1395,7 +1405,6 @@ int swm_profile_step(swm_handle s, double t, double dt, float* ms, int* launches
     if (launches) launches[c] = cnt[c];
   }
   ms[3] = tot;
-  CK(cudaMemcpy(s->h_ctl, s->ctl, sizeof(JacobiCtl), cudaMemcpyDeviceToHost));
   s->lam_fresh = false;
   for (int k = 0; k < s->n_solves && k < kMaxSolves; ++k) s->stats.jacobi_iters[k] = s->h_ctl->iters[k];
   s->stats.n_solves = s->n_solves;
