@@ -862,21 +862,16 @@ __global__ void __launch_bounds__(RHS_NT, MODE == 1 ? 3 : 2)
   rhs_tile<MODE>(a, &tm, blockIdx.x * RHS_TX, blockIdx.y * RHS_TY);
 }
 
-// Up to kRhsGroup states of one grid, block z of the grid state z, in tiles of TX x TX.  The
-// small tiles, which have an SM to themselves, take as many threads as a phase has items
-// (360 first sweeps of an 8 x 8 tile).
-template <int TX>
-constexpr int kGroupNT = TX == RHS_SMALL ? 384 : RHS_NT;
+// Up to kRhsGroup states of one grid, block z of the grid state z, in tiles of TX x TX.
 template <int MODE, int TX>
-__global__ void __launch_bounds__(kGroupNT<TX>, TX == RHS_SMALL ? 1 : (MODE == 1 ? 3 : 2))
-    rhs_group_kernel(const __grid_constant__ RhsGroup g) {
+__global__ void __launch_bounds__(RHS_NT, MODE == 1 ? 3 : 2) rhs_group_kernel(const __grid_constant__ RhsGroup g) {
   static_assert(sizeof(RhsArgs) % 8 == 0 && sizeof(RhsArgs) / 8 <= RHS_NT, "descriptor copy");
   __shared__ __align__(16) RhsArgs sa;
   if (threadIdx.x < sizeof(RhsArgs) / 8)
     reinterpret_cast<unsigned long long*>(&sa)[threadIdx.x] =
         reinterpret_cast<const unsigned long long*>(&g.a[blockIdx.z])[threadIdx.x];
   __syncthreads();
-  rhs_tile<MODE, kGroupNT<TX>, TX, TX>(sa, nullptr, blockIdx.x * TX, blockIdx.y * TX);
+  rhs_tile<MODE, RHS_NT, TX, TX>(sa, nullptr, blockIdx.x * TX, blockIdx.y * TX);
 }
 
 template <int MODE, int TX>
@@ -888,7 +883,7 @@ static cudaError_t launch_group(const RhsGroup& g, int n, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   const Grid& gr = g.a[0].gr;
   dim3 grd((gr.nx + TX - 1) / TX, (gr.ny + TX - 1) / TX, n);
-  rhs_group_kernel<MODE, TX><<<grd, kGroupNT<TX>, bytes, s>>>(g);
+  rhs_group_kernel<MODE, TX><<<grd, RHS_NT, bytes, s>>>(g);
   return cudaGetLastError();
 }
 
