@@ -221,7 +221,7 @@ static int jacobi_form(const swm_params& p) {
 
 // The three substeps of an mPDeC5 correction depend only on the previous correction, so
 // their systems are solved by one launch: one set of passes, barriers and tails instead
-// of three.  That takes up to 17 more planes; beyond
+// of three.  That takes up to 16 more planes; beyond
 // kGroupCells one system alone keeps every SM busy for many passes' worth of rows, and
 // the memory is left to larger grids.
 constexpr size_t kGroupCells = size_t(1) << 23;
