@@ -347,7 +347,8 @@ constexpr double kBand = 0x1p-20;
 // the launch starts), by one thread: everything its block wrote before a block barrier is
 // visible to every block after it (the arrival releases, the poll acquires; both are
 // ordered with the block's other threads by the block barriers around this).  The count
-// only grows, so an arrival is one atomic and a wait one polled word.  False when the wait gave up (status -4).
+// only grows, modulo 2^32 (barrier_open), so an arrival is one atomic and a wait one
+// polled word.  False when the wait gave up (status -4).
 __device__ __forceinline__ bool arrive_and_wait(unsigned int* ctr, unsigned int nth,
                                                 long long spin_limit, int* status) {
   const unsigned int target = nth * gridDim.x;
@@ -358,7 +359,7 @@ __device__ __forceinline__ bool arrive_and_wait(unsigned int* ctr, unsigned int 
     long long spins = 0;
     for (;;) {
       asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(c) : "l"(ctr) : "memory");
-      if (c >= target) break;
+      if (barrier_open(c, target)) break;
       if (++spins > spin_limit || spin_limit <= 0) {
         ok = false;
         atomicExch(status, -4);

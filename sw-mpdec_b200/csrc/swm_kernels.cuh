@@ -6,6 +6,7 @@
 
 #include "swm_device.cuh"
 #include "swm_rhs.cuh"
+#include "swm_rules.h"
 
 namespace swm {
 

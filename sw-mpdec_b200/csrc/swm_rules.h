@@ -1,0 +1,21 @@
+// swm_rules.h -- rules of the solvers' control flow as plain functions, for device and
+// host code alike (a host compiler builds them as they are for the tests).
+#pragma once
+
+#ifdef __CUDACC__
+#define SWM_HD __host__ __device__ __forceinline__
+#else
+#define SWM_HD inline
+#endif
+
+namespace swm {
+
+// A grid barrier's arrival count has reached the target of its n-th use, n times the
+// blocks.  Both grow by one per arrival modulo 2^32 and are never further apart than the
+// blocks of a grid (no block arrives at a use before all have arrived at the one before
+// it), so the sign of their difference tells, also where they pass 2^32.
+SWM_HD bool barrier_open(unsigned int count, unsigned int target) {
+  return (int)(count - target) >= 0;
+}
+
+}  // namespace swm
