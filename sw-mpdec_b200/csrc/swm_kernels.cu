@@ -580,7 +580,7 @@ __device__ __noinline__ bool solve_exact(const ExactGrid& g, const Sys& y, SysSt
     }
     acc_reduce<1>(acc, s_acc);
     __syncthreads();
-    const int slot = *pass % kResSlots;
+    const int slot = *pass;
     if (threadIdx.x < 6) {
       const unsigned long long v = (&s_acc[0][0])[threadIdx.x];
       if (v) atomicAdd(&(&g.acc[slot][0][0])[threadIdx.x], v);
@@ -591,11 +591,11 @@ __device__ __noinline__ bool solve_exact(const ExactGrid& g, const Sys& y, SysSt
     if (!s_ok) return false;
     if (threadIdx.x < 6) (&s_tot[0][0])[threadIdx.x] = __ldcg(&(&g.acc[slot][0][0])[threadIdx.x]);
     if (blockIdx.x == 0 && threadIdx.x < 6) {
-      (&g.acc[(*pass + 2) % kResSlots][0][0])[threadIdx.x] = 0ull;
+      (&g.acc[ring_at(slot, 2, kResSlots)][0][0])[threadIdx.x] = 0ull;
       __threadfence();
     }
     __syncthreads();
-    if (threadIdx.x == 0) ++*pass;
+    if (threadIdx.x == 0) *pass = ring_at(slot, 1, kResSlots);
     if (first && limbs_le(s_tot[0][0], s_tot[0][1], s_tot[0][2], g.thresh)) {
       stop = 0;
       break;
@@ -659,9 +659,9 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
       s_ch = ch;
     }
   };
-  int pass = 0;  // warp 0: position in the ring of sums
+  int slot = 0;  // warp 0: position in the ring of sums
   if (warp == 0) {
-    pass = *((volatile int*)&ctl->pass_next);
+    slot = *((volatile int*)&ctl->pass_next);
     if (lane < a.nsys) {
       const JacobiSys& y = a.sys[lane];
       const int hint = y.hint_idx >= 0 ? __ldcg(&ctl->iters[y.hint_idx]) : 0;
@@ -735,7 +735,6 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
     __syncthreads();
     if (warp == 0) {
       // the block's sums, the grid barrier, then every block's decisions from the totals
-      const int slot = pass % kResSlots;
       static_assert(kMaxSys * (T + 1) <= 32, "a lane per sum");
       const int q = lane / (T + 1), t = lane % (T + 1);
       const bool mine = q < a.nsys && st[q < kMaxSys ? q : 0].active;
@@ -752,7 +751,7 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
         if (mine) s_tot[q][t] = __ldcg(&ctl->sum[slot][q][t]);
         if (blockIdx.x == 0) {  // recycle the slot of the pass before this one
           for (int z = lane; z < kMaxSys * (kMaxBlock + 1); z += 32)
-            (&ctl->sum[(pass + 2) % kResSlots][0][0])[z] = 0.;
+            (&ctl->sum[ring_at(slot, 2, kResSlots)][0][0])[z] = 0.;
           __threadfence();
         }
         __syncwarp();
@@ -763,7 +762,7 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
         }
         __syncwarp();
         plan();
-        ++pass;
+        slot = ring_at(slot, 1, kResSlots);
       }
     }
     __syncthreads();
@@ -786,7 +785,7 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
     ctl->iters[a.sys[threadIdx.x].solve_idx] = S.zero ? 0 : S.k;
     if (S.maxhit) atomicCAS(&ctl->status, 0, 1);
     if (threadIdx.x == 0) {
-      *((volatile int*)&ctl->pass_next) = pass;
+      *((volatile int*)&ctl->pass_next) = slot;
       *((volatile int*)&ctl->exact_next) = s_xpass;
     }
   }
@@ -907,7 +906,8 @@ __global__ void __launch_bounds__(kStripNT, FORM == kSysRecip ? 3 : 2)
     return sys_start(d.maxiter, d.b, d.xa, direct(d), a.hint ? __ldg(&a.hint[sys]) : 0, blk);
   };
   __syncthreads();
-  for (int pass = 0;; ++pass) {
+  bool begun = false;  // the systems' states are in memory
+  for (int slot = 0;; slot = ring_at(slot, 1, 3), begun = true) {
     for (int w = me; w < nwork;) {
       unsigned int nw = 0;
       if (lane == 0) nw = (unsigned int)warps + atomicAdd(&ctl->work, 1u);
@@ -918,7 +918,7 @@ __global__ void __launch_bounds__(kStripNT, FORM == kSysRecip ? 3 : 2)
       int Tp, first, active = 1;
       const double* xin;
       double* xout;
-      if (pass == 0) {  // the states are written by the first decisions
+      if (!begun) {  // the states are written by the first decisions
         const SysState S = start(d, sys);
         Tp = S.Tp;
         first = 1;
@@ -958,7 +958,7 @@ __global__ void __launch_bounds__(kStripNT, FORM == kSysRecip ? 3 : 2)
     for (int p = blockIdx.x + gridDim.x * threadIdx.x; p < nsys; p += gridDim.x * blockDim.x) {
       const JacobiArgs& d = a.descs[p];
       StripBatchState& B = a.st[p];
-      SysState S = pass == 0 ? start(d, p) : B.s;
+      SysState S = begun ? B.s : start(d, p);
       if (!S.active) continue;
       double sum[T + 1];
 #pragma unroll
@@ -970,17 +970,17 @@ __global__ void __launch_bounds__(kStripNT, FORM == kSysRecip ? 3 : 2)
       sys_decide<RECIP>(S, (double)d.nx * d.ny, d.maxiter, thresh, d.b, d.xa, d.xb, direct(d), sum,
                         a.hint ? __ldg(&a.hint[p]) : 0, blk);
       B.s = S;
-      if (S.active) atomicAdd(&ctl->nact[pass % 3], 1);
+      if (S.active) atomicAdd(&ctl->nact[slot], 1);
       if (S.exact) atomicAdd(&ctl->nexact, 1);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       ctl->work = 0u;
-      ctl->nact[(pass + 1) % 3] = 0;  // read by everyone before the barrier above
+      ctl->nact[ring_at(slot, 1, 3)] = 0;  // read by everyone before the barrier above
     }
     __syncthreads();
     if (threadIdx.x == 0) {
       s_ok = arrive_and_wait(bar, ++s_nbar, a.spin_limit, &ctl->status);
-      s_nact = __ldcg(&ctl->nact[pass % 3]);
+      s_nact = __ldcg(&ctl->nact[slot]);
       s_nexact = __ldcg(&ctl->nexact);
     }
     __syncthreads();

@@ -37,8 +37,8 @@ struct JacobiCtl {
   unsigned int bar[kMaxSolves];  // barrier arrivals of the launch whose first solve it is
   int iters[kMaxSolves];  // iterations of each solve of the current step
   int status;             // 0 ok, 1 maxiter, -4 watchdog
-  int pass_next;          // pass counter carried across solves (sum ring position)
-  int exact_next;         // the same of exact passes (acc ring position)
+  int pass_next;          // the next pass's position in the ring of sums, across solves
+  int exact_next;         // the next exact pass's position in the ring of limbs
 };
 
 struct AssembleArgs {

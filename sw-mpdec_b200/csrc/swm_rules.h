@@ -18,4 +18,12 @@ SWM_HD bool barrier_open(unsigned int count, unsigned int target) {
   return (int)(count - target) >= 0;
 }
 
+// Position `steps` (0..n) after `pos` (0..n-1) in a ring of n.  The passes of a step can
+// be more than an int counts (13 solves of any jacobi_maxiter), so positions are kept,
+// not pass numbers.
+SWM_HD int ring_at(int pos, int steps, int n) {
+  const int p = pos + steps;
+  return p >= n ? p - n : p;
+}
+
 }  // namespace swm

@@ -13,6 +13,7 @@ SOURCE = r"""
 #include "swm_rules.h"
 extern "C" {
 int barrier_open(unsigned c, unsigned t) { return swm::barrier_open(c, t); }
+int ring_at(int pos, int steps, int n) { return swm::ring_at(pos, steps, n); }
 }
 """
 
@@ -38,3 +39,10 @@ def test_barrier_opens_at_the_last_arrival_also_past_2_to_32(lib, blocks):
             got = lib.barrier_open(ctypes.c_uint(arrived % 2 ** 32),
                                    ctypes.c_uint(target % 2 ** 32))
             assert bool(got) == (arrived >= target), (nth, arrived - target)
+
+
+def test_ring_positions_stay_in_the_ring(lib):
+    for n in (3, 4):
+        for pos in range(n):
+            for steps in range(n + 1):
+                assert lib.ring_at(pos, steps, n) == (pos + steps) % n
