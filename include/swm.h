@@ -255,10 +255,13 @@ SWM_API int swm_jacobi_noalloc(int nx, int ny, const double *cS, const double *c
 /* Checked build only (libswm_checked.so, -DSWM_CHECKED): the device-side index checks
  * at the kernels' wrapped-index sites record a failure instead of touching memory out
  * of range.  Returns, and clears, the site of the first failing check (0 none; 1 RHS
- * tile load, 2/3 Jacobi tile loads, 4 CSR columns, 5 mPDeC2 compatibility read, 6
- * ensemble work item) and the number of failing checks; SWM_ERR_UNSUPPORTED in the
- * normal build. */
+ * tile load, 2/3 shared-memory Jacobi tile loads of the persistent ensemble step, 4 CSR
+ * columns, 5 mPDeC2 compatibility read, 6 ensemble work item, 7 register tiles and 8
+ * strips of the Jacobi, loads and stores, 9 neighbours of its one-sweep passes) and the
+ * number of failing checks; SWM_ERR_UNSUPPORTED in the normal build. */
 SWM_API int swm_debug_checked_status(int *site, unsigned long long *count);
+/* The sites whose checks ran since the last call (bit s: site s), read and cleared. */
+SWM_API int swm_debug_checked_sites(unsigned int *seen);
 
 /* ---- batched ensembles ---- */
 typedef struct swm_batch *swm_batch_handle;

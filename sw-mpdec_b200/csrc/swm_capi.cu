@@ -1615,6 +1615,20 @@ int swm_debug_checked_status(int* site, unsigned long long* count) {
   return SWM_OK;
 }
 
+int swm_debug_checked_sites(unsigned int* seen) {
+  if (!seen) return fail(SWM_ERR_PARAM, "null argument");
+#ifdef SWM_CHECKED
+  unsigned int m[3] = {0, 0, 0};
+  if (check_record_kernels_sites(&m[0]) || check_record_rhs_fast_sites(&m[1]) ||
+      check_record_rhs_exact_sites(&m[2]))
+    return fail(SWM_ERR_CUDA, "reading the checked-build records failed");
+  *seen = m[0] | m[1] | m[2];
+  return SWM_OK;
+#else
+  return fail(SWM_ERR_UNSUPPORTED, "not a checked build (-DSWM_CHECKED)");
+#endif
+}
+
 int swm_debug_set_tma(swm_handle s, int enable) {
   if (!s) return fail(SWM_ERR_PARAM, "null handle");
   s->tma = enable != 0;

@@ -56,16 +56,19 @@ __device__ __forceinline__ int wrap(int i, int n) {
 // loads of the RHS and the Jacobi, CSR column reads, the mPDeC2 compatibility read,
 // ensemble work items) check their index against the array's extent; a failing check
 // records its site (the first one, and a count) and the access is skipped, so that a
-// wrong index shows up as a status instead of a memory fault.  Without the flag the
-// checks compile to nothing.
+// wrong index shows up as a status instead of a memory fault.  Every check also notes
+// that its site was reached.  Without the flag the checks compile to nothing.
 enum {
-  kChkRhsLoad = 1, kChkJacPairs, kChkJacCells, kChkCsr, kChkCompat2, kChkEnsItem
+  kChkRhsLoad = 1, kChkJacPairs, kChkJacCells, kChkCsr, kChkCompat2, kChkEnsItem,
+  kChkJacTile, kChkJacStrip, kChkJacExact, kChkSites
 };
 #ifdef SWM_CHECKED
 // one record per translation unit (each unit's device code is a module of its own)
 static __device__ int g_swm_check_site;
 static __device__ unsigned long long g_swm_check_count;
+static __device__ int g_swm_check_seen[kChkSites];
 __device__ __forceinline__ bool swm_in_range(long long i, long long n, int site) {
+  *((volatile int*)&g_swm_check_seen[site]) = 1;
   if (i >= 0 && i < n) return true;
   atomicCAS(&g_swm_check_site, 0, site);
   atomicAdd(&g_swm_check_count, 1ull);
@@ -73,7 +76,7 @@ __device__ __forceinline__ bool swm_in_range(long long i, long long n, int site)
 }
 #define SWM_IN_RANGE(i, n, site) ::swm::swm_in_range((long long)(i), (long long)(n), (site))
 // Host reader of this unit's record, read and cleared: site of the first failing check
-// (0 none) and the number of failing checks.
+// (0 none) and the number of failing checks; fn_sites: the sites reached (bit s: site s).
 #define SWM_CHECK_READER(fn)                                                             \
   int fn(int* site, unsigned long long* count) {                                       \
     int zero = 0;                                                                      \
@@ -83,6 +86,15 @@ __device__ __forceinline__ bool swm_in_range(long long i, long long n, int site)
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_swm_check_site, &zero, sizeof(int)); \
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_swm_check_count, &zc, sizeof(zc));  \
     return e == cudaSuccess ? 0 : -1;                                                  \
+  }                                                                                    \
+  int fn##_sites(unsigned int* seen) {                                                 \
+    int mark[::swm::kChkSites], none[::swm::kChkSites] = {};                           \
+    cudaError_t e = cudaMemcpyFromSymbol(mark, g_swm_check_seen, sizeof(mark));        \
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_swm_check_seen, none, sizeof(none)); \
+    *seen = 0;                                                                         \
+    for (int s = 1; s < ::swm::kChkSites && e == cudaSuccess; ++s)                     \
+      if (mark[s]) *seen |= 1u << s;                                                   \
+    return e == cudaSuccess ? 0 : -1;                                                  \
   }
 #else
 #define SWM_IN_RANGE(i, n, site) true
@@ -90,6 +102,10 @@ __device__ __forceinline__ bool swm_in_range(long long i, long long n, int site)
   int fn(int* site, unsigned long long* count) {  \
     *site = -1;                                     \
     *count = 0;                                     \
+    return 0;                                       \
+  }                                                 \
+  int fn##_sites(unsigned int* seen) {              \
+    *seen = 0;                                      \
     return 0;                                       \
   }
 #endif

@@ -530,6 +530,9 @@ __device__ __forceinline__ double cell_update(const ExactGrid& g, const Sys& y, 
   } else {
     const int im = i == 0 ? g.nx - 1 : i - 1, ip = i == g.nx - 1 ? 0 : i + 1;
     const int jm = j == 0 ? g.ny - 1 : j - 1, jp = j == g.ny - 1 ? 0 : j + 1;
+    if (!SWM_IN_RANGE(im, g.nx, kChkJacExact) || !SWM_IN_RANGE(ip, g.nx, kChkJacExact) ||
+        !SWM_IN_RANGE(jm, g.ny, kChkJacExact) || !SWM_IN_RANGE(jp, g.ny, kChkJacExact))
+      return 0.;
     const size_t r = (size_t)j * g.pitch, c = r + i;
     p = __dmul_rn(y.cS[c], __ldcg(&xin[(size_t)jm * g.pitch + i]));
     p = __dadd_rn(p, __dmul_rn(y.cW[c], __ldcg(&xin[r + im])));

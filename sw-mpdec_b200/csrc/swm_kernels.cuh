@@ -297,6 +297,9 @@ size_t ensemble_smem_bytes(int tb, int precision);
 int check_record_kernels(int* site, unsigned long long* count);
 int check_record_rhs_fast(int* site, unsigned long long* count);
 int check_record_rhs_exact(int* site, unsigned long long* count);
+int check_record_kernels_sites(unsigned int* seen);
+int check_record_rhs_fast_sites(unsigned int* seen);
+int check_record_rhs_exact_sites(unsigned int* seen);
 
 // Host launchers (swm_kernels.cu, swm_rhs_*.cu)
 cudaError_t launch_rhs_batch_fast(int mode, const RhsArgs* descs, const int4* work, int nwork,

@@ -80,6 +80,13 @@ __device__ __forceinline__ StripLane strip_lane(int nx, int pitch, int strip, bo
   return L;
 }
 
+// (checked build) the pair's columns and row lie in the grid
+__device__ __forceinline__ bool pair_in_grid([[maybe_unused]] const StripLane& L,
+                                             [[maybe_unused]] int gj, [[maybe_unused]] int nx,
+                                             [[maybe_unused]] int ny, [[maybe_unused]] int site) {
+  return SWM_IN_RANGE(L.c0, nx, site) && SWM_IN_RANGE(L.c1, nx, site) && SWM_IN_RANGE(gj, ny, site);
+}
+
 __device__ __forceinline__ double2 ldcg2(const double* p) {
   return __ldcg(reinterpret_cast<const double2*>(p));
 }
@@ -100,12 +107,12 @@ __device__ __forceinline__ void pair_store(double* row, const StripLane& L, doub
 // Copy of row gj of the system and of the iterate into ring words dst[0 .. PL) (stride 32
 // words: one per lane).
 template <int FORM, typename Sys>
-__device__ __forceinline__ void strip_copy(const Sys& y, const double* xin, int nx, int pitch,
-                                           int gj, const StripLane& L, double2* dst) {
+__device__ __forceinline__ void strip_copy(const Sys& y, const double* xin, int nx, int ny,
+                                           int pitch, int gj, const StripLane& L, double2* dst) {
   using G = Strip<FORM>;
   const size_t row = (size_t)gj * pitch;
   const size_t k0 = row + L.c0, k1 = row + L.c1;
-  if (!SWM_IN_RANGE(L.c0, nx, kChkJacPairs) || !SWM_IN_RANGE(L.c1, nx, kChkJacPairs)) return;
+  if (!pair_in_grid(L, gj, nx, ny, kChkJacStrip)) return;
   auto plane = [&](int w, const double* p) {
     if (L.wide) {
       cp_async16(dst + 32 * w, p + k0);
@@ -245,7 +252,7 @@ __device__ __forceinline__ void strip_chunk(const Sys& y, const double* xin, dou
   int gj = wrap(j0 - Tp, ny);       // row of the next copy
 #pragma unroll
   for (int q = 0; q < NS - 1; ++q) {
-    if (q < total) strip_copy<FORM>(y, xin, nx, pitch, gj, L, mine + q * SLOT);
+    if (q < total) strip_copy<FORM>(y, xin, nx, ny, pitch, gj, L, mine + q * SLOT);
     cp_async_commit();
     gj = gj + 1 == ny ? 0 : gj + 1;
   }
@@ -274,7 +281,7 @@ __device__ __forceinline__ void strip_chunk(const Sys& y, const double* xin, dou
       double2* prev = mine + ((s - 1) & (NS - 1)) * SLOT;
       cf[(u + NL - 1) % NL] = strip_row<FORM>(prev, bad);  // row s - 1 of the system
       // the slot of row s - 1 is free: copy row s + NS - 1 into it
-      if (s + NS - 1 < total) strip_copy<FORM>(y, xin, nx, pitch, gj, L, prev);
+      if (s + NS - 1 < total) strip_copy<FORM>(y, xin, nx, ny, pitch, gj, L, prev);
       cp_async_commit();
       gj = gj + 1 == ny ? 0 : gj + 1;
       if (first && (unsigned)(s - Tp) < (unsigned)rows) {  // x^0 = b
@@ -302,7 +309,8 @@ __device__ __forceinline__ void strip_chunk(const Sys& y, const double* xin, dou
         n = v;
         if (t == Tp) res = v;
       }
-      if ((unsigned)(s - 2 * Tp) < (unsigned)rows)  // row s - Tp of x^{Tp}
+      if ((unsigned)(s - 2 * Tp) < (unsigned)rows &&  // row s - Tp of x^{Tp}
+          pair_in_grid(L, gs, nx, ny, kChkJacStrip))
         pair_store(xout + (size_t)gs * opitch, L, res);
       gs = gs + 1 == ny ? 0 : gs + 1;
     }
@@ -352,6 +360,12 @@ __device__ __forceinline__ void tile_rows(const JacobiSys& y, int nx, int ny, in
 #pragma unroll
   for (int r = 0; r < RW; ++r) {
     const size_t row = (size_t)gj * pitch;
+    const bool in = pair_in_grid(L, gj, nx, ny, kChkJacTile);
+    gj = gj + 1 == ny ? 0 : gj + 1;
+    if (!in) {
+      cf[r] = StripRow<FORM>{};
+      continue;
+    }
     if constexpr (FORM == kSysCsr) {
       const double *m0 = y.mass + 5 * (row + L.c0), *m1 = y.mass + 5 * (row + L.c1);
       if (L.wide) {
@@ -378,7 +392,6 @@ __device__ __forceinline__ void tile_rows(const JacobiSys& y, int nx, int ny, in
       cf[r].D = pair_load(y.cD + row, L);
     }
     if constexpr (FORM != kSysRecip) cf[r].B = pair_load(y.b + row, L);
-    gj = gj + 1 == ny ? 0 : gj + 1;
   }
 #pragma unroll
   for (int r = 0; r < RW; ++r) strip_rcp<FORM, true>(cf[r], bad);
@@ -407,7 +420,8 @@ __device__ __forceinline__ void tile_pass(const double* xin, double* xout, int n
   int gj = g0;
 #pragma unroll
   for (int r = 0; r < RW; ++r) {
-    x[r] = pair_load(xin + (size_t)gj * pitch, L);
+    x[r] = pair_in_grid(L, gj, nx, ny, kChkJacTile) ? pair_load(xin + (size_t)gj * pitch, L)
+                                                    : make_double2(0., 0.);
     gj = gj + 1 == ny ? 0 : gj + 1;
   }
   // rows this tile delivers, and counts
@@ -454,7 +468,8 @@ __device__ __forceinline__ void tile_pass(const double* xin, double* xout, int n
   gj = g0;
 #pragma unroll
   for (int r = 0; r < RW; ++r) {
-    if ((unsigned)(r0 + r) < rows) pair_store(xout + (size_t)gj * pitch, L, x[r]);
+    if ((unsigned)(r0 + r) < rows && pair_in_grid(L, gj, nx, ny, kChkJacTile))
+      pair_store(xout + (size_t)gj * pitch, L, x[r]);
     gj = gj + 1 == ny ? 0 : gj + 1;
   }
   if constexpr (FORM != kSysRecip) {

@@ -33,6 +33,7 @@ EXPORTS = [
     "swm_debug_set_tma", "swm_batch_debug_set_launches", "swm_batch_get_launch_info",
     "swm_batch_debug_phase_times", "swm_batch_debug_set_spin_limit",
     "swm_debug_checked_status",
+    "swm_debug_checked_sites",
 ]
 
 
@@ -126,6 +127,7 @@ def load():
     lib.swm_batch_debug_phase_times.argtypes = [vp, dp, ctypes.c_int, P(ctypes.c_int)]
     lib.swm_batch_debug_set_spin_limit.argtypes = [vp, ctypes.c_longlong]
     lib.swm_debug_checked_status.argtypes = [P(ctypes.c_int), P(ctypes.c_ulonglong)]
+    lib.swm_debug_checked_sites.argtypes = [P(ctypes.c_uint)]
     lib.swm_jacobi_noalloc.argtypes = ([ctypes.c_int, ctypes.c_int] + [vp] * 7 +
                                        [ctypes.c_int, ctypes.c_double, ctypes.c_int,
                                         P(ctypes.c_int), vp])
@@ -330,6 +332,13 @@ def checked_status():
     site, count = ctypes.c_int(), ctypes.c_ulonglong()
     _check(lib.swm_debug_checked_status(ctypes.byref(site), ctypes.byref(count)))
     return site.value, count.value
+
+
+def checked_sites():
+    """The set of sites whose index checks ran in the checked build, cleared."""
+    seen = ctypes.c_uint()
+    _check(load().swm_debug_checked_sites(ctypes.byref(seen)))
+    return {s for s in range(32) if seen.value >> s & 1}
 
 
 def inject_alloc_failure(nth):
