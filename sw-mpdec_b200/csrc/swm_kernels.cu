@@ -386,7 +386,7 @@ __device__ __forceinline__ int even_pass(int left, int blk) {
 // What a pass's outcome means for a system.  n: its cells; sum: the pass's residual
 // sums; hint: sweeps of the same substep's previous solve, or 0; out: the destination, or
 // b where a pass must not write it directly.
-template <bool RECIP>
+template <int FORM>
 __device__ __forceinline__ void sys_decide(SysState& S, double n, int maxiter, double thresh,
                                            const double* b, double* xa, double* xb, double* out,
                                            const double* sum, int hint, int blk) {
@@ -395,8 +395,12 @@ __device__ __forceinline__ void sys_decide(SysState& S, double n, int maxiter, d
     S.xin = S.xout;
     return;
   }
-  if (!RECIP && !(sum[1] < 0.5 * kBadSum)) {
-    S.exact = 1;  // an operand the fast divisions do not take
+  if (FORM != kSysRecip && !S.safe && !(sum[1] < 0.5 * kBadSum)) {
+    S.safe = 1;  // an operand the fast divisions do not take: the same pass again
+    return;
+  }
+  if (FORM == kSysCsr && S.safe && sum[1] >= 0.5 * kBadSum) {
+    S.exact = 1;  // a centre slot
     S.active = 0;
     return;
   }
@@ -476,7 +480,7 @@ __device__ __forceinline__ SysState sys_start(int maxiter, const double* b, doub
   S.k = 0;
   S.active = 1;
   S.first = 1;
-  S.rollback = S.zero = S.maxhit = S.exact = 0;
+  S.rollback = S.zero = S.maxhit = S.exact = S.safe = 0;
   S.r_prev = -1.f;
   return S;
 }
@@ -626,23 +630,25 @@ __device__ __noinline__ bool solve_exact(const ExactGrid& g, const Sys& y, SysSt
 
 // TILES: a block per tile and passes of up to TILES sweeps (small grids); 0: a warp per
 // chunk of a strip, passes of up to kPassT.
-template <int FORM, int TILES>
-__global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
-                                  TILES ? 1 : (FORM == kSysRecip ? 3 : 2))
-    jacobi_kernel(const __grid_constant__ JacobiGroup a) {
-  using G = Strip<FORM>;
-  constexpr int T = TILES ? TILES : kPassT, NW = TILES ? kTileWarps : kStripWarps;
-  using TG = Tile<FORM, T>;
+template <int TILES>
+struct PassShared {
+  static constexpr int T = TILES ? TILES : kPassT, NW = TILES ? kTileWarps : kStripWarps;
   static_assert(T <= kMaxBlock, "residual sums of a pass");
+  SysState st[kMaxSys];
+  double sum[NW][kMaxSys][T + 1], tot[kMaxSys][T + 1];
+  int ok, slot, xpass, nact, ch, act[kMaxSys], hint[kMaxSys];  // slot, xpass: ring positions
+  unsigned int nbar;
+};
+
+// Passes over the active systems until none is left, or a barrier wait gave up (sh.ok).
+template <int FORM, int TILES, bool SAFE>
+__device__ __forceinline__ void solve_passes(const JacobiGroup& a, PassShared<TILES>& sh) {
   extern __shared__ __align__(16) unsigned char jring[];
-  __shared__ SysState st[kMaxSys];
-  __shared__ double s_sum[NW][kMaxSys][T + 1], s_tot[kMaxSys][T + 1];
-  __shared__ int s_ok, s_xpass, s_nact, s_ch, s_act[kMaxSys], s_hint[kMaxSys];
-  __shared__ unsigned int s_nbar;
+  using G = Strip<FORM>;
+  constexpr int T = PassShared<TILES>::T, NW = PassShared<TILES>::NW;
+  using TG = Tile<FORM, T>;
   JacobiCtl* ctl = a.ctl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int blk = a.block < 1 ? 1 : (a.block > T ? T : a.block);
-  const double thresh = limbs_value(a.thresh[0], a.thresh[1], a.thresh[2]);
   const int strips = (a.nx + TG::UX - 1) / TG::UX, warps = gridDim.x * kStripWarps;
   const int tiles = TILES ? strips * ((a.ny + TG::UY - 1) / TG::UY) : 0;
   static_assert(TILES || G::U == TG::UX, "strips deliver as many columns as tiles");
@@ -651,42 +657,26 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
   auto plan = [&]() {
     int na = 0, most = 0;
     for (int q = 0; q < a.nsys; ++q)
-      if (st[q].active) {
-        if (lane == 0) s_act[na] = q;
+      if (sh.st[q].active) {
+        if (lane == 0) sh.act[na] = q;
         ++na;
-        most = max(most, st[q].Tp);
+        most = max(most, sh.st[q].Tp);
       }
     const int ch = !TILES && na ? strip_chunks(na, strips, a.ny, most, warps) : 1;
     if (lane == 0) {
-      s_nact = na;
-      s_ch = ch;
+      sh.nact = na;
+      sh.ch = ch;
     }
   };
-  int slot = 0;  // warp 0: position in the ring of sums
-  if (warp == 0) {
-    slot = *((volatile int*)&ctl->pass_next);
-    if (lane < a.nsys) {
-      const JacobiSys& y = a.sys[lane];
-      const int hint = y.hint_idx >= 0 ? __ldcg(&ctl->iters[y.hint_idx]) : 0;
-      s_hint[lane] = hint;
-      st[lane] = sys_start(a.maxiter, y.b, y.xa, y.out, hint, blk);
-    }
-    if (lane == 0) {
-      s_xpass = *((volatile int*)&ctl->exact_next);
-      s_nbar = 0;
-      s_ok = 1;
-    }
-    __syncwarp();
-    plan();
-  }
+  if (warp == 0) plan();
   __syncthreads();
   StripRow<FORM> cf[TILES ? TG::RW : 1];  // tiles: the rows held, of tile `held`
   int held = -1;
   bool held_bad = false;
-  while (s_nact > 0) {
-    for (int q = lane; q < kMaxSys * (T + 1); q += 32) (&s_sum[warp][0][0])[q] = 0.;
+  while (sh.nact > 0) {
+    for (int q = lane; q < kMaxSys * (T + 1); q += 32) (&sh.sum[warp][0][0])[q] = 0.;
     __syncwarp();
-    const int nact = s_nact;
+    const int nact = sh.nact;
     auto aligned = [&](const JacobiSys& y, const SysState& S) {
       unsigned long long al = (unsigned long long)S.xin | (unsigned long long)S.xout |
                               (unsigned long long)y.b;
@@ -699,39 +689,40 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
     };
     if constexpr (TILES) {
       for (int it = blockIdx.x; it < nact * tiles; it += gridDim.x) {
-        const int q = s_act[it / tiles], tile = it % tiles;
+        const int q = sh.act[it / tiles], tile = it % tiles;
         const JacobiSys& y = a.sys[q];
-        const SysState& S = st[q];
+        const SysState& S = sh.st[q];
         const int Tp = S.Tp, strip = tile % strips, j0 = (tile / strips) * TG::UY;
         const StripLane L = strip_lane<T>(a.nx, a.nx, strip, aligned(y, S));
         if (held != q * tiles + tile) {  // a block with one tile keeps its rows of the system
           held = q * tiles + tile;
           held_bad = false;
-          tile_rows<FORM>(y, a.nx, a.ny, a.nx, wrap(j0 + warp * TG::RW - T, a.ny), L, cf, held_bad);
+          tile_rows<FORM, SAFE>(y, a.nx, a.ny, a.nx, wrap(j0 + warp * TG::RW - T, a.ny), L, cf,
+                                held_bad);
         }
-        tile_pass<FORM, T>(S.xin, S.xout, a.nx, a.ny, a.nx, Tp, S.first != 0, j0, L, cf, held_bad,
-                           ring, s_sum[warp][q]);
+        tile_pass<FORM, T, SAFE>(S.xin, S.xout, a.nx, a.ny, a.nx, Tp, S.first != 0, j0, L, cf,
+                                 held_bad, ring, sh.sum[warp][q]);
         __syncthreads();  // the edge rows are read
       }
     } else {
-      const int ch = s_ch, R = (a.ny + ch - 1) / ch, items = nact * strips * ch;
+      const int ch = sh.ch, R = (a.ny + ch - 1) / ch, items = nact * strips * ch;
       // items in (system, chunk, strip) order over all CTAs first, so that few items
       // spread over many SMs and neighbouring strips stream together
       for (int it = warp * gridDim.x + blockIdx.x; it < items; it += warps) {
         const int strip = it % strips, rest = it / strips;
-        const int q = s_act[rest / ch], j0 = (rest % ch) * R, rows = min(R, a.ny - j0);
+        const int q = sh.act[rest / ch], j0 = (rest % ch) * R, rows = min(R, a.ny - j0);
         if (rows <= 0) continue;
         const JacobiSys& y = a.sys[q];
-        const SysState& S = st[q];
+        const SysState& S = sh.st[q];
         const int Tp = S.Tp;
         double sum[T + 1];
-        strip_pass<FORM>(y, S.xin, S.xout, a.nx, a.ny, a.nx, a.nx, Tp, S.first != 0, strip, j0,
-                         rows, aligned(y, S), ring, sum);
+        strip_pass<FORM, SAFE>(y, S.xin, S.xout, a.nx, a.ny, a.nx, a.nx, Tp, S.first != 0, strip,
+                               j0, rows, aligned(y, S), ring, sum);
 #pragma unroll
         for (int t = 0; t <= T; ++t) {
           if (t > Tp) break;
           const double v = warp_sum(sum[t]);
-          if (lane == 0) s_sum[warp][q][t] += v;
+          if (lane == 0) sh.sum[warp][q][t] += v;
         }
       }
     }
@@ -739,57 +730,115 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
     if (warp == 0) {
       // the block's sums, the grid barrier, then every block's decisions from the totals
       static_assert(kMaxSys * (T + 1) <= 32, "a lane per sum");
-      const int q = lane / (T + 1), t = lane % (T + 1);
-      const bool mine = q < a.nsys && st[q < kMaxSys ? q : 0].active;
+      const int slot = sh.slot, q = lane / (T + 1), t = lane % (T + 1);
+      const bool mine = q < a.nsys && sh.st[q < kMaxSys ? q : 0].active;
       if (mine) {
-        double v = s_sum[0][q][t];
-        for (int w = 1; w < NW; ++w) v += s_sum[w][q][t];
+        double v = sh.sum[0][q][t];
+        for (int w = 1; w < NW; ++w) v += sh.sum[w][q][t];
         if (v != 0.) atomicAdd(&ctl->sum[slot][q][t], v);
       }
       __syncwarp();
       if (lane == 0)
-        s_ok = arrive_and_wait(&ctl->bar[a.sys[0].solve_idx], ++s_nbar, a.spin_limit, &ctl->status);
+        sh.ok = arrive_and_wait(&ctl->bar[a.sys[0].solve_idx], ++sh.nbar, a.spin_limit,
+                                &ctl->status);
       __syncwarp();
-      if (s_ok) {
-        if (mine) s_tot[q][t] = __ldcg(&ctl->sum[slot][q][t]);
+      if (sh.ok) {
+        if (mine) sh.tot[q][t] = __ldcg(&ctl->sum[slot][q][t]);
         if (blockIdx.x == 0) {  // recycle the slot of the pass before this one
           for (int z = lane; z < kMaxSys * (kMaxBlock + 1); z += 32)
             (&ctl->sum[ring_at(slot, 2, kResSlots)][0][0])[z] = 0.;
           __threadfence();
         }
         __syncwarp();
-        if (lane < a.nsys && st[lane].active) {
+        if (lane < a.nsys && sh.st[lane].active) {
           const JacobiSys& y = a.sys[lane];
-          sys_decide<FORM == kSysRecip>(st[lane], (double)a.nx * a.ny, a.maxiter, thresh, y.b, y.xa,
-                                        y.xb, y.out, s_tot[lane], s_hint[lane], blk);
+          const int blk = a.block < 1 ? 1 : (a.block > T ? T : a.block);
+          const double thresh = limbs_value(a.thresh[0], a.thresh[1], a.thresh[2]);
+          sys_decide<FORM>(sh.st[lane], (double)a.nx * a.ny, a.maxiter, thresh, y.b, y.xa, y.xb,
+                           y.out, sh.tot[lane], sh.hint[lane], blk);
+          // its passes come after the fast ones'
+          if (!SAFE && sh.st[lane].safe) sh.st[lane].active = 0;
         }
         __syncwarp();
         plan();
-        slot = ring_at(slot, 1, kResSlots);
+        if (lane == 0) sh.slot = ring_at(slot, 1, kResSlots);
       }
     }
     __syncthreads();
-    if (!s_ok) return;
+    if (!sh.ok) return;
   }
+}
+
+// The systems that the fast passes left: by passes with IEEE divisions, or one sweep at a
+// time.  One call out of line: what it needs must not come out of the fast passes'
+// registers.
+template <int FORM, int TILES>
+__device__ __noinline__ void solve_rest(const JacobiGroup& a, PassShared<TILES>& sh) {
+  if constexpr (FORM != kSysRecip) {
+    if (threadIdx.x < a.nsys) sh.st[threadIdx.x].active = sh.st[threadIdx.x].safe;
+    __syncwarp();  // (warp 0 reads them first)
+    solve_passes<FORM, TILES, true>(a, sh);
+    if (!sh.ok) return;
+  }
+  JacobiCtl* ctl = a.ctl;
   const ExactGrid eg{a.nx,   a.ny,     a.nx,       a.maxiter, a.thresh, a.rowstart, a.cols,
                      ctl->acc, &ctl->bar[a.sys[0].solve_idx], &ctl->status, a.spin_limit};
   for (int q = 0; q < a.nsys; ++q)
-    if (st[q].exact && !solve_exact<FORM>(eg, a.sys[q], st[q], &s_xpass, &s_nbar)) return;
+    if (sh.st[q].exact && !solve_exact<FORM>(eg, a.sys[q], sh.st[q], &sh.xpass, &sh.nbar)) {
+      __syncthreads();
+      if (threadIdx.x == 0) sh.ok = 0;
+      __syncthreads();
+      return;
+    }
+}
+
+template <int FORM, int TILES>
+__global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
+                                  TILES ? 1 : (FORM == kSysRecip ? 3 : 2))
+    jacobi_kernel(const __grid_constant__ JacobiGroup a) {
+  constexpr int T = PassShared<TILES>::T;
+  __shared__ PassShared<TILES> sh;
+  JacobiCtl* ctl = a.ctl;
+  if (threadIdx.x < 32) {
+    if (threadIdx.x < a.nsys) {
+      const JacobiSys& y = a.sys[threadIdx.x];
+      const int blk = a.block < 1 ? 1 : (a.block > T ? T : a.block);
+      const int hint = y.hint_idx >= 0 ? __ldcg(&ctl->iters[y.hint_idx]) : 0;
+      sh.hint[threadIdx.x] = hint;
+      sh.st[threadIdx.x] = sys_start(a.maxiter, y.b, y.xa, y.out, hint, blk);
+    }
+    if (threadIdx.x == 0) {
+      sh.slot = *((volatile int*)&ctl->pass_next);
+      sh.xpass = *((volatile int*)&ctl->exact_next);
+      sh.nbar = 0;
+      sh.ok = 1;
+    }
+    __syncwarp();
+  }
+  solve_passes<FORM, TILES, false>(a, sh);
+  if (!sh.ok) return;
+  bool rest = false;
+  for (int q = 0; q < a.nsys; ++q) rest = rest || sh.st[q].safe || sh.st[q].exact;
+  if (rest) {
+    __syncthreads();
+    solve_rest<FORM, TILES>(a, sh);
+    if (!sh.ok) return;
+  }
   // deliver the final iterates (haVec of the reference) to their destinations
   const int n = a.nx * a.ny;
   for (int q = 0; q < a.nsys; ++q) {
     const JacobiSys& y = a.sys[q];
-    if (!st[q].zero && st[q].xin == y.out) continue;
+    if (!sh.st[q].zero && sh.st[q].xin == y.out) continue;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
-      y.out[c] = st[q].zero ? 0. : __ldcg(&st[q].xin[c]);
+      y.out[c] = sh.st[q].zero ? 0. : __ldcg(&sh.st[q].xin[c]);
   }
   if (blockIdx.x == 0 && threadIdx.x < a.nsys) {
-    const SysState& S = st[threadIdx.x];
+    const SysState& S = sh.st[threadIdx.x];
     ctl->iters[a.sys[threadIdx.x].solve_idx] = S.zero ? 0 : S.k;
     if (S.maxhit) atomicCAS(&ctl->status, 0, 1);
     if (threadIdx.x == 0) {
-      *((volatile int*)&ctl->pass_next) = slot;
-      *((volatile int*)&ctl->exact_next) = s_xpass;
+      *((volatile int*)&ctl->pass_next) = sh.slot;
+      *((volatile int*)&ctl->exact_next) = sh.xpass;
     }
   }
 }
@@ -918,7 +967,7 @@ __global__ void __launch_bounds__(kStripNT, FORM == kSysRecip ? 3 : 2)
       const int4 it = a.items[w - set * a.nitems];
       const int sys = set * a.nprob + it.x;
       const JacobiArgs& d = a.descs[sys];
-      int Tp, first, active = 1;
+      int Tp, first, active = 1, safe = 0;
       const double* xin;
       double* xout;
       if (!begun) {  // the states are written by the first decisions
@@ -932,6 +981,7 @@ __global__ void __launch_bounds__(kStripNT, FORM == kSysRecip ? 3 : 2)
         active = __ldcg(&S->active);
         Tp = __ldcg(&S->Tp);
         first = __ldcg(&S->first);
+        safe = __ldcg(&S->safe);
         xin = reinterpret_cast<const double*>(__ldcg(reinterpret_cast<const unsigned long long*>(&S->xin)));
         xout = reinterpret_cast<double*>(__ldcg(reinterpret_cast<const unsigned long long*>(&S->xout)));
       }
@@ -941,14 +991,24 @@ __global__ void __launch_bounds__(kStripNT, FORM == kSysRecip ? 3 : 2)
             (unsigned long long)xin | (unsigned long long)xout | (unsigned long long)d.b |
             (unsigned long long)d.cS | (unsigned long long)d.cW | (unsigned long long)d.cE |
             (unsigned long long)d.cN | (unsigned long long)d.cD;
-        double sum[T + 1];
-        strip_pass<FORM>(d, xin, xout, nx, ny, pitch, pitch, Tp, first != 0, it.y, it.z, it.w,
-                         (al & 15ull) == 0, ring, sum);
+        auto add = [&](const double (&sum)[T + 1]) {
 #pragma unroll
-        for (int t = 0; t <= T; ++t) {
-          if (t > Tp) break;
-          sum[t] = warp_sum(sum[t]);
-          if (lane == t && sum[t] != 0.) atomicAdd(&a.st[sys].sum[t], sum[t]);
+          for (int t = 0; t <= T; ++t) {
+            if (t > Tp) break;
+            const double v = warp_sum(sum[t]);
+            if (lane == t && v != 0.) atomicAdd(&a.st[sys].sum[t], v);
+          }
+        };
+        if (!RECIP && safe) {  // (its sums are in local memory)
+          double sum[T + 1];
+          strip_pass_safe<FORM>(d, xin, xout, nx, ny, pitch, pitch, Tp, first != 0, it.y, it.z,
+                                it.w, (al & 15ull) == 0, ring, sum);
+          add(sum);
+        } else {
+          double sum[T + 1];
+          strip_pass<FORM, false>(d, xin, xout, nx, ny, pitch, pitch, Tp, first != 0, it.y, it.z,
+                                  it.w, (al & 15ull) == 0, ring, sum);
+          add(sum);
         }
       }
       w = (int)__shfl_sync(0xffffffffu, nw, 0);
@@ -970,7 +1030,7 @@ __global__ void __launch_bounds__(kStripNT, FORM == kSysRecip ? 3 : 2)
         B.sum[t] = 0.;
       }
       const double thresh = limbs_value(d.thresh[0], d.thresh[1], d.thresh[2]);
-      sys_decide<RECIP>(S, (double)d.nx * d.ny, d.maxiter, thresh, d.b, d.xa, d.xb, direct(d), sum,
+      sys_decide<FORM>(S, (double)d.nx * d.ny, d.maxiter, thresh, d.b, d.xa, d.xb, direct(d), sum,
                         a.hint ? __ldg(&a.hint[p]) : 0, blk);
       B.s = S;
       if (S.active) atomicAdd(&ctl->nact[slot], 1);

@@ -204,6 +204,7 @@ struct SysState {
   int zero;         // converged before the first sweep: the reference returns 0
   int maxhit;
   int exact;        // left to solve_exact, which goes on from xin
+  int safe;         // its passes divide by IEEE divisions
   float r_prev;     // residual sum of the last sweep of the previous pass (planning)
 };
 constexpr int kJacobiBatchWarps = 4;  // warps per block of the batched solve

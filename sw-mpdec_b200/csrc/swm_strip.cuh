@@ -156,9 +156,10 @@ __device__ __forceinline__ bool strip_num(double x) {
 }
 // RN(1/D) of a row: strips form one per step, without a branch; tiles once per load, by
 // __drcp_rn, whose branches keep the registers of a thread's rows from all being live.
-template <int FORM, bool TILE>
+// (SAFE passes divide by D.)
+template <int FORM, bool TILE, bool SAFE>
 __device__ __forceinline__ void strip_rcp(StripRow<FORM>& r, bool& bad) {
-  if constexpr (FORM != kSysRecip) {
+  if constexpr (FORM != kSysRecip && !SAFE) {
     bad |= !strip_range(r.D.x) || !strip_range(r.D.y);
     if constexpr (TILE) {
       r.R = make_double2(__drcp_rn(r.D.x), __drcp_rn(r.D.y));
@@ -173,7 +174,7 @@ __device__ __forceinline__ void strip_rcp(StripRow<FORM>& r, bool& bad) {
 // sum rounded, in the reference's CSR order (the zero centre slot adds an exact zero);
 // RECIP: b/D - sum of the divided row.  part: the S, W and E products; full: the rest.
 // The quotient is formed by div_mk from RN(1/D), the correctly rounded one for operands
-// in strip_range.
+// in strip_range; SAFE: by the IEEE division, for any operands.
 template <int FORM>
 __device__ __forceinline__ double2 pair_part(const StripRow<FORM>& c, double2 south, double2 mid,
                                              double west, double east) {
@@ -184,7 +185,7 @@ __device__ __forceinline__ double2 pair_part(const StripRow<FORM>& c, double2 so
   p.y = __dadd_rn(p.y, __dmul_rn(c.E.y, east));
   return p;
 }
-template <int FORM>
+template <int FORM, bool SAFE>
 __device__ __forceinline__ double2 pair_full(const StripRow<FORM>& c, double2 part, double2 north,
                                              bool& bad) {
   const double px = __dadd_rn(part.x, __dmul_rn(c.N.x, north.x));
@@ -193,18 +194,20 @@ __device__ __forceinline__ double2 pair_full(const StripRow<FORM>& c, double2 pa
     return make_double2(__dsub_rn(c.D.x, px), __dsub_rn(c.D.y, py));
   } else {
     const double ax = __dsub_rn(c.B.x, px), ay = __dsub_rn(c.B.y, py);
+    if constexpr (SAFE) return make_double2(__ddiv_rn(ax, c.D.x), __ddiv_rn(ay, c.D.y));
     bad |= !strip_num(ax) || !strip_num(ay);
     return make_double2(div_mk(ax, c.D.x, c.R.x), div_mk(ay, c.D.y, c.R.y));
   }
 }
 
 // A chunk or tile with an operand outside those ranges adds this to its first residual
-// sum, and the solve goes on one sweep at a time with IEEE divisions (solve_exact).
+// sum: the pass is redone, and the solve goes on, with SAFE passes.  So does one with a
+// non-zero CSR centre slot, whose product all passes leave out as the exact zero it is in a
+// Patankar system; a SAFE pass that reports it leaves the solve to solve_exact.
 constexpr double kBadSum = 0x1p1000;
 
-// bad: an operand the fast sweeps do not take (strip_ok; CSR: a non-zero centre slot,
-// whose product the sweeps leave out as the exact zero it is in a Patankar system).
-template <int FORM>
+// bad: an operand the pass does not take.
+template <int FORM, bool SAFE>
 __device__ __forceinline__ StripRow<FORM> strip_row(const double2* w, bool& bad) {
   StripRow<FORM> r;
   if constexpr (FORM == kSysCsr) {
@@ -224,7 +227,7 @@ __device__ __forceinline__ StripRow<FORM> strip_row(const double2* w, bool& bad)
     r.D = w[128];
     if constexpr (FORM == kSysDiv) r.B = w[160];
   }
-  strip_rcp<FORM, false>(r, bad);
+  strip_rcp<FORM, false, SAFE>(r, bad);
   return r;
 }
 
@@ -237,7 +240,7 @@ __device__ __forceinline__ StripRow<FORM> strip_row(const double2* w, bool& bad)
 // NL sweeps are formed first: few dependent operations per sweep are left in series.
 // Steps before a sweep's first row compute on the zeros and unit rows set below and
 // deliver nothing.
-template <int FORM, int NL, typename Sys>
+template <int FORM, int NL, bool SAFE, typename Sys>
 __device__ __forceinline__ void strip_chunk(const Sys& y, const double* xin, double* xout,
                                             int nx, int ny, int pitch, int opitch, int Tp,
                                             bool first, int strip, int j0, int rows, bool aligned,
@@ -279,7 +282,7 @@ __device__ __forceinline__ void strip_chunk(const Sys& y, const double* xin, dou
       cp_async_wait<NS - 2>();  // row s has arrived
       double2 n = mine[(s & (NS - 1)) * SLOT + 32 * G::XPL];
       double2* prev = mine + ((s - 1) & (NS - 1)) * SLOT;
-      cf[(u + NL - 1) % NL] = strip_row<FORM>(prev, bad);  // row s - 1 of the system
+      cf[(u + NL - 1) % NL] = strip_row<FORM, SAFE>(prev, bad);  // row s - 1 of the system
       // the slot of row s - 1 is free: copy row s + NS - 1 into it
       if (s + NS - 1 < total) strip_copy<FORM>(y, xin, nx, ny, pitch, gj, L, prev);
       cp_async_commit();
@@ -301,7 +304,7 @@ __device__ __forceinline__ void strip_chunk(const Sys& y, const double* xin, dou
 #pragma unroll
       for (int t = 1; t <= NL; ++t) {
         const double2 m = x[t - 1][(u + 2 * NL - t) & 1];
-        const double2 v = pair_full<FORM>(cf[(u + NL - t) % NL], part[t - 1], n, bad);
+        const double2 v = pair_full<FORM, SAFE>(cf[(u + NL - t) % NL], part[t - 1], n, bad);
         const bool in = (unsigned)(s - t - Tp) < (unsigned)rows;
         if (in && L.own0) sum[t] = __dadd_rn(sum[t], fabs(__dsub_rn(v.x, m.x)));
         if (in && L.own1) sum[t] = __dadd_rn(sum[t], fabs(__dsub_rn(v.y, m.y)));
@@ -321,7 +324,7 @@ __device__ __forceinline__ void strip_chunk(const Sys& y, const double* xin, dou
 
 // Tp sweeps over one chunk by the code of the next even number of sweeps, the lane's
 // sums in sum.
-template <int FORM, typename Sys>
+template <int FORM, bool SAFE, typename Sys>
 __device__ __forceinline__ void strip_pass(const Sys& y, const double* xin, double* xout,
                                            int nx, int ny, int pitch, int opitch, int Tp,
                                            bool first, int strip, int j0, int rows, bool aligned,
@@ -329,11 +332,21 @@ __device__ __forceinline__ void strip_pass(const Sys& y, const double* xin, doub
   static_assert(kPassT == 4, "the pass lengths below");
 #pragma unroll
   for (int t = 0; t <= kPassT; ++t) sum[t] = 0.;
-  if (Tp <= 2)
-    strip_chunk<FORM, 2>(y, xin, xout, nx, ny, pitch, opitch, Tp, first, strip, j0, rows, aligned,
-                         ring, sum);
+  if (Tp <= 2 && !SAFE)
+    strip_chunk<FORM, 2, SAFE>(y, xin, xout, nx, ny, pitch, opitch, Tp, first, strip, j0, rows,
+                               aligned, ring, sum);
   else
-    strip_chunk<FORM, 4>(y, xin, xout, nx, ny, pitch, opitch, Tp, first, strip, j0, rows, aligned,
+    strip_chunk<FORM, 4, SAFE>(y, xin, xout, nx, ny, pitch, opitch, Tp, first, strip, j0, rows,
+                               aligned, ring, sum);
+}
+// SAFE out of line, for a loop that also holds the other: its registers must not come out
+// of that one's.
+template <int FORM, typename Sys>
+__device__ __noinline__ void strip_pass_safe(const Sys& y, const double* xin, double* xout,
+                                             int nx, int ny, int pitch, int opitch, int Tp,
+                                             bool first, int strip, int j0, int rows, bool aligned,
+                                             double2* ring, double (&sum)[kPassT + 1]) {
+  strip_pass<FORM, true>(y, xin, xout, nx, ny, pitch, opitch, Tp, first, strip, j0, rows, aligned,
                          ring, sum);
 }
 
@@ -354,7 +367,7 @@ struct Tile {
 };
 
 // The rows of the system a thread holds (pair of columns L.c0, L.c1; rows gj, gj + 1, ..).
-template <int FORM, int RW>
+template <int FORM, bool SAFE, int RW>
 __device__ __forceinline__ void tile_rows(const JacobiSys& y, int nx, int ny, int pitch, int gj,
                                           const StripLane& L, StripRow<FORM> (&cf)[RW], bool& bad) {
 #pragma unroll
@@ -394,7 +407,7 @@ __device__ __forceinline__ void tile_rows(const JacobiSys& y, int nx, int ny, in
     if constexpr (FORM != kSysRecip) cf[r].B = pair_load(y.b + row, L);
   }
 #pragma unroll
-  for (int r = 0; r < RW; ++r) strip_rcp<FORM, true>(cf[r], bad);
+  for (int r = 0; r < RW; ++r) strip_rcp<FORM, true, SAFE>(cf[r], bad);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -406,7 +419,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 // Tp <= T sweeps over the tile at (i0, j0) whose rows of the system are in cf; the warp's
 // residual sums are added to sum[0..T] (shared memory) as strip_chunk's.  Every thread of
 // the block takes part.
-template <int FORM, int T>
+template <int FORM, int T, bool SAFE>
 __device__ __forceinline__ void tile_pass(const double* xin, double* xout, int nx, int ny,
                                           int pitch, int Tp, bool first, int j0,
                                           const StripLane& L,
@@ -456,7 +469,7 @@ __device__ __forceinline__ void tile_pass(const double* xin, double* xout, int n
       const double2 m = x[r];
       const double2 part = pair_part<FORM>(cf[r], south, m, __shfl_up_sync(0xffffffffu, m.y, 1),
                                            __shfl_down_sync(0xffffffffu, m.x, 1));
-      const double2 v = pair_full<FORM>(cf[r], part, r + 1 < RW ? x[r + 1 < RW ? r + 1 : r] : hi, bad);
+      const double2 v = pair_full<FORM, SAFE>(cf[r], part, r + 1 < RW ? x[r + 1 < RW ? r + 1 : r] : hi, bad);
       const bool in = (unsigned)(r0 + r) < rows;
       if (in && L.own0) s = __dadd_rn(s, fabs(__dsub_rn(v.x, m.x)));
       if (in && L.own1) s = __dadd_rn(s, fabs(__dsub_rn(v.y, m.y)));
