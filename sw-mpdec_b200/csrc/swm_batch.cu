@@ -534,32 +534,31 @@ static int batch_tune(swm_batch* b) {
   cudaEvent_t e0, e1;
   BCK(cudaEventCreate(&e0));
   BCK(cudaEventCreate(&e1));
-  float best = 1e30f;
-  Cand pick = cands[0];
-  // A form whose first schedule takes a fifth longer than the best so far is not tried
-  // further (256-problem split ensemble: 42 ms a step per phase, 60 ms for the persistent
-  // form's best schedule): the trials are paid by the first step.
-  bool skip[2] = {false, false};
-  for (const auto& c : cands) {
-    if (skip[c.persistent]) continue;
+  // The trials are paid by the first step: a form whose first schedule is far behind is
+  // left (256-problem split ensemble: 37 ms a step per phase, 57 ms for the persistent
+  // form's best schedule).
+  auto trial = [&](const Cand& c, float* ms) -> int {
     for (int rep = 0; rep < 2; ++rep) {  // first repetition warms the kernels
       BCK(cudaEventRecord(e0, b->stream));
-      if ((rc = batch_enqueue(b, c.persistent, c.block, c.grid))) return rc;
+      if (int rc = batch_enqueue(b, c.persistent, c.block, c.grid)) return rc;
       BCK(cudaEventRecord(e1, b->stream));
       BCK(cudaStreamSynchronize(b->stream));
-      if ((rc = batch_copy_state(b, false))) return rc;
+      if (int rc = batch_copy_state(b, false)) return rc;
     }
-    float ms = 0.f;
-    BCK(cudaEventElapsedTime(&ms, e0, e1));
-    if (ms > 1.2f * best) skip[c.persistent] = true;
-    if (ms < best) {
-      best = ms;
-      pick = c;
-    }
-  }
-  BCK(cudaStreamSynchronize(b->stream));
+    BCK(cudaEventElapsedTime(ms, e0, e1));
+    return SWM_OK;
+  };
+  const int kept = fastest_schedule(
+      (int)cands.size(), [&](int i) { return cands[i].persistent ? 1 : 0; },
+      [&](int i) {
+        float ms = 0.f;
+        return (rc = trial(cands[i], &ms)) ? -1.f : ms;
+      });
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  if (kept < 0) return rc;
+  const Cand pick = cands[kept];
+  BCK(cudaStreamSynchronize(b->stream));
   b->persistent = pick.persistent;
   b->block = pick.block;
   b->ens_grid = pick.grid;

@@ -26,4 +26,28 @@ SWM_HD int ring_at(int pos, int steps, int n) {
   return p >= n ? p - n : p;
 }
 
+// The fastest of n schedules, tried in order: form(i) is 0 or 1, time(i) its time, negative
+// when it failed (which ends the search: -1).  A form whose first schedule takes a fifth
+// longer than the best so far is not tried further; a later schedule of a form says
+// nothing about the others.
+template <typename Form, typename Time>
+inline int fastest_schedule(int n, Form form, Time time) {
+  int pick = -1;
+  float best = 0.f;
+  bool tried[2] = {}, skip[2] = {};
+  for (int i = 0; i < n; ++i) {
+    const int f = form(i);
+    if (skip[f]) continue;
+    const float ms = time(i);
+    if (ms < 0.f) return -1;
+    if (!tried[f] && pick >= 0 && ms > 1.2f * best) skip[f] = true;
+    tried[f] = true;
+    if (pick < 0 || ms < best) {
+      best = ms;
+      pick = i;
+    }
+  }
+  return pick;
+}
+
 }  // namespace swm
