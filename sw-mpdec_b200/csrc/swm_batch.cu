@@ -523,8 +523,8 @@ static int batch_tune(swm_batch* b) {
   for (bool pers : {false, true}) {
     if (b->mode_fixed && pers != b->persistent) continue;
     for (int c : kCandidates) {
-      if (!pers) {  // the strips sweep at most 4 times per pass
-        if (c <= 4) cands.push_back({false, c, 0});
+      if (!pers) {
+        if (c <= kPassT) cands.push_back({false, c, 0});
         continue;
       }
       cands.push_back({true, c, b->ens_max[c]});
@@ -766,7 +766,7 @@ int swm_batch_cells(swm_batch_handle b, long long* cells) {
 int swm_batch_get_stats(swm_batch_handle b, int* jacobi_block, long long* iters_total,
                         int* last_iters) {
   if (!b) return bfail(SWM_ERR_PARAM, "null handle");
-  if (jacobi_block) *jacobi_block = b->block;
+  if (jacobi_block) *jacobi_block = b->persistent ? b->block : std::min(b->block, kPassT);
   if (iters_total) *iters_total = b->iters_total;
   if (last_iters)
     for (size_t k = 0; k < b->h_iters.size(); ++k) last_iters[k] = b->h_iters[k];

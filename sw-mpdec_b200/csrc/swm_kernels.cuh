@@ -207,6 +207,7 @@ struct SysState {
   int safe;         // its passes divide by IEEE divisions
   float r_prev;     // residual sum of the last sweep of the previous pass (planning)
 };
+constexpr int kPassT = 4;  // sweeps per pass of the strips at most
 constexpr int kJacobiBatchWarps = 4;  // warps per block of the batched solve
 constexpr int kBatchSums = 8;  // residual sums of a pass, padded
 struct StripBatchState {

@@ -30,7 +30,7 @@ constexpr int kStripNT = 32 * kStripWarps;
 constexpr int kStripSlots = 4;                   // ring rows: three copies ahead of the sweeps
 constexpr int kStripCols = 64;                   // columns a warp loads
 
-constexpr int kPassT = 4;  // sweeps per pass at most; even: pairs keep their alignment
+static_assert(kPassT % 2 == 0, "pairs keep their alignment");
 
 template <int FORM>
 struct Strip {
