@@ -336,13 +336,11 @@ cudaError_t launch_combo(const ComboArgs& a, cudaStream_t s) {
 // on the exact sum of |dx| rounded to multiples of 2^-100.  A pass sums |dx| in FP64, in
 // any order: n terms, so within n 2^-53 < 2^-24 of the sum of the unrounded terms, and
 // those are within n 2^-101 of the rounded ones.  Outside kBand of the threshold the
-// order therefore cannot change the decision; a sum inside the band (about one solve in
+// order therefore cannot change the decision (stop_decision); a sum inside the band (about one solve in
 // 10^5, or tol = 0) hands the system to solve_exact, which goes on from the pass's input
 // one sweep at a time with exact integer sums.  The iterates and the stop index depend
 // on neither tiling, launch shape nor atomic order.
 // ---------------------------------------------------------------------------
-constexpr double kBand = 0x1p-20;
-
 // Grid barrier number `nth` (1, 2, ..) of a launch on its own arrival counter (zero when
 // the launch starts), by one thread: everything its block wrote before a block barrier is
 // visible to every block after it (the arrival releases, the poll acquires; both are
@@ -368,13 +366,6 @@ __device__ __forceinline__ bool arrive_and_wait(unsigned int* ctr, unsigned int 
     }
   }
   return ok;
-}
-
-// 1 stop, 0 go on, -1 inside the band (NaN and infinite sums go on, as in exact sums).
-__device__ __forceinline__ int stop_decision(double s, double thresh, double n) {
-  const double slack = n * 0x1p-100;
-  if (!(s <= thresh * (1.0 + kBand) + slack)) return 0;
-  return s <= thresh * (1.0 - kBand) - slack ? 1 : -1;
 }
 
 // Sweeps of a pass when `left` more are expected: as few passes as blk allows, evenly.

@@ -26,6 +26,20 @@ SWM_HD int ring_at(int pos, int steps, int n) {
   return p >= n ? p - n : p;
 }
 
+// Half width, relative to the threshold, of the band of FP64 residual sums that leave the
+// decision to exact sums.
+constexpr double kBand = 0x1p-20;
+
+// A pass's sum s of n terms, in any order, against the stop threshold: 1 stop, 0 go on, -1
+// inside the band (NaN and infinite sums go on, as in exact sums).  n 2^-100 covers the
+// truncation of the exact rule's terms; kBand the rounding of s (within n 2^-53 < 2^-24)
+// and of thresh, the double nearest the limbs (limbs_value: within 2^-51).
+SWM_HD int stop_decision(double s, double thresh, double n) {
+  const double slack = n * 0x1p-100;
+  if (!(s <= thresh * (1.0 + kBand) + slack)) return 0;
+  return s <= thresh * (1.0 - kBand) - slack ? 1 : -1;
+}
+
 // The fastest of n schedules, tried in order: form(i) is 0 or 1, time(i) its time, negative
 // when it failed (which ends the search: -1).  A form whose first schedule takes a fifth
 // longer than the best so far is not tried further; a later schedule of a form says

@@ -63,7 +63,9 @@ __device__ __forceinline__ bool limbs_le(unsigned long long s2, unsigned long lo
   return s0 <= t[2];
 }
 
-// Approximate value of a limb sum (2^-100 units) for planning only.
+// The value of a limb sum (2^-100 units), rounded: three conversions and two sums of
+// non-negative terms, within 2^-51 of it, which the band around the stop threshold
+// (kBand) covers.
 __device__ __forceinline__ double limbs_value(unsigned long long s2, unsigned long long s1,
                                               unsigned long long s0) {
   return __dadd_rn(__dadd_rn(__dmul_rn((double)s2, 0x1p-20), __dmul_rn((double)s1, 0x1p-60)),
