@@ -247,7 +247,7 @@ static RhsArgs make_rhs_args(swm_solver* s, const double* h, const double* hu, c
   a.src_cols = s->src_cols;
   a.src_rows = s->src_rows;
   a.bgrad = s->bgrad;
-  a.over_len = fast_patankar(s->p) ? 0 : 1;
+  a.over_len = fluxes_over_len(s->p.timescheme, fast_patankar(s->p)) ? 1 : 0;
   a.status = &s->ctl->status;
   return a;
 }

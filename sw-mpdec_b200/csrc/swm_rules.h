@@ -40,6 +40,10 @@ SWM_HD int stop_decision(double s, double thresh, double n) {
   return s <= thresh * (1.0 - kBand) - slack ? 1 : -1;
 }
 
+// Whether the RHS leaves its mass fluxes over dx, dy: only the exact assembly (time schemes
+// 5 to 7, not the fast forms) reads the quotients.
+SWM_HD bool fluxes_over_len(int timescheme, bool fast) { return timescheme > 4 && !fast; }
+
 // The fastest of n schedules, tried in order: form(i) is 0 or 1, time(i) its time, negative
 // when it failed (which ends the search: -1).  A form whose first schedule takes a fifth
 // longer than the best so far is not tried further; a later schedule of a form says
