@@ -221,9 +221,11 @@ static int jacobi_form(const swm_params& p) {
 
 // The three substeps of an mPDeC5 correction depend only on the previous correction, so
 // their systems are solved by one launch: one set of passes, barriers and tails instead
-// of three.  That takes up to 16 more planes; beyond
-// kGroupCells one system alone keeps every SM busy for many passes' worth of rows, and
-// the memory is left to larger grids.
+// of three, and in the exact forms one assembly instead of three.  Measured per step (B200),
+// one by one / together: FP64 256^2 943 / 761 us, 1024^2 8947 / 8667, 2048^2 33778 / 33574,
+// 2896^2 66976 / 66715; CSR 2048^2 34200 / 33908; split 1024^2 3003 / 2751, 2048^2 10419 /
+// 10231, 2896^2 20269 / 20273.  It takes 13 more planes (FP64), 15 (CSR) or 3 (split): beyond
+// kGroupCells, where nothing is left to gain, the memory is left to larger grids.
 constexpr size_t kGroupCells = size_t(1) << 23;
 
 static RhsArgs make_rhs_args(swm_solver* s, const double* h, const double* hu, const double* hv,
@@ -319,10 +321,13 @@ static void prof_mark(swm_solver* s, int cls) {
 // few tiles (fewer launches and part-filled last rounds), in 8 x 8 tiles while even the
 // 16 x 16 tiles of all states would fill less than half of the SMs.  Measured per mPDeC5
 // step (one RHS, then four times three; B200), separate / one launch / one launch of 8 x 8
-// tiles: FP64 50^2 487 / 198 / 124 us, 100^2 490 / 205 / 221, 512^2 2251 / 2153 / 3456;
-// split 50^2 191 / 74 / 54, 512^2 668 / 600 / 1143, 1024^2 2282 / 2254 / -.  A group
-// launch stages its state's arguments in shared memory and loads tiles without TMA, which
-// costs 2.8% of a large grid's RHS.
+// tiles: FP64 50^2 (48 tiles of three states) 337 / 136 / 75 us, 100^2 (147) 337 / 133 / 144,
+// 512^2 1995 / 1903 / 2921, 1024^2 (12288) 7414 / 7290 / -, 2048^2 28806 / 28709 / -; split
+// 50^2 166 / 65 / 54, 100^2 167 / 64 / 73, 512^2 566 / 510 / 836, 1024^2 1900 / 1867 / -, 1448^2
+// 3695 / 3702 / -, 2048^2 7190 / 7285 / -: a group launch stages its state's arguments in
+// shared memory and loads tiles without TMA.  (From 75 to 100 tiles 8 x 8 ones are still
+// ahead: FP64 72^2 91 against 123 us, mPDeC2 160^2 53.8 against 54.6; at 144, mPDeC2 192^2,
+// behind by 66 to 55.)
 constexpr long long kRhsSmallTiles = 64, kRhsGroupTiles = 3 * 4096;
 
 static int launch_rhs_states(swm_solver* s, const RhsArgs* a, int n) {

@@ -97,7 +97,6 @@ struct AssembleMultiArgs {
 
 struct JacobiArgs {
   int nx, ny;
-  int solve_idx;          // slot in ctl->iters
   int maxiter;
   int pitch;              // stencil: row pitch of b, the coefficient planes and xa/xb
                           // (<= 0: nx); out is unpadded
@@ -315,9 +314,7 @@ cudaError_t launch_assemble_batch(const AssembleArgs* descs, const int2* blk, in
 cudaError_t launch_jacobi_batch(const StripBatchArgs& a, int grid_blocks, bool recip,
                                 cudaStream_t s);
 int jacobi_batch_grid_blocks(int device, bool recip);
-// Work items of one problem's set of a batched solve: strips x chunks of at most `rows`
-// rows, evenly.
-int jacobi_batch_strips(int nx);
+int jacobi_batch_strips(int nx);  // strips of a grid nx cells wide
 cudaError_t launch_dt_batch(const DtBatchDesc* d, const int2* blk, int nblk, int nprob,
                             unsigned long long* lam, int* bad, double* dt, cudaStream_t s);
 cudaError_t launch_rhs_fast(int mode, const RhsArgs& a, const RhsTma& tm, cudaStream_t s);

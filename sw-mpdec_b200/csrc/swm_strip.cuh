@@ -7,8 +7,9 @@
 //          computes row s - t from the rows of x^{t-1} that the previous step and the
 //          previous sweep left in registers.  Rows come through a ring in shared memory
 //          that only their own lane reads, so there is no barrier in the walk;
-//  tiles   (passes of up to 4 or 8 sweeps) a block holds a 64-column tile, a few rows per warp; the warps exchange their
-//          edge rows through shared memory after every sweep.
+//  tiles   (passes of up to 4 or 8 sweeps) a block holds a 64-column tile, a few rows per
+//          warp; the warps exchange their edge rows through shared memory after every
+//          sweep.
 // In both, west and east neighbours come from the next lanes, and each row of the system
 // is read once per pass (tiles: once per solve when every block has one tile).
 //
@@ -29,7 +30,6 @@ constexpr int kStripWarps = kJacobiBatchWarps;   // warps of a CTA (independent 
 constexpr int kStripNT = 32 * kStripWarps;
 constexpr int kStripSlots = 4;                   // ring rows: three copies ahead of the sweeps
 constexpr int kStripCols = 64;                   // columns a warp loads
-
 static_assert(kPassT % 2 == 0, "pairs keep their alignment");
 
 template <int FORM>
