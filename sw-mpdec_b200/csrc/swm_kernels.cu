@@ -640,6 +640,8 @@ __device__ __forceinline__ void solve_passes(const JacobiGroup& a, PassShared<TI
   using TG = Tile<FORM, T>;
   JacobiCtl* ctl = a.ctl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int blk = a.block < 1 ? 1 : (a.block > T ? T : a.block);
+  const double thresh = limbs_value(a.thresh[0], a.thresh[1], a.thresh[2]);
   const int strips = (a.nx + TG::UX - 1) / TG::UX, warps = gridDim.x * kStripWarps;
   const int tiles = TILES ? strips * ((a.ny + TG::UY - 1) / TG::UY) : 0;
   static_assert(TILES || G::U == TG::UX, "strips deliver as many columns as tiles");
@@ -743,8 +745,6 @@ __device__ __forceinline__ void solve_passes(const JacobiGroup& a, PassShared<TI
         __syncwarp();
         if (lane < a.nsys && sh.st[lane].active) {
           const JacobiSys& y = a.sys[lane];
-          const int blk = a.block < 1 ? 1 : (a.block > T ? T : a.block);
-          const double thresh = limbs_value(a.thresh[0], a.thresh[1], a.thresh[2]);
           sys_decide<FORM>(sh.st[lane], (double)a.nx * a.ny, a.maxiter, thresh, y.b, y.xa, y.xb,
                            y.out, sh.tot[lane], sh.hint[lane], blk);
           // its passes come after the fast ones'
@@ -760,27 +760,28 @@ __device__ __forceinline__ void solve_passes(const JacobiGroup& a, PassShared<TI
   }
 }
 
-// The systems that the fast passes left: by passes with IEEE divisions, or one sweep at a
-// time.  One call out of line: what it needs must not come out of the fast passes'
-// registers.
+// The systems left to single sweeps.  False when a barrier wait gave up.
 template <int FORM, int TILES>
-__device__ __noinline__ void solve_rest(const JacobiGroup& a, PassShared<TILES>& sh) {
-  if constexpr (FORM != kSysRecip) {
-    if (threadIdx.x < a.nsys) sh.st[threadIdx.x].active = sh.st[threadIdx.x].safe;
-    __syncwarp();  // (warp 0 reads them first)
-    solve_passes<FORM, TILES, true>(a, sh);
-    if (!sh.ok) return;
-  }
+__device__ __forceinline__ bool solve_singly(const JacobiGroup& a, PassShared<TILES>& sh) {
   JacobiCtl* ctl = a.ctl;
   const ExactGrid eg{a.nx,   a.ny,     a.nx,       a.maxiter, a.thresh, a.rowstart, a.cols,
                      ctl->acc, &ctl->bar[a.sys[0].solve_idx], &ctl->status, a.spin_limit};
   for (int q = 0; q < a.nsys; ++q)
-    if (sh.st[q].exact && !solve_exact<FORM>(eg, a.sys[q], sh.st[q], &sh.xpass, &sh.nbar)) {
-      __syncthreads();
-      if (threadIdx.x == 0) sh.ok = 0;
-      __syncthreads();
-      return;
-    }
+    if (sh.st[q].exact && !solve_exact<FORM>(eg, a.sys[q], sh.st[q], &sh.xpass, &sh.nbar))
+      return false;
+  return true;
+}
+
+// The systems that the fast passes left: by passes with IEEE divisions, then by single
+// sweeps.  One call out of line: what it needs must not come out of the fast passes'
+// registers.  (The divided rows have no such passes: a call like this one cost their strips
+// 4% at 2048^2, 1766 against 1696 us a step.)
+template <int FORM, int TILES>
+__device__ __noinline__ bool solve_rest(const JacobiGroup& a, PassShared<TILES>& sh) {
+  if (threadIdx.x < a.nsys) sh.st[threadIdx.x].active = sh.st[threadIdx.x].safe;
+  __syncwarp();  // (warp 0 reads them first)
+  solve_passes<FORM, TILES, true>(a, sh);
+  return sh.ok && solve_singly<FORM, TILES>(a, sh);
 }
 
 template <int FORM, int TILES>
@@ -812,8 +813,11 @@ __global__ void __launch_bounds__(TILES ? kTileNT : kStripNT,
   for (int q = 0; q < a.nsys; ++q) rest = rest || sh.st[q].safe || sh.st[q].exact;
   if (rest) {
     __syncthreads();
-    solve_rest<FORM, TILES>(a, sh);
-    if (!sh.ok) return;
+    if constexpr (FORM == kSysRecip) {
+      if (!solve_singly<FORM, TILES>(a, sh)) return;
+    } else {
+      if (!solve_rest<FORM, TILES>(a, sh)) return;
+    }
   }
   // deliver the final iterates (haVec of the reference) to their destinations
   const int n = a.nx * a.ny;
