@@ -44,13 +44,12 @@ METRIC = "mPDeC5 cell-steps/s at 2048Â²: split-precision vs FP64 GPU at L1 err â
 PEAKS_FALLBACK = {"hbm_gbs": 6650.0}
 
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the split
-# step's kernels, each from one earlier ncu capture at 2048x2048 (4,194,304 cells):
-# constants, not measured by this run.  Each names the commit of the capture; a kernel
-# changed after it makes the figure stale.  Scaled by cells for other grid sizes (the
-# traffic of these kernels grows with the cell count).
+# step's dominant kernel, from one earlier ncu capture at 2048x2048 (4,194,304 cells,
+# profiles/step_kernels.md): a constant, not measured by this run.  It names the commit of
+# the capture; a kernel changed after it makes the figure stale.  Scaled by cells for other
+# grid sizes (the kernel's traffic grows with the cell count).
 NCU_TRAFFIC_2048 = {
-    "rhs": (101655552.0 + 91263232.0, "2c446c5"),
-    "jacobi": (403459328.0 + 58311680.0, "77d112e"),
+    "rhs": (101301248.0 + 89963776.0, "26f529b"),
 }
 
 # Accuracy leg: the island case (stated hump at x = 2) at 256^2 up to t = 0.8, by which

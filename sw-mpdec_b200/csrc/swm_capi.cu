@@ -222,10 +222,10 @@ static int jacobi_form(const swm_params& p) {
 // The three substeps of an mPDeC5 correction depend only on the previous correction, so
 // their systems are solved by one launch: one set of passes, barriers and tails instead
 // of three, and in the exact forms one assembly instead of three.  Measured per step (B200),
-// one by one / together: FP64 256^2 943 / 761 us, 1024^2 8947 / 8667, 2048^2 33778 / 33574,
-// 2896^2 66976 / 66715; CSR 2048^2 34200 / 33908; split 1024^2 3003 / 2751, 2048^2 10419 /
-// 10231, 2896^2 20269 / 20273.  It takes 13 more planes (FP64), 15 (CSR) or 3 (split): beyond
-// kGroupCells, where nothing is left to gain, the memory is left to larger grids.
+// one by one / together: FP64 256^2 945 / 762 us, 1024^2 8948 / 8663, 2048^2 33812 / 33603,
+// 2896^2 66998 / 66755; CSR 2048^2 34251 / 33959; split 1024^2 3012 / 2759, 2048^2 10385 /
+// 10131, 2896^2 20152 / 20085.  It takes 13 more planes (FP64), 15 (CSR) or 3 (split): beyond
+// kGroupCells, where little is left to gain, the memory is left to larger grids.
 constexpr size_t kGroupCells = size_t(1) << 23;
 
 static RhsArgs make_rhs_args(swm_solver* s, const double* h, const double* hu, const double* hv,

@@ -881,11 +881,11 @@ JacobiGrid jacobi_grid(int form, int device) {
 
 // Which pieces a solve is cut into, by how many rounds they make over the resident blocks.
 // Measured per step (13 solves of 8 to 11 sweeps, B200), 8-sweep tiles / 4-sweep tiles /
-// strips: split 50^2 130 / 148 / 197 us, 320^2 (168 and 126 tiles of a launch's three
-// systems over 148 blocks) 187 / 174 / 279, 512^2 (396 and 300) 252 / 291 / 322, 768^2 (864
-// and 630) 410 / 447 / 408, 1024^2 713 / 733 / 547; FP64 400^2 (351 and 240) 293 / 281 / 355,
-// 512^2 (528 and 390) 397 / 361 / 433, 600^2 (741 and 495) 478 / 449 / 429; CSR 600^2 562 / 537
-// / 512; mPDeC2 257^2 (54 and 35) 67 / 85 / 149.  One round of either length beats two (a block
+// strips: split 50^2 136 / 152 / 201 us, 320^2 (168 and 126 tiles of a launch's three
+// systems over 148 blocks) 190 / 174 / 292, 512^2 (396 and 300) 252 / 295 / 332, 768^2 (864
+// and 630) 414 / 457 / 421, 1024^2 721 / 746 / 555; FP64 400^2 (351 and 240) 287 / 280 / 355,
+// 512^2 (528 and 390) 397 / 358 / 434, 600^2 (741 and 495) 479 / 449 / 430; CSR 600^2 559 / 537
+// / 510; mPDeC2 257^2 (54 and 35) 69 / 88 / 148.  One round of either length beats two (a block
 // keeps its rows of the system for the whole solve), the longer passes win up to three
 // rounds (within 5% everywhere), strips beyond.
 constexpr int kTileWaves = 3;

@@ -852,7 +852,7 @@ __device__ __forceinline__ void rhs_tile(const RhsArgs& a, const RhsTma* tm, con
 // deviation can limit.  2048^2 island, one launch: 666 -> 553 us (256 threads; 288 or 320
 // at three blocks spill: 680, 667).
 // FP64 form: bound by the FP64 pipe (76% of its cycles, 7300 operations a cell with a
-// bathymetry source).  1024^2 island, one launch: 637 -> 548 us by reciprocals without
+// bathymetry source).  1024^2 island, one launch: 637 -> 561 us by reciprocals without
 // branches (rcp_mk), quotients of four operations (div_mk2), fused exact factors in the
 // smoothness indicators and the limiter left early.  384 threads (80 registers, spills)
 // 630 before those; 16 x 14 tiles, whose phases fill their rounds of threads, 564.
